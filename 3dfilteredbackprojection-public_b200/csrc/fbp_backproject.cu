@@ -34,6 +34,7 @@
 
 #include "fbp_internal.h"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -1925,134 +1926,373 @@ int launch_bp_batch(fbp_context* L, BPLaunchPlan* const* plans, int n, const lon
 // 2D backprojection (parallel beam and flat-detector fan beam, FBP2D.cpp:96-122
 // and FBP2D.cpp:31-52 with FBP3D's FDK weight restricted to v = 0).
 //
-// The whole filtered sinogram of a 2D job (at most a few MB) sits in L2, so the
-// 3D kernels' TMA window ring, footprint pass and per-view producer would cost
-// more than the taps. A CTA owns a 32 x 32 pixel tile; per chunk of kChunk2D
-// views one warp computes each view's tile-local projective coefficients in
-// FP64 (one view per lane, re-based to the tile origin so FP32 stays
-// accurate) and the detector window the tile needs; all threads then stage the
-// chunk's windows (zero outside the detector) in shared memory and each thread
-// accumulates four pixels of one column: per view one reciprocal of the
-// distance ratio (fan beam), one bilinear tap from shared memory, one FMA.
-constexpr int kTile2D = 32;    // pixels per tile side
-constexpr int kChunk2D = 64;   // views per staged chunk
-constexpr int kPix2D = 4;      // pixels per thread along z
-constexpr int kWin2DMax = 512; // widest staged window (samples): 64 x 512 floats = 128 KB
+// What bounds it is shared memory: a linear tap reads two FP32 samples, 8
+// bytes an update. Everything else of a tap - the projected position, its
+// floor and fraction, the distance weight - is shared by the pixels of a
+// rotational orbit: on a circular orbit the pixel (X, Z) at view k and its
+// image under the rotation that takes view k to view k + j Q project to the
+// same detector position. The filtered rows are packed so that one element
+// holds the samples of the SLOTS rows that such an orbit reads at one detector
+// position:
+//   SLOTS 4  one turn, K % 4 == 0, square image: rows g + j K/4
+//   SLOTS 4  half a turn of parallel beam, K even, square image: rows g,
+//            g + K/2 and the same two mirrored (the view half a turn on)
+//   SLOTS 2  one turn, K even: rows g, g + K/2; any other parallel-beam view
+//            set: row g and its mirror image (the half-turned pixel, same view)
+//   SLOTS 1  any other fan-beam view set
+// In phase m (rows g + m Q of the representative pixel, m < PHASES) the
+// pixel's rotation r reads slot (m + r) mod SLOTS. The phases are the outer
+// loop and the sums stay in slot order, turned by one slot between phases.
+//
+// A CTA owns a 32 x 32 tile of representative pixels, four pixels of one
+// column a thread. A producer warp computes each step's tile-local projective
+// coefficients and window origin in FP64 (one step a lane, re-based to the
+// window so FP32 stays accurate) and copies the windows into a ring of
+// shared-memory entries of kSteps2D steps with cp.async.bulk; the packed rows
+// carry `pad` zero columns on either side, so a window that leaves the
+// detector is an ordinary copy. The views are split over the CTAs of a cluster
+// when the tiles alone would leave SMs idle; the partial sums are added in
+// rank order through distributed shared memory, so results do not depend on
+// timing.
+//
+// Measured (the packing included), before = one 32 x 32 tile of plain pixels
+// a CTA with its setup and staging between block barriers: fan 1024^2, 1440
+// views 2297 -> 523 us (84% of the shared-memory rate while a SM has work),
+// 1441 views 2301 -> 1172 us; fan 512^2, 720 views 467 -> 81 us; parallel
+// 256^2, 360 views 132 -> 21 us (about 12 us of it two launches and a CTA's
+// start).
+constexpr int kTile2D = 32;     // representative pixels per tile side
+constexpr int kPix2D = 4;       // pixels per thread along z
+constexpr int kSteps2D = 4;     // views per ring entry
+constexpr int kWin2DMax = 516;  // widest staged window (columns)
+constexpr int kMaxRing2D = 6;   // ring entries
+constexpr int kMaxSplit2D = 4;  // CTAs that share a tile's views (one cluster)
+constexpr int kPart2D = kTile2D + 1;  // row pitch of the partial sums (no bank conflicts across rows)
+
+struct alignas(16) Coef2D {
+  float Nx, Nz, N0;  // (u - u0) D, affine in the tile-local pixel
+  float Dx, Dz, D0;
+  float pad[2];
+};
 
 struct BP2DArgs {
-  const float* sino;  // [views][pitch] filtered rows
+  const float* rows;  // [groups][pitch][SLOTS]: column c is detector column c - pad
   long long pitch;
   float* image;       // [nz][nx]
   const double2* trig;
-  double sod, sdd, du, vox, cu;
-  int nu, nviews, nx, nz;
-  int wmax;           // staged window width (floats) of one view
+  double vox, cu;
+  double du_per_mm;   // detector columns per unit of u D (cone: sdd / (sod du); parallel: 1 / du)
+  double inv_sod;     // cone: D = 1 + (X cos + Z sin) inv_sod
+  int nu, nx, nz;
+  int groups, phases;
+  int pad, win;       // zero columns either side, staged columns of a window
+  int ring;           // ring entries
   float scale;
   int* err;
 };
 
-template <bool CONE>
-__global__ void __launch_bounds__(256) bp2d_kernel(const BP2DArgs a) {
-  extern __shared__ __align__(16) unsigned char smem2d[];
-  float* win = reinterpret_cast<float*>(smem2d);                       // kChunk2D x wmax
-  float4* cof = reinterpret_cast<float4*>(win + kChunk2D * a.wmax);    // (Nx, Nz, N0, bu2) per view
-  float4* dco = cof + kChunk2D;                                        // (Dx, Dz, D0, u0 bits) per view
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ix0 = blockIdx.x * kTile2D, iz0 = blockIdx.y * kTile2D;
-  const int tx = lane, tz = warp * kPix2D;
-  float acc[kPix2D];
+// rows [view][pitch] -> [g][column][SLOTS] with zero columns outside the detector
+template <int SLOTS>
+__global__ void pack2d_kernel(const float* __restrict__ src, long long spitch, int nu, int groups, int pad, int mirror,
+                              long long pitch, float* __restrict__ out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, u = c - pad;
+  if (c >= pitch) return;
+  const bool in = u >= 0 && u < nu;
+  for (int g = blockIdx.y; g < groups; g += gridDim.y) {
+    float v[SLOTS];
 #pragma unroll
-  for (int j = 0; j < kPix2D; ++j) acc[j] = 0.f;
-  bool bad = false;
-  const double Xc = (ix0 + 0.5 - 0.5 * a.nx) * a.vox, Zc = (iz0 + 0.5 - 0.5 * a.nz) * a.vox;
-  for (int k0 = 0; k0 < a.nviews; k0 += kChunk2D) {
-    const int nk = min(kChunk2D, a.nviews - k0);
-    __syncthreads();  // the previous chunk's windows are no longer read
-    if (warp == 0) {
-      for (int v = lane; v < nk; v += 32) {
-        const double c = a.trig[k0 + v].x, s = a.trig[k0 + v].y;
-        double Dx = 0.0, Dz = 0.0, D0 = 1.0, Ux, Uz, U0;
-        if (CONE) {
-          const double K = a.sdd / (a.sod * a.du);
-          Dx = a.vox * c / a.sod;
-          Dz = a.vox * s / a.sod;
-          D0 = (a.sod + Xc * c + Zc * s) / a.sod;
-          Ux = -a.vox * s * K;
-          Uz = a.vox * c * K;
-          U0 = (-Xc * s + Zc * c) * K;
-        } else {
-          Ux = -a.vox * s / a.du;
-          Uz = a.vox * c / a.du;
-          U0 = (-Xc * s + Zc * c) / a.du;
+    for (int s = 0; s < SLOTS; ++s) {
+      // slots past `mirror` rows are the first ones' mirror images
+      const int row = s < mirror ? s : s - mirror, at = s < mirror ? u : nu - 1 - u;
+      v[s] = in ? __ldg(src + (long long)(g + row * groups) * spitch + at) : 0.f;
+    }
+    float* o = out + ((long long)g * pitch + c) * SLOTS;
+    if constexpr (SLOTS == 4) *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+    else if constexpr (SLOTS == 2) *reinterpret_cast<float2*>(o) = make_float2(v[0], v[1]);
+    else o[0] = v[0];
+  }
+}
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+template <bool CONE, int SLOTS>
+__global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(128) unsigned char smem2d[];
+  constexpr int NCW = 8;
+  constexpr int ALIGN = 4 / SLOTS;  // columns per 16 bytes
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), nsplit = (int)cluster.num_blocks();
+  const int E = a.ring;
+  const uint32_t win_bytes = (uint32_t)(a.win * SLOTS * 4);
+  float* part = reinterpret_cast<float*>(smem2d);  // [SLOTS][32][kPart2D]
+  unsigned char* wins = smem2d + sizeof(float) * SLOTS * kTile2D * kPart2D;  // a multiple of 128 bytes
+  Coef2D* coef = reinterpret_cast<Coef2D*>(wins + (size_t)E * kSteps2D * win_bytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(coef + E * kSteps2D);
+  uint64_t* empty = full + E;
+  volatile int* s_abort = reinterpret_cast<volatile int*>(empty + E);
+  if (tid == 0) {
+    *s_abort = *(volatile int*)a.err != 0;
+    for (int e = 0; e < E; ++e) {
+      mbar_init(&full[e], 1);
+      mbar_init(&empty[e], NCW);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  const int ix0 = blockIdx.x * kTile2D, iz0 = blockIdx.y * kTile2D;
+  // this CTA's row groups, in every phase
+  const int g0 = (int)((long long)a.groups * rank / nsplit), g1 = (int)((long long)a.groups * (rank + 1) / nsplit);
+  const int ng = g1 - g0, entries = (ng + kSteps2D - 1) / kSteps2D;
+  const bool run = *s_abort == 0;  // an error already recorded: nothing is computed, the cluster still meets below
+
+  float acc[SLOTS][kPix2D];
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s)
+#pragma unroll
+    for (int j = 0; j < kPix2D; ++j) acc[s][j] = 0.f;
+
+  if (run && warp == NCW) {
+    // ---------------------------------------------------------------- producer
+    // the packed rows (and whatever ran before them) are complete from here on
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const double Xc = (ix0 + 0.5 - 0.5 * a.nx) * a.vox, Zc = (iz0 + 0.5 - 0.5 * a.nz) * a.vox;
+    int seq = 0;  // entries filled
+    bool ok = true;
+    for (int m = 0; m < a.phases && ok; ++m)
+      for (int gb = 0; gb < ng && ok; gb += 32) {
+        Coef2D cf{};
+        int start = 0;
+        if (gb + lane < ng) {
+          const int k = g0 + gb + lane + m * a.groups;
+          const double c = a.trig[k].x, s = a.trig[k].y;
+          double Dx = 0.0, Dz = 0.0, D0 = 1.0;
+          if (CONE) {
+            Dx = a.vox * a.inv_sod * c;
+            Dz = a.vox * a.inv_sod * s;
+            D0 = 1.0 + (Xc * c + Zc * s) * a.inv_sod;
+          }
+          const double Ux = -a.vox * s * a.du_per_mm, Uz = a.vox * c * a.du_per_mm;
+          const double U0 = (-Xc * s + Zc * c) * a.du_per_mm;
+          // Detector window over the tile's four corners (u is monotonic along
+          // each edge, so the corners bound it). FP32 is enough here, to well
+          // under the window's margin; the FP64 chain of a lane is what delays
+          // a CTA's first steps, so it holds no division.
+          float umin = 3e38f, umax = -3e38f, dmin = 3e38f;
+          const float fUx = (float)Ux, fUz = (float)Uz, fU0 = (float)U0;
+          const float fDx = (float)Dx, fDz = (float)Dz, fD0 = (float)D0;
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) {
+            const float x = (cc & 1) ? (float)(kTile2D - 1) : 0.f, z = (cc & 2) ? (float)(kTile2D - 1) : 0.f;
+            const float D = fmaf(fDx, x, fmaf(fDz, z, fD0));
+            const float n = fmaf(fUx, x, fmaf(fUz, z, fU0));
+            const float u = (CONE ? n * rcp_approx(D) : n) + (float)a.cu;
+            dmin = fminf(dmin, D);
+            umin = fminf(umin, u);
+            umax = fmaxf(umax, u);
+          }
+          // one column of margin on each side for the FP32 rounding of u; a
+          // window that starts left of the padding or past the detector holds
+          // zeros only, whatever its origin
+          const int cap = 1 << 20;
+          const int u0 = (int)floorf(fminf(fmaxf(umin - 1.f, (float)-cap), (float)cap)) & ~(ALIGN - 1);
+          const bool fits = floorf(umax) + 3.f - (float)u0 <= (float)a.win;
+          if (!(dmin > 1e-6f) || !fits) atomicCAS(a.err, 0, kDevFootprint);
+          start = min(max(u0 + a.pad, 0), a.pad + (a.nu + ALIGN - 1) / ALIGN * ALIGN);
+          const double du0 = a.cu - u0;  // u - u0 = (N . (x, z, 1)) / D with N re-based
+          cf.Nx = (float)(Ux + du0 * Dx);
+          cf.Nz = (float)(Uz + du0 * Dz);
+          cf.N0 = (float)(U0 + du0 * D0);
+          cf.Dx = (float)Dx;
+          cf.Dz = (float)Dz;
+          cf.D0 = (float)D0;
         }
-        // detector window over the tile's four corners (u is monotonic along
-        // each edge, so the corners bound it)
-        double umin = 1e300, umax = -1e300, dmin = 1e300;
-        for (int cc = 0; cc < 4; ++cc) {
-          const double x = (cc & 1) ? kTile2D - 1 : 0, z = (cc & 2) ? kTile2D - 1 : 0;
-          const double D = Dx * x + Dz * z + D0;
-          dmin = fmin(dmin, D);
-          const double u = (Ux * x + Uz * z + U0) / D + a.cu;
-          umin = fmin(umin, u);
-          umax = fmax(umax, u);
+        const int left = min(32, ng - gb);
+        for (int i = 0; i < left; i += kSteps2D) {
+          const int e = seq % E, n = min(kSteps2D, left - i);
+          if (seq >= E && !mbar_wait(&empty[e], ((seq / E) & 1) ^ 1, a.err)) {
+            ok = false;
+            *s_abort = 1;
+            break;
+          }
+          if (lane >= i && lane < i + n) coef[e * kSteps2D + lane - i] = cf;
+          __syncwarp();
+          if (lane == 0) mbar_arrive_expect_tx(&full[e], (uint32_t)n * win_bytes);
+          __syncwarp();
+          if (lane >= i && lane < i + n)
+            bulk_load(wins + (size_t)(e * kSteps2D + lane - i) * win_bytes,
+                      a.rows + ((long long)(g0 + gb + lane) * a.pitch + start) * SLOTS, win_bytes, &full[e]);
+          __syncwarp();
+          ++seq;
         }
-        // one sample of margin on each side for the FP32 rounding of u
-        const int u0 = (int)floor(umin) - 1;
-        const int need = (int)floor(umax) + 3 - u0;
-        if (dmin <= 1e-6 || need > a.wmax) atomicCAS(a.err, 0, kDevFootprint);
-        const double du0 = a.cu - u0;  // u - u0 = (N . (x, z, 1)) / D with N re-based
-        cof[v] = make_float4((float)(Ux + du0 * Dx), (float)(Uz + du0 * Dz), (float)(U0 + du0 * D0),
-                             __int_as_float(min(need, a.wmax) - 2));
-        dco[v] = make_float4((float)Dx, (float)Dz, (float)D0, __int_as_float(u0));
       }
-    }
-    __syncthreads();
-    // stage the chunk's windows: row k0 + v, the samples u0 .. u0 + need - 1
-    // that its taps can read (zero outside the detector)
-    for (int i = tid; i < nk * a.wmax; i += blockDim.x) {
-      const int v = i / a.wmax, e = i - v * a.wmax;
-      if (e > __float_as_int(cof[v].w) + 1) continue;
-      const int u = __float_as_int(dco[v].w) + e;
-      win[i] = (u >= 0 && u < a.nu) ? __ldg(a.sino + (long long)(k0 + v) * a.pitch + u) : 0.f;
-    }
-    __syncthreads();
-    const float fx = (float)tx;
-    for (int v = 0; v < nk; ++v) {
-      const float4 N = cof[v], D = dco[v];
-      const int bu2 = __float_as_int(N.w);
-      const float* w = win + v * a.wmax;
+    // leave only when every copy issued into this CTA's memory has landed
+    for (int q = max(0, seq - E); q < seq; ++q) mbar_wait(&full[q % E], (q / E) & 1, a.err);
+  } else if (run) {
+    // --------------------------------------------------------------- consumers
+    const float fx = (float)lane, fz = (float)(warp * kPix2D);
+    const uint32_t wbase = smem_u32(wins);
+    // bit patterns of kMagic + column, column in [0, win - 2]: bounds the reads
+    const int lo = (int)kMagicBits, hi = (int)kMagicBits + a.win - 2;
+    const float2 magic2 = make_float2(kMagic, kMagic);
+    int e = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int m = 0; m < a.phases && ok; ++m) {
+      for (int q = 0; q < entries; ++q) {
+        if (!mbar_wait(&full[e], ph, a.err)) {
+          ok = false;
+          *s_abort = 1;
+          break;
+        }
+        const int n = min(kSteps2D, ng - q * kSteps2D);
+        for (int i = 0; i < n; ++i) {
+          const float4 N = *reinterpret_cast<const float4*>(&coef[e * kSteps2D + i]);
+          const float2 D = *reinterpret_cast<const float2*>(&coef[e * kSteps2D + i].Dz);
+          const uint32_t c0 = wbase + (uint32_t)(e * kSteps2D + i) * win_bytes - kMagicBits * (4u * SLOTS);
+          // pixels j, j + 1 as packed pairs, stepped along z
+          const float n0 = fmaf(N.x, fx, fmaf(N.y, fz, N.z)), d0 = fmaf(N.w, fx, fmaf(D.x, fz, D.y));
+          float2 num = make_float2(n0, n0 + N.y), den = make_float2(d0, d0 + D.x);
+          const float2 nstep = make_float2(2.f * N.y, 2.f * N.y), dstep = make_float2(2.f * D.x, 2.f * D.x);
+#pragma unroll
+          for (int j = 0; j < kPix2D; j += 2) {
+            if (j) {
+              num = fadd2(num, nstep);
+              if (CONE) den = fadd2(den, dstep);
+            }
+            float2 u = num, W = make_float2(1.f, 1.f);
+            if (CONE) {
+              const float2 rD = make_float2(rcp_approx(den.x), rcp_approx(den.y));
+              u = make_float2(__fmul_rn(num.x, rD.x), __fmul_rn(num.y, rD.y));
+              W = make_float2(__fmul_rn(rD.x, rD.x), __fmul_rn(rD.y, rD.y));
+            }
+            const float2 t = fadd2_rz(u, magic2);
+            const float2 fu = fsub2(u, fsub2(t, magic2));
+            const float wb[2] = {CONE ? W.x * fu.x : fu.x, CONE ? W.y * fu.y : fu.y};
+            const float wa[2] = {W.x - wb[0], W.y - wb[1]};
+            const int bits[2] = {max(min(__float_as_int(t.x), hi), lo), max(min(__float_as_int(t.y), hi), lo)};
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+              const uint32_t at = (uint32_t)bits[p] * (4u * SLOTS) + c0;
+              if constexpr (SLOTS == 4) {
+                const uint4 A = lds_u4(at), B = lds_u4(at + 16);
+                const float2 wa2 = make_float2(wa[p], wa[p]), wb2 = make_float2(wb[p], wb[p]);
+                float2 s01 = make_float2(acc[0][j + p], acc[1][j + p]), s23 = make_float2(acc[2][j + p], acc[3][j + p]);
+                s01 = ffma2(wa2, make_float2(__uint_as_float(A.x), __uint_as_float(A.y)), s01);
+                s23 = ffma2(wa2, make_float2(__uint_as_float(A.z), __uint_as_float(A.w)), s23);
+                s01 = ffma2(wb2, make_float2(__uint_as_float(B.x), __uint_as_float(B.y)), s01);
+                s23 = ffma2(wb2, make_float2(__uint_as_float(B.z), __uint_as_float(B.w)), s23);
+                acc[0][j + p] = s01.x, acc[1][j + p] = s01.y, acc[2][j + p] = s23.x, acc[3][j + p] = s23.y;
+              } else if constexpr (SLOTS == 2) {
+                const float2 A = lds_f32x2(at), B = lds_f32x2(at + 8);
+                float2 s01 = make_float2(acc[0][j + p], acc[1][j + p]);
+                s01 = ffma2(make_float2(wa[p], wa[p]), A, s01);
+                s01 = ffma2(make_float2(wb[p], wb[p]), B, s01);
+                acc[0][j + p] = s01.x, acc[1][j + p] = s01.y;
+              } else {
+                acc[0][j + p] = fmaf(wa[p], lds_f32(at), acc[0][j + p]);
+                acc[0][j + p] = fmaf(wb[p], lds_f32(at + 4), acc[0][j + p]);
+              }
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[e]);
+        if (++e == E) {
+          e = 0;
+          ph ^= 1;
+        }
+      }
+      // the next phase's slot s belongs to the rotation of this phase's slot s - 1
 #pragma unroll
       for (int j = 0; j < kPix2D; ++j) {
-        const float fz = (float)(tz + j);
-        const float num = fmaf(N.x, fx, fmaf(N.y, fz, N.z));
-        float u, W;
-        if (CONE) {
-          const float rD = __frcp_rn(fmaf(D.x, fx, fmaf(D.y, fz, D.z)));
-          u = num * rD;
-          W = rD * rD;
-        } else {
-          u = num;
-          W = 1.f;
-        }
-        const float fu = floorf(u);
-        const int iu = (int)fu;
-        if (iu >= 0 && iu <= bu2) {
-          const float t = u - fu, a0 = w[iu], a1 = w[iu + 1];
-          acc[j] = fmaf(W, fmaf(t, a1 - a0, a0), acc[j]);
-        } else {
-          bad = true;
-        }
+        const float t = acc[SLOTS - 1][j];
+#pragma unroll
+        for (int s = SLOTS - 1; s > 0; --s) acc[s][j] = acc[s - 1][j];
+        acc[0][j] = t;
       }
     }
   }
-  if (bad) atomicCAS(a.err, 0, kDevFootprint);
-  const int ix = ix0 + tx;
-  if (ix < a.nx)
+  if (warp < NCW) {
+    // after `phases` turns rotation r sits in slot (r + phases) mod SLOTS
 #pragma unroll
-    for (int j = 0; j < kPix2D; ++j) {
-      const int iz = iz0 + tz + j;
-      if (iz < a.nz) a.image[(size_t)iz * a.nx + ix] = acc[j] * a.scale;
+    for (int s = 0; s < SLOTS; ++s) {
+      const int r = (s + SLOTS - a.phases % SLOTS) % SLOTS;
+#pragma unroll
+      for (int j = 0; j < kPix2D; ++j) part[(r * kTile2D + warp * kPix2D + j) * kPart2D + lane] = acc[s][j];
     }
+  }
+  __syncwarp();
+  if (nsplit > 1) cluster.sync();
+  else __syncthreads();
+  // The tile's SLOTS rotated images, a 32-pixel line of image x a warp: for
+  // the quarter turns (x, z) -> (n-1-z, x) -> (n-1-x, n-1-z) -> (z, n-1-x)
+  // image x runs along the tile's z. Pixels that are their own image (the
+  // middle row / the centre of an odd size) are written by rotation 0 alone.
+  const bool skip = *s_abort != 0;
+  for (int l = rank + nsplit * warp; l < SLOTS * kTile2D && !skip && warp < NCW; l += nsplit * NCW) {
+    const int r = l / kTile2D, i = l - r * kTile2D;
+    const bool turned = SLOTS == 4 && (r & 1);
+    const int x = turned ? i : lane, z = turned ? lane : i;
+    const float* own = part + (r * kTile2D + z) * kPart2D + x;
+    float sum;
+    if (nsplit == 1) {
+      sum = *own;
+    } else {  // all ranks' loads in flight, added in rank order
+      float v[kMaxSplit2D];
+#pragma unroll
+      for (int q = 0; q < kMaxSplit2D; ++q) v[q] = q < nsplit ? *cluster.map_shared_rank(own, q) : 0.f;
+      sum = v[0];
+#pragma unroll
+      for (int q = 1; q < kMaxSplit2D; ++q) sum += v[q];
+    }
+    const int ix = ix0 + x, iz = iz0 + z;
+    bool in = ix < a.nx && iz < a.nz;
+    int ox = ix, oz = iz;
+    if (SLOTS == 4) {
+      const int n = a.nx, h = n / 2;  // representatives: x < n - h, z < h, and the centre of an odd size
+      in = ix < n - h && (iz < h || (r == 0 && iz == h && ix == h && (n & 1)));
+      if (r == 1) ox = n - 1 - iz, oz = ix;
+      if (r == 2) ox = n - 1 - ix, oz = n - 1 - iz;
+      if (r == 3) ox = iz, oz = n - 1 - ix;
+    } else if (SLOTS == 2) {
+      in = ix < a.nx && (iz < a.nz / 2 || (r == 0 && iz == a.nz / 2 && (a.nz & 1)));
+      if (r == 1) ox = a.nx - 1 - ix, oz = a.nz - 1 - iz;
+    }
+    if (in) a.image[(size_t)oz * a.nx + ox] = sum * a.scale;
+  }
+  __syncwarp();
+  if (nsplit > 1) cluster.sync();  // no CTA leaves while another reads its sums
+}
+
+template <bool CONE, int SLOTS>
+cudaError_t launch_bp2d_cfg(const BP2DArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
+  auto kern = bp2d_kernel<CONE, SLOTS>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(256 + 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = grid.z;
+  // the CTAs start (barriers, cluster) while the packing kernel drains
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
 int launch_bp2d(fbp_context* ctx, const BPGeom& g, const float* sino, long long pitch, float* image) {
@@ -2068,35 +2308,84 @@ int launch_bp2d(fbp_context* ctx, const BPGeom& g, const float* sino, long long 
     if (dmin < 0.05) return FBP_ERR_UNSUPPORTED;  // the source inside or near the image: general path
     width *= g.sdd / (g.sod * dmin);
   }
-  const int wmax = ((int)std::ceil(width) + 4 + 3) / 4 * 4;
-  if (wmax > kWin2DMax) return FBP_ERR_UNSUPPORTED;
+  if (!(width < kWin2DMax)) return FBP_ERR_UNSUPPORTED;
+  const int win = ((int)std::ceil(width) + 8 + 3) / 4 * 4;
+  if (win > kWin2DMax) return FBP_ERR_UNSUPPORTED;
+  // rotational orbits of the view set
+  const double turns = g.span / (2.0 * pi);
+  const long long whole = llround(turns), halves = llround(2.0 * turns);
+  const bool full_turn = fabs(turns - (double)whole) < 1e-9;
+  const bool half_turn = !full_turn && fabs(2.0 * turns - (double)halves) < 1e-9;  // an odd number of halves
+  const bool square = g.nx == g.nz;
+  const int K = g.nviews;
+  // Four slots halve the work of two, but also the tiles: below one CTA a SM
+  // (the cluster split included) two are faster (parallel 256^2, 360 views,
+  // half a turn: 27.1 us with four slots, 21.0 with two)
+  const int half = ((g.nx + 1) / 2 + kTile2D - 1) / kTile2D;
+  const bool four = square && half * half * kMaxSplit2D >= ctx->num_sms;
+  int slots = 1, groups = K, phases = 1, mirror = 1;  // mirror: rows of an element before their mirror images
+  if (four && full_turn && whole % 4 == 1 && K % 4 == 0) {
+    slots = 4, groups = K / 4, phases = 4, mirror = 4;
+  } else if (four && !cone && half_turn && halves % 4 == 1 && K % 2 == 0) {
+    slots = 4, groups = K / 2, phases = 2, mirror = 2;
+  } else if (full_turn && (whole % 2 == 1 || whole % 2 == -1) && K % 2 == 0) {
+    slots = 2, groups = K / 2, phases = 2, mirror = 2;
+  } else if (!cone) {
+    slots = 2, groups = K, phases = 1, mirror = 1;
+  }
+  const int rx = slots == 4 ? (g.nx + 1) / 2 : g.nx, rz = slots == 1 ? g.nz : (g.nz + 1) / 2;
+  const int tiles_x = (rx + kTile2D - 1) / kTile2D, tiles_z = (rz + kTile2D - 1) / kTile2D;
+  const long long tiles = (long long)tiles_x * tiles_z;
   if (int rc = ensure_trig(ctx, g)) return rc;
   BP2DArgs a;
-  a.sino = sino;
-  a.pitch = pitch;
+  a.pad = win;
+  a.win = win;
+  a.pitch = (g.nu + 3) / 4 * 4 + 2LL * win;
+  const size_t bytes = sizeof(float) * (size_t)a.pitch * groups * slots;
+  float* rows = static_cast<float*>(scratch(ctx, bytes));
+  if (!rows) return FBP_ERR_OUT_OF_MEMORY;
+  const dim3 pgrid((unsigned)((a.pitch + 255) / 256), std::min(groups, 65535));
+  if (slots == 4)
+    pack2d_kernel<4><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
+  else if (slots == 2)
+    pack2d_kernel<2><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
+  else
+    pack2d_kernel<1><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
+  if (int rc = launched(ctx, "pack2d_kernel")) return rc;
+  a.rows = rows;
   a.image = image;
   a.trig = ctx->d_trig;
-  a.sod = g.sod;
-  a.sdd = g.sdd;
-  a.du = g.du;
   a.vox = g.vox;
   a.cu = 0.5 * g.nu - 0.5;
+  a.du_per_mm = cone ? g.sdd / (g.sod * g.du) : 1.0 / g.du;
+  a.inv_sod = cone ? 1.0 / g.sod : 0.0;
   a.nu = g.nu;
-  a.nviews = g.nviews;
   a.nx = g.nx;
   a.nz = g.nz;
-  a.wmax = wmax;
-  a.scale = cone ? (float)(pi / g.nviews * g.sdd / (g.sod * g.du)) : (float)(pi / g.nviews / g.du);
+  a.groups = groups;
+  a.phases = phases;
+  a.scale = cone ? (float)(pi / K * g.sdd / (g.sod * g.du)) : (float)(pi / K / g.du);
   a.err = ctx->d_err;
-  const size_t smem = sizeof(float) * kChunk2D * wmax + 2 * sizeof(float4) * kChunk2D;
-  auto kern = cone ? bp2d_kernel<true> : bp2d_kernel<false>;
-  if (int rc = cuda_check(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    (int)(sizeof(float) * kChunk2D * kWin2DMax + 2 * sizeof(float4) * kChunk2D)),
-                          "bp2d_kernel shared memory"))
-    return rc;
-  const dim3 grid((g.nx + kTile2D - 1) / kTile2D, (g.nz + kTile2D - 1) / kTile2D);
-  kern<<<grid, 256, smem, ctx->stream>>>(a);
-  return launched(ctx, "bp2d_kernel");
+  const size_t entry = (size_t)kSteps2D * (win * slots * 4 + sizeof(Coef2D)) + 2 * sizeof(uint64_t);
+  const size_t fixed = sizeof(float) * slots * kTile2D * kPart2D + 16;
+  a.ring = (int)std::max<size_t>(2, std::min<size_t>(kMaxRing2D, (48 * 1024) / entry));
+  size_t smem = fixed + a.ring * entry;
+  // Split the views over a cluster until one and a half tiles a SM are in
+  // flight (fan 512^2, 720 views, 64 tiles: 158.8, 89.2, 81.1, 91.9 us split
+  // 1, 2, 4, 8 ways; 1024^2, 1440 views, 256 tiles: 522.9, 526.1, 520.7,
+  // 558.7 us). Clusters of 8 leave SMs of a GPC over.
+  int split = 1;
+  while (split < kMaxSplit2D && 2 * tiles * split < 3LL * ctx->num_sms && groups >= 16 * split) split *= 2;
+  // CTAs that all find an SM of their own must not share one (the tap's
+  // shared-memory rate is per SM): ask for more than half an SM's memory
+  if (tiles * split <= ctx->num_sms) smem = std::max<size_t>(smem, 116 * 1024);
+  const dim3 grid(tiles_x, tiles_z, split);
+  cudaError_t e;
+  if (slots == 4) e = cone ? launch_bp2d_cfg<true, 4>(a, grid, smem, ctx->stream) : launch_bp2d_cfg<false, 4>(a, grid, smem, ctx->stream);
+  else if (slots == 2) e = cone ? launch_bp2d_cfg<true, 2>(a, grid, smem, ctx->stream) : launch_bp2d_cfg<false, 2>(a, grid, smem, ctx->stream);
+  else e = cone ? launch_bp2d_cfg<true, 1>(a, grid, smem, ctx->stream) : launch_bp2d_cfg<false, 1>(a, grid, smem, ctx->stream);
+  if (e == cudaSuccess) ctx->launches++;
+  return cuda_check(ctx, e, "bp2d_kernel");
 }
 
 int launch_clip(fbp_context* ctx, float* vol, int nx, int ny, int nz, int y_limit) {
