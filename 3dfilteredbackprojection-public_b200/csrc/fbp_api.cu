@@ -708,7 +708,7 @@ int fbp_destroy(fbp_context* ctx) {
     cudaFree(ctx->d_trig);
     cudaFree(ctx->d_span);
     cudaFree(ctx->d_stage2d);
-    cudaFree(ctx->ftab.twiddle);
+    cudaFree(ctx->ftab.tws);
     cudaFree(ctx->ftab.hbr);
     cudaFree(ctx->ftab.kernel);
     cudaFree(ctx->ttab.th);

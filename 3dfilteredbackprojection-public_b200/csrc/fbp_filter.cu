@@ -10,12 +10,22 @@
 //
 // Algorithm: two real rows are packed as the real and imaginary parts of one
 // complex row (the filter response H is real and even, so the filtered rows
-// come back as the real and imaginary parts). Forward transform is a
-// decimation-in-frequency radix-2 FFT (natural order in, bit-reversed out),
-// the spectrum is multiplied by H[bitrev(k)]/n, and the inverse is a
-// decimation-in-time radix-2 FFT (bit-reversed in, natural order out), so no
+// come back as the real and imaginary parts). The forward transform is a
+// decimation-in-frequency FFT (natural order in, bit-reversed out), the
+// spectrum is multiplied by H[bitrev(k)]/n, and the inverse is a
+// decimation-in-time FFT (bit-reversed in, natural order out), so no
 // bit-reversal permutation is ever executed. Row padding to n samples is the
 // reference's (next power of two >= width, FastFourierTransformGPU.cpp:258-262).
+//
+// The transforms run in registers: a thread holds E = 8 or 16 samples whose
+// indices differ in log2(E) index bits and does those radix-2 stages at once
+// (constant twiddles inside, one table twiddle per sample after them); the
+// row is exchanged through shared memory between such phases only. n = 512 is
+// three phases of three bits (two exchanges each way), n = 1024 .. 4096 three
+// phases of up to four bits. The samples a thread holds in the last forward
+// phase are those of the first inverse phase, and those of the last inverse
+// phase are the ones it loaded, so the row is read from and written to memory
+// from registers.
 //
 // The filter response and the spatial kernel are generated on the GPU in
 // FP64 from the band-limited ramp kernel (h(0) = 1/4, h(odd k) = -1/(pi k)^2,
@@ -52,42 +62,102 @@ __device__ __forceinline__ double filter_window(int filter, double f) {
   }
 }
 
-// H[k] for k < n (one thread per k), FP64.
-__global__ void response_kernel(int n, int filter, double* H) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  long long kk = k <= n / 2 ? k : (long long)k - n;
-  double f = fabs((double)kk) / n;
-  if (filter == FBP_FILTER_RAMP_SAMPLED) {
-    H[k] = f;
-    return;
-  }
-  double s = 0.25;  // j = 0 term (cos 0 = 1)
-  for (int j = 1; j < n; j += 2) {
-    long long jj = j <= n / 2 ? j : (long long)j - n;
-    long long p = ((long long)j * k) % n;
-    s += ramp_tap(jj) * cospi(2.0 * (double)p / n);
-  }
-  H[k] = s * filter_window(filter, f);
+// Register phases of the n = 2^L transform: E = 2^fft_ebits(L) samples a
+// thread; phase k covers the E index bits below the first k E, the last phase
+// what is left. E keeps the number of phases (the exchanges) lowest with the
+// fewest registers.
+__host__ __device__ constexpr int fft_ebits(int L) { return L <= 4 ? L : (L == 7 || L == 12) ? 4 : 3; }
+__host__ __device__ constexpr int fft_phases(int L) { return L == 0 ? 1 : (L + fft_ebits(L) - 1) / fft_ebits(L); }
+// Lowest index bit of phase k (not the last one) and its first entry in the
+// twiddle table: phase k's table is [slot 1 .. E - 1][d < 2^lo].
+__host__ __device__ constexpr int fft_lo(int L, int k) { return L - (k + 1) * fft_ebits(L); }
+__host__ __device__ constexpr int fft_tw_offset(int L, int k) {
+  int o = 0;
+  for (int i = 0; i < k; ++i) o += ((1 << fft_ebits(L)) - 1) << fft_lo(L, i);
+  return o;
 }
 
-// From H: hbr (bit-reversed, divided by n), twiddles, spatial kernel g.
-__global__ void tables_kernel(int n, int log2n, const double* H, float* hbr, float2* tw, float* g) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const unsigned r = log2n > 0 ? __brev((unsigned)k) >> (32 - log2n) : 0u;  // n = 1: the one sample
-  hbr[k] = (float)(H[r] / n);
-  if (k < n / 2) {
-    double s, c;
-    sincospi(-2.0 * (double)k / n, &s, &c);
-    tw[k] = make_float2((float)c, (float)s);
+// The filter tables are O(n^2) sums of FP64 cosines. One block takes one
+// entry; the cosines cos(2 pi p / n) come from a table that the block fills
+// (n / 4 + 1 values, the other quadrants by symmetry) instead of one FP64
+// cosine and one 64-bit remainder per term: at n = 2048, 1.39 ms before.
+constexpr int kTableThreads = 128;
+
+__device__ __forceinline__ void fill_quarter_cos(int n, double* q) {
+  for (int i = threadIdx.x; i <= n / 4; i += blockDim.x) q[i] = cospi(2.0 * (double)i / n);
+}
+__device__ __forceinline__ double quarter_cos(const double* q, int n, unsigned p) {  // cos(2 pi p / n), p taken mod n
+  p &= (unsigned)(n - 1);
+  if (n < 4) return n == 1 || p == 0 ? 1.0 : -1.0;
+  const unsigned h = p <= (unsigned)n / 2 ? p : n - p;  // cos is even about n / 2
+  return h <= (unsigned)n / 4 ? q[h] : -q[n / 2 - h];
+}
+__device__ __forceinline__ double block_sum(double v) {
+  __shared__ double part[kTableThreads / 32];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = 0.0;
+  for (int i = 0; i < kTableThreads / 32; ++i) v += part[i];
+  return v;
+}
+
+// H[k], FP64: the transform of the wrapped band-limited ramp times the window.
+__global__ void __launch_bounds__(kTableThreads) response_kernel(int n, int filter, double* H) {
+  extern __shared__ double quarter[];
+  if (filter != FBP_FILTER_RAMP_SAMPLED) fill_quarter_cos(n, quarter);
+  __syncthreads();
+  for (int k = blockIdx.x; k <= n / 2; k += gridDim.x) {
+    const double f = (double)k / n;
+    double h = f;
+    if (filter != FBP_FILTER_RAMP_SAMPLED) {
+      // odd taps j and n - j are equal and share their cosine
+      double s = 0.0;
+      for (int j = 1 + 2 * (int)threadIdx.x; j < n; j += 2 * kTableThreads)
+        s += ramp_tap(j <= n / 2 ? j : n - j) * quarter_cos(quarter, n, (unsigned)j * (unsigned)k);
+      h = (0.25 + block_sum(s)) * filter_window(filter, f);  // j = 0 term 1/4 (cos 0 = 1)
+    }
+    if (threadIdx.x == 0) {
+      H[k] = h;
+      if (k > 0 && k < n - k) H[n - k] = h;  // even
+    }
   }
-  double acc = 0.0;
-  for (int j = 0; j < n; j++) {
-    long long p = ((long long)j * k) % n;
-    acc += H[j] * cospi(2.0 * (double)p / n);
+}
+
+// From H: hbr (bit-reversed, divided by n), the phases' twiddles and (kernel
+// != nullptr) the spatial kernel g.
+__global__ void __launch_bounds__(kTableThreads) tables_kernel(int n, int log2n, const double* H, float* hbr,
+                                                               float2* tws, float* g) {
+  extern __shared__ double quarter[];
+  if (g) fill_quarter_cos(n, quarter);
+  __syncthreads();
+  const int stride = gridDim.x * blockDim.x;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
+    const unsigned r = log2n > 0 ? __brev((unsigned)k) >> (32 - log2n) : 0u;  // n = 1: the one sample
+    hbr[k] = (float)(H[r] / n);
   }
-  g[k] = (float)(acc / n);
+  const int e = fft_ebits(log2n);
+  for (int k = 0; k + 1 < fft_phases(log2n); ++k) {
+    const int lo = fft_lo(log2n, k), off = fft_tw_offset(log2n, k);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ((1 << e) - 1) << lo; i += stride) {
+      const int slot = (i >> lo) + 1, d = i & ((1 << lo) - 1);
+      double s, c;  // exp(-2 pi i bitrev(slot) d / 2^(lo + e))
+      sincospi(-2.0 * (double)((__brev((unsigned)slot) >> (32 - e)) * (unsigned)d) / (double)(1 << (lo + e)), &s, &c);
+      tws[off + i] = make_float2((float)c, (float)s);
+    }
+  }
+  if (!g) return;
+  for (int k = blockIdx.x; k <= n / 2; k += gridDim.x) {
+    double acc = 0.0;
+    for (int j = threadIdx.x; j < n; j += kTableThreads)
+      acc += H[j] * quarter_cos(quarter, n, (unsigned)j * (unsigned)k);
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) {
+      g[k] = (float)(acc / n);
+      if (k > 0 && k < n - k) g[n - k] = (float)(acc / n);  // even
+    }
+  }
 }
 
 __global__ void twiddle_kernel(int n, float2* tw) {
@@ -105,228 +175,289 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a * conj(b)
   return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
 
-// Shared memory of filter_fft_kernel: per-stage twiddle tables (n - 1
-// float2: 2^lh entries for stage lh at offset 2^lh - 1), then the rows'
-// buffer (P x n float2) from a 16-byte boundary.
-__host__ __device__ constexpr size_t fft_buf_offset(int n) { return (sizeof(float2) * n + 15) / 16 * 16; }
-__host__ __device__ constexpr size_t fft_smem_bytes(int n, int pairs) {
-  return fft_buf_offset(n) + sizeof(float2) * n * pairs;
-}
-
 struct FilterKArgs {
   RowSet rs;
-  int n, log2n, pairs_per_cta;
   long long npairs;
-  const float2* tw;
+  const float2* tws;
   const float* hbr;
 };
 
-// Butterfly passes over the P rows of `buf` (n = 2^L complex samples each).
-// Two radix-2 stages are done per pass on four elements in registers (the
-// same operations in the same order as two separate radix-2 stages, with half
-// the shared-memory round trips and barriers).
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n sub.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
+// a exp(-2 pi i j / 16) (CONJ: its conjugate), j < 8 a constant after unrolling
+template <bool CONJ>
+__device__ __forceinline__ float2 rot16(float2 a, int j) {
+  constexpr float c1 = 0.92387953251128675613f, c2 = 0.70710678118654752440f, c3 = 0.38268343236508977173f;
+  if (j == 0) return a;
+  if (j == 4) return CONJ ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+  const float c[8] = {1.f, c1, c2, c3, 0.f, -c3, -c2, -c1};
+  const float s[8] = {0.f, c3, c2, c1, 1.f, c1, c2, c3};
+  const float2 w = make_float2(c[j], -s[j]);
+  return CONJ ? cmulc(a, w) : cmul(a, w);
+}
+
+// Radix-2 stages over the low Q bits of the register index, decimation in
+// frequency (highest bit first) and its inverse.
+template <int E, int Q>
+__device__ __forceinline__ void dif_regs(float2 (&x)[E]) {
+#pragma unroll
+  for (int b = Q - 1; b >= 0; --b)
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (!(i >> b & 1)) {
+        const float2 u = x[i], v = x[i + (1 << b)];
+        x[i] = cadd(u, v);
+        x[i + (1 << b)] = rot16<false>(csub(u, v), (i & ((1 << b) - 1)) << (3 - b));
+      }
+}
+template <int E, int Q>
+__device__ __forceinline__ void dit_regs(float2 (&x)[E]) {
+#pragma unroll
+  for (int b = 0; b < Q; ++b)
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (!(i >> b & 1)) {
+        const float2 u = x[i], v = rot16<true>(x[i + (1 << b)], (i & ((1 << b) - 1)) << (3 - b));
+        x[i] = cadd(u, v);
+        x[i + (1 << b)] = csub(u, v);
+      }
+}
+
+// Place of sample p in the exchange buffer (linear over XOR). Half a warp of
+// 8-byte accesses is free of bank conflicts when its places differ in the low
+// four bits. A phase's threads step through its low lo index bits and then
+// from bit lo + log2 E on, the last phase's from bit log2 E on; XORing bits
+// 4, 5, 6 (E = 8) or 4 .. 7 (E = 16) into the low four as below makes every
+// one of these patterns a permutation of the 16 bank pairs.
+template <int L>
+__host__ __device__ constexpr int fft_place(int p) {
+  return fft_ebits(L) == 3 ? p ^ ((p >> 3) & 14) ^ ((p >> 6) & 1) : p ^ ((p >> 4) & 15);
+}
+
+// Element I of the phase's twiddles at w0: volatile, so that the table stays
+// in L1 and out of the registers between pairs.
+template <int I>
+__device__ __forceinline__ float2 load_twiddle(const float2* w0) {
+  float2 w;
+  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2 + %3];" : "=f"(w.x), "=f"(w.y) : "l"(w0), "n"(I * (int)sizeof(float2)));
+  return w;
+}
+// x[i] *= twiddle i (CONJ: its conjugate) for i = 1 .. E - 1
+template <int E, int LO, bool CONJ, int I = 1>
+__device__ __forceinline__ void twiddle_regs(float2 (&x)[E], const float2* w0) {
+  if constexpr (I < E) {
+    const float2 w = load_twiddle<((I - 1) << LO)>(w0);
+    x[I] = CONJ ? cmulc(x[I], w) : cmul(x[I], w);
+    twiddle_regs<E, LO, CONJ, I + 1>(x, w0);
+  }
+}
+
+// Forward phases K .. and inverse phases K .. 0 around the last one: the
+// phase's radix-2 stages and twiddles in registers, then the exchange. Every
+// place is written and read by the same thread within a phase, so one barrier
+// between the write and the next phase's read orders an exchange.
+template <int L, int K, int E, class At, class Sync>
+__device__ __forceinline__ void fft_forward(float2 (&x)[E], const float2* tws, int t, At& at, Sync& sync) {
+  if constexpr (K + 1 < fft_phases(L)) {
+    constexpr int LO = fft_lo(L, K);
+    dif_regs<E, fft_ebits(L)>(x);
+    twiddle_regs<E, LO, false>(x, tws + fft_tw_offset(L, K) + (t & ((1 << LO) - 1)));
+#pragma unroll
+    for (int i = 0; i < E; ++i) at(K, i) = x[i];
+    sync();
+#pragma unroll
+    for (int i = 0; i < E; ++i) x[i] = at(K + 1, i);
+    fft_forward<L, K + 1>(x, tws, t, at, sync);
+  }
+}
+template <int L, int K, int E, class At, class Sync>
+__device__ __forceinline__ void fft_inverse(float2 (&x)[E], const float2* tws, int t, At& at, Sync& sync) {
+  if constexpr (K >= 0) {
+    constexpr int LO = fft_lo(L, K);
+#pragma unroll
+    for (int i = 0; i < E; ++i) at(K + 1, i) = x[i];
+    sync();
+#pragma unroll
+    for (int i = 0; i < E; ++i) x[i] = at(K, i);
+    twiddle_regs<E, LO, true>(x, tws + fft_tw_offset(L, K) + (t & ((1 << LO) - 1)));
+    dit_regs<E, fft_ebits(L)>(x);
+    fft_inverse<L, K - 1>(x, tws, t, at, sync);
+  }
+}
+
+// One group of n / E threads filters a pair of rows at a time, grid-stride
+// over the pairs; a block holds as many groups as its size allows. Groups of
+// up to a warp synchronise by warp, larger ones through a named barrier each.
 //
-// Bank conflicts: sample a of the buffer lives at fsw(a), its low four bits
-// XORed with 5 x bits 4-5 of a. A half-warp of 8-byte accesses is
-// conflict-free when its 16 addresses differ in the low four bits; the
-// butterflies touch blk R s + j + r s (j < s, 16 / s consecutive blocks per
-// half-warp for s < 16): for s >= 16 the 16 addresses are one aligned run
-// (the XOR permutes it), for s = 4 (R = 4) bits 2-3 become r ^ (blk & 3), for
-// s = 1 (R = 4, the middle pass) bits 0-1 become r ^ (blk >> 2 & 3); radix-2
-// passes only run at s >= n / 2. Each stage reads its own contiguous twiddle
-// table (stage lh: T[i] = exp(-2 pi i i / 2^(lh + 1)), i < 2^lh), so lanes
-// with consecutive j read consecutive twiddles.
-__device__ __forceinline__ int fsw(int a) { return a ^ (((a >> 4) & 3) * 5); }
-struct FftRows {
-  float2* buf;
-  const float2* tws;  // per-stage tables, stage lh at offset 2^lh - 1
-  int n, L, P;
-  __device__ __forceinline__ const float2* T(int lh) const { return tws + ((1 << lh) - 1); }
-  __device__ __forceinline__ float2& at(int a) const { return buf[fsw(a)]; }
-};
-
-// forward DIF radix-2 stage lh (half-size h = 2^lh)
-__device__ __forceinline__ void fwd_r2(const FftRows& f, int lh) {
-  const int h = 1 << lh, half = f.n >> 1;
-  const float2* T = f.T(lh);
-  for (int b = threadIdx.x; b < f.P * half; b += blockDim.x) {
-    const int p = b >> (f.L - 1), q = b & (half - 1);
-    const int j = q & (h - 1), blk = q >> lh;
-    const int d = p * f.n + (blk << (lh + 1)) + j;
-    const float2 x0 = f.at(d), x1 = f.at(d + h);
-    f.at(d) = make_float2(x0.x + x1.x, x0.y + x1.y);
-    f.at(d + h) = cmul(make_float2(x0.x - x1.x, x0.y - x1.y), T[j]);
-  }
-}
-
-// forward DIF stages lh and lh - 1 (lh >= 1) on blocks of 2^(lh + 1)
-__device__ __forceinline__ void fwd_r4(const FftRows& f, int lh) {
-  const int h = 1 << lh, h2 = h >> 1, quarter = f.n >> 2;
-  const float2 *T = f.T(lh), *T1 = f.T(lh - 1);
-  for (int b = threadIdx.x; b < f.P * quarter; b += blockDim.x) {
-    const int p = b / quarter, q = b - p * quarter;
-    const int j = q & (h2 - 1), blk = q >> (lh - 1);
-    const int d = p * f.n + (blk << (lh + 1)) + j;
-    const float2 e0 = f.at(d), e1 = f.at(d + h2), e2 = f.at(d + h), e3 = f.at(d + h + h2);
-    const float2 t0 = make_float2(e0.x + e2.x, e0.y + e2.y);
-    const float2 t2 = cmul(make_float2(e0.x - e2.x, e0.y - e2.y), T[j]);
-    const float2 t1 = make_float2(e1.x + e3.x, e1.y + e3.y);
-    const float2 t3 = cmul(make_float2(e1.x - e3.x, e1.y - e3.y), T[j + h2]);
-    const float2 w = T1[j];
-    f.at(d) = make_float2(t0.x + t1.x, t0.y + t1.y);
-    f.at(d + h2) = cmul(make_float2(t0.x - t1.x, t0.y - t1.y), w);
-    f.at(d + h) = make_float2(t2.x + t3.x, t2.y + t3.y);
-    f.at(d + h + h2) = cmul(make_float2(t2.x - t3.x, t2.y - t3.y), w);
-  }
-}
-
-// inverse DIT radix-2 stage lh
-__device__ __forceinline__ void inv_r2(const FftRows& f, int lh) {
-  const int h = 1 << lh, half = f.n >> 1;
-  const float2* T = f.T(lh);
-  for (int b = threadIdx.x; b < f.P * half; b += blockDim.x) {
-    const int p = b >> (f.L - 1), q = b & (half - 1);
-    const int j = q & (h - 1), blk = q >> lh;
-    const int d = p * f.n + (blk << (lh + 1)) + j;
-    const float2 x0 = f.at(d);
-    const float2 x1 = cmulc(f.at(d + h), T[j]);
-    f.at(d) = make_float2(x0.x + x1.x, x0.y + x1.y);
-    f.at(d + h) = make_float2(x0.x - x1.x, x0.y - x1.y);
-  }
-}
-
-// inverse DIT stages lh and lh + 1 on blocks of 2^(lh + 2)
-__device__ __forceinline__ void inv_r4(const FftRows& f, int lh) {
-  const int h = 1 << lh, quarter = f.n >> 2;
-  const float2 *T = f.T(lh), *T1 = f.T(lh + 1);
-  for (int b = threadIdx.x; b < f.P * quarter; b += blockDim.x) {
-    const int p = b / quarter, q = b - p * quarter;
-    const int j = q & (h - 1), blk = q >> lh;
-    const int d = p * f.n + (blk << (lh + 2)) + j;
-    const float2 e0 = f.at(d), e1 = f.at(d + h), e2 = f.at(d + 2 * h), e3 = f.at(d + 3 * h);
-    const float2 w = T[j];
-    const float2 x1 = cmulc(e1, w), x3 = cmulc(e3, w);
-    const float2 a0 = make_float2(e0.x + x1.x, e0.y + x1.y), a1 = make_float2(e0.x - x1.x, e0.y - x1.y);
-    const float2 a2 = make_float2(e2.x + x3.x, e2.y + x3.y), a3 = make_float2(e2.x - x3.x, e2.y - x3.y);
-    const float2 y = cmulc(a2, T1[j]), z = cmulc(a3, T1[j + h]);
-    f.at(d) = make_float2(a0.x + y.x, a0.y + y.y);
-    f.at(d + 2 * h) = make_float2(a0.x - y.x, a0.y - y.y);
-    f.at(d + h) = make_float2(a1.x + z.x, a1.y + z.y);
-    f.at(d + 3 * h) = make_float2(a1.x - z.x, a1.y - z.y);
-  }
-}
-
-// The last two forward stages (1, 0), the response H (bit-reversed, / n) and
-// the first two inverse stages (0, 1) of each block of four, in registers.
-__device__ __forceinline__ void middle_r4(const FftRows& f, const float* hb) {
-  const int quarter = f.n >> 2;
-  const float2 w1 = f.T(1)[1], w0 = f.T(0)[0];
-  for (int b = threadIdx.x; b < f.P * quarter; b += blockDim.x) {
-    const int p = b / quarter, q = b - p * quarter;
-    const int d = p * f.n + 4 * q;
-    const float4 h4 = __ldg(reinterpret_cast<const float4*>(hb) + q);  // the response from global memory (L1)
-    const float hq[4] = {h4.x, h4.y, h4.z, h4.w};
-    const float2 e0 = f.at(d), e1 = f.at(d + 1), e2 = f.at(d + 2), e3 = f.at(d + 3);
-    // forward stage 1 (pairs 0-2 with w0, 1-3 with w1), stage 0 (pairs 0-1, 2-3 with w0)
-    const float2 t0 = make_float2(e0.x + e2.x, e0.y + e2.y);
-    const float2 t2 = cmul(make_float2(e0.x - e2.x, e0.y - e2.y), w0);
-    const float2 t1 = make_float2(e1.x + e3.x, e1.y + e3.y);
-    const float2 t3 = cmul(make_float2(e1.x - e3.x, e1.y - e3.y), w1);
-    float2 s0 = make_float2(t0.x + t1.x, t0.y + t1.y);
-    float2 s1 = cmul(make_float2(t0.x - t1.x, t0.y - t1.y), w0);
-    float2 s2 = make_float2(t2.x + t3.x, t2.y + t3.y);
-    float2 s3 = cmul(make_float2(t2.x - t3.x, t2.y - t3.y), w0);
-    s0 = make_float2(s0.x * hq[0], s0.y * hq[0]);
-    s1 = make_float2(s1.x * hq[1], s1.y * hq[1]);
-    s2 = make_float2(s2.x * hq[2], s2.y * hq[2]);
-    s3 = make_float2(s3.x * hq[3], s3.y * hq[3]);
-    // inverse stage 0 (pairs 0-1, 2-3 with w0), stage 1 (pairs 0-2 with w0, 1-3 with w1)
-    const float2 x1 = cmulc(s1, w0), x3 = cmulc(s3, w0);
-    const float2 a0 = make_float2(s0.x + x1.x, s0.y + x1.y), a1 = make_float2(s0.x - x1.x, s0.y - x1.y);
-    const float2 a2 = make_float2(s2.x + x3.x, s2.y + x3.y), a3 = make_float2(s2.x - x3.x, s2.y - x3.y);
-    const float2 y = cmulc(a2, w0), z = cmulc(a3, w1);
-    f.at(d) = make_float2(a0.x + y.x, a0.y + y.y);
-    f.at(d + 2) = make_float2(a0.x - y.x, a0.y - y.y);
-    f.at(d + 1) = make_float2(a1.x + z.x, a1.y + z.y);
-    f.at(d + 3) = make_float2(a1.x - z.x, a1.y - z.y);
-  }
-}
-
-// One CTA filters `pairs_per_cta` row pairs per iteration, grid-stride.
-__global__ void __launch_bounds__(256) filter_fft_kernel(FilterKArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = a.n;
-  float2* tws = reinterpret_cast<float2*>(smem_raw);
-  float2* buf = reinterpret_cast<float2*>(smem_raw + fft_buf_offset(n));
-  // stage lh's table from the n / 2 twiddles exp(-2 pi i k / n)
-  for (int i = threadIdx.x; i < n - 1; i += blockDim.x) {
-    const int lh = 31 - __clz(i + 1), k = i + 1 - (1 << lh);
-    tws[i] = a.tw[k << (a.log2n - 1 - lh)];
-  }
-  const float* hb = a.hbr;
+// Bound: the load / store unit (78-83% busy: exchanges, twiddles and the two
+// half-written elements of a pair). Measured into FP32 pairs, before = radix-4
+// passes through shared memory with block barriers: 138240 rows of 384 (n =
+// 512) 819 -> 211 us (637 MB: 3.0 TB/s), 138240 rows of 768 (n = 1024) 1628 ->
+// 493 us, 92160 rows of 1536 (n = 2048) 2288 -> 646 us. Four blocks a SM at 64
+// registers spill and are 1-14% slower, E = 16 for n = 1024, 2048 1.4 times
+// slower, the twiddles held in registers (one block a SM) 2 times.
+template <int L>
+__global__ void __launch_bounds__(256, fft_ebits(L) == 4 ? 2 : 3) filter_fft_kernel(const FilterKArgs a) {
+  constexpr int EB = fft_ebits(L), E = 1 << EB, N = 1 << L, T = N / E, NP = fft_phases(L);
+  constexpr int REM = L - (NP - 1) * EB;  // index bits of the last phase
+  extern __shared__ __align__(16) float2 fft_buf[];
+  const int grp = threadIdx.x / T, t = threadIdx.x % T;
   const RowSet& rs = a.rs;
-  const int P = a.pairs_per_cta;
-  const FftRows f{buf, tws, n, a.log2n, P};
-  const long long ngroups = (a.npairs + P - 1) / P;
-  for (long long grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
-    __syncthreads();
-    // load P pairs: real part row 2p, imaginary part row 2p + 1, zero padded
-    for (int idx = threadIdx.x; idx < P * n; idx += blockDim.x) {
-      int p = idx / n, i = idx - p * n;
-      long long pr = grp * P + p;
-      float re = 0.f, im = 0.f;
-      if (pr < a.npairs && i < rs.m) {
-        long long r0 = 2 * pr;
-        re = load_pre(rs, r0, i);
-        if (r0 + 1 < rs.rows) im = load_pre(rs, r0 + 1, i);
+  const unsigned mask = T >= 32 ? 0xffffffffu : ((1u << (T & 31)) - 1u) << ((threadIdx.x & 31) / T * T);
+  auto sync = [&]() {
+    if constexpr (T <= 32) __syncwarp(mask);
+    else asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(T) : "memory");
+  };
+  float h[E];  // response at this thread's samples of the last phase: E t .. E t + E - 1
+#pragma unroll
+  for (int i = 0; i < E; ++i) h[i] = a.hbr[E * t + i];
+  // Slot i of phase k holds sample (t >> lo << (lo + EB)) | (i << lo) | (t mod
+  // 2^lo), of the last phase E t + i; off[k] is slot 0's place in bytes, and
+  // the place being linear, slot i's is off[k] ^ place(i << lo).
+  uint32_t off[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    const int lo = k == NP - 1 ? 0 : fft_lo(L, k);
+    off[k] = ((uint32_t)grp << (L + 3)) | (uint32_t)(fft_place<L>((t >> lo << (lo + EB)) | (t & ((1 << lo) - 1))) * 8);
+  }
+  auto at = [&](int k, int i) -> float2& {
+    const int lo = k == NP - 1 ? 0 : fft_lo(L, k);
+    return *reinterpret_cast<float2*>(reinterpret_cast<char*>(fft_buf) + (off[k] ^ (uint32_t)(fft_place<L>(i << lo) * 8)));
+  };
+  const int groups = blockDim.x / T;
+  for (long long pr = (long long)blockIdx.x * groups + grp; pr < a.npairs; pr += (long long)gridDim.x * groups) {
+    const long long r0 = 2 * pr;
+    const bool two = r0 + 1 < rs.rows;
+    const float* s0 = rs.data + r0 * rs.pitch + t;
+    const float* s1 = two ? s0 + rs.pitch : s0;
+    const int left = rs.m - t;  // sample t + i T exists for i T < left
+    float2 x[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {  // real part row r0, imaginary part row r0 + 1, zero padded
+      x[i] = make_float2(0.f, 0.f);
+      if (i * T < left) x[i] = make_float2(s0[i * T], two ? s1[i * T] : 0.f);
+    }
+    if (rs.log_norm) {
+#pragma unroll
+      for (int i = 0; i < E; ++i)
+        if (i * T < left) {
+          x[i].x = -logf(fmaxf(x[i].x, 1e-30f * rs.log_base) / rs.log_base);
+          if (two) x[i].y = -logf(fmaxf(x[i].y, 1e-30f * rs.log_base) / rs.log_base);
+        }
+    }
+    if (rs.weight) {
+      const long long rb = two ? r0 + 1 : r0;
+      const int iv0 = rs.sinogram ? (int)(r0 / rs.n_views) : (int)(r0 % rs.n_v);
+      const int iv1 = rs.sinogram ? (int)(rb / rs.n_views) : (int)(rb % rs.n_v);
+      const float v0 = (iv0 + 0.5f - 0.5f * rs.n_v + rs.w_voff) * rs.w_dv;
+      const float v1 = (iv1 + 0.5f - 0.5f * rs.n_v + rs.w_voff) * rs.w_dv;
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const float u = (t + i * T + 0.5f - 0.5f * rs.m) * rs.w_du;
+        const float uu = rs.w_sdd * rs.w_sdd + u * u;
+        x[i].x *= rs.w_sdd * rsqrtf(uu + v0 * v0);
+        x[i].y *= rs.w_sdd * rsqrtf(uu + v1 * v1);
       }
-      f.at(idx) = make_float2(re, im);
     }
-    __syncthreads();
-    // forward DIF (natural order in, bit-reversed out): an odd stage first,
-    // then pairs of stages down to stage 2
-    int lh = f.L - 1;
-    if (f.L & 1) {
-      fwd_r2(f, lh--);
-      __syncthreads();
-    }
-    for (; lh >= 3; lh -= 2) {
-      fwd_r4(f, lh);
-      __syncthreads();
-    }
-    int next;  // first inverse stage still to do
-    if (lh == 1) {
-      middle_r4(f, hb);
-      next = 2;
-    } else {  // n <= 2: the response on its own
-      for (int idx = threadIdx.x; idx < P * n; idx += blockDim.x) {
-        const float hv = hb[idx & (n - 1)];
-        const float2 x = f.at(idx);
-        f.at(idx) = make_float2(x.x * hv, x.y * hv);
+    fft_forward<L, 0>(x, a.tws, t, at, sync);
+    dif_regs<E, REM>(x);
+#pragma unroll
+    for (int i = 0; i < E; ++i) x[i] = make_float2(x[i].x * h[i], x[i].y * h[i]);
+    dit_regs<E, REM>(x);
+    fft_inverse<L, NP - 2>(x, a.tws, t, at, sync);
+    const int v0 = rs.out_layout == kLayoutPair32 ? (int)(r0 % rs.n_v) : 0;
+    if (rs.out_layout == kLayoutPair32 && !rs.sinogram && two && v0 + 1 < rs.n_v) {
+      // rows v0, v0 + 1 of one view: element v0 + 1 whole, the near halves of its neighbours
+      float2* o0 = static_cast<float2*>(rs.out) + pair_row(rs, (int)(r0 / rs.n_v), v0) * rs.out_pitch + t;
+      float2 *o1 = o0 + rs.out_pitch, *o2 = o1 + rs.out_pitch;
+      const bool first = v0 == 0, last = v0 + 1 == rs.n_v - 1;
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        if (i * T >= left) continue;
+        o1[i * T] = x[i];
+        o0[i * T].y = x[i].x;
+        o2[i * T].x = x[i].y;
+        if (first) o0[i * T].x = 0.f;
+        if (last) o2[i * T].y = 0.f;
       }
-      next = 0;
-    }
-    __syncthreads();
-    // inverse DIT (bit-reversed in, natural order out): pairs of stages, then an odd last one
-    for (; next + 1 < f.L; next += 2) {
-      inv_r4(f, next);
-      __syncthreads();
-    }
-    if (next < f.L) {
-      inv_r2(f, next);
-      __syncthreads();
-    }
-    // store
-    for (int idx = threadIdx.x; idx < P * n; idx += blockDim.x) {
-      int p = idx / n, i = idx - p * n;
-      long long pr = grp * P + p;
-      if (pr >= a.npairs || i >= rs.m) continue;
-      float2 y = f.at(idx);
-      long long r0 = 2 * pr;
-      store_row_sample(rs, r0, i, y.x);
-      if (r0 + 1 < rs.rows) store_row_sample(rs, r0 + 1, i, y.y);
+    } else if (rs.out_layout == kLayoutRaw32) {
+      float* d0 = rs.data + r0 * rs.pitch + t;
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        if (i * T >= left) continue;
+        d0[i * T] = x[i].x;
+        if (two) d0[rs.pitch + i * T] = x[i].y;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const int c = t + i * T;
+        if (c >= rs.m) continue;
+        store_row_sample(rs, r0, c, x[i].x);
+        if (two) store_row_sample(rs, r0 + 1, c, x[i].y);
+      }
     }
   }
+}
+
+template <int L>
+cudaError_t launch_fft_cfg(const FilterKArgs& a, int num_sms, cudaStream_t stream) {
+  constexpr int T = (1 << L) >> fft_ebits(L), MAXG = 256 / T;
+  // few pairs: a group a block, so that they spread over the SMs
+  int groups = (int)std::max<long long>(1, std::min<long long>(MAXG, a.npairs / num_sms));
+  if (T * groups < 32) groups = std::min(MAXG, 32 / T);
+  const size_t smem = fft_phases(L) > 1 ? sizeof(float2) * ((size_t)groups << L) : 0;
+  auto kern = filter_fft_kernel<L>;
+  int per_sm = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T * groups, smem);
+  if (e != cudaSuccess) return e;
+  const long long blocks = (a.npairs + groups - 1) / groups;
+  kern<<<(unsigned)std::min<long long>(blocks, (long long)num_sms * std::max(1, per_sm)), T * groups, smem, stream>>>(a);
+  return cudaGetLastError();
+}
+
+// The filter kernel of padded length n = 2^log2n, n <= 4096.
+cudaError_t launch_fft(const FilterKArgs& a, int log2n, int num_sms, cudaStream_t stream) {
+  switch (log2n) {
+    case 0: return launch_fft_cfg<0>(a, num_sms, stream);
+    case 1: return launch_fft_cfg<1>(a, num_sms, stream);
+    case 2: return launch_fft_cfg<2>(a, num_sms, stream);
+    case 3: return launch_fft_cfg<3>(a, num_sms, stream);
+    case 4: return launch_fft_cfg<4>(a, num_sms, stream);
+    case 5: return launch_fft_cfg<5>(a, num_sms, stream);
+    case 6: return launch_fft_cfg<6>(a, num_sms, stream);
+    case 7: return launch_fft_cfg<7>(a, num_sms, stream);
+    case 8: return launch_fft_cfg<8>(a, num_sms, stream);
+    case 9: return launch_fft_cfg<9>(a, num_sms, stream);
+    case 10: return launch_fft_cfg<10>(a, num_sms, stream);
+    case 11: return launch_fft_cfg<11>(a, num_sms, stream);
+    case 12: return launch_fft_cfg<12>(a, num_sms, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+// The filter tables for n: the response and the tables that follow from it
+// (g may be nullptr).
+cudaError_t launch_tables(int n, int log2n, int filter, double* H, float* hbr, float2* tws, float* g,
+                          cudaStream_t stream) {
+  const size_t smem = sizeof(double) * (n / 4 + 1);
+  const int blocks = std::min(n / 2 + 1, 1024);
+  response_kernel<<<blocks, kTableThreads, smem, stream>>>(n, filter, H);
+  tables_kernel<<<blocks, kTableThreads, smem, stream>>>(n, log2n, H, hbr, tws, g);
+  return cudaGetLastError();
 }
 
 __global__ void elementwise_pre_kernel(RowSet rs) {
@@ -635,15 +766,16 @@ int ensure_filter_tables(fbp_context* ctx, int n, int filter) {
   if (filter < 0 || filter > FBP_FILTER_RAMP_SAMPLED)
     return set_error(ctx, FBP_ERR_INVALID_ARGUMENT, "unknown filter type");
   if (n > t.cap) {  // grow only: a context serving many row lengths stops allocating
-    cudaFree(t.twiddle);
+    cudaFree(t.tws);
     cudaFree(t.hbr);
     cudaFree(t.kernel);
-    t.twiddle = nullptr;
+    t.tws = nullptr;
     t.hbr = nullptr;
     t.kernel = nullptr;
     t.n = 0;
     t.cap = 0;
-    if (cuda_check(ctx, cudaMalloc(&t.twiddle, sizeof(float2) * (n / 2 + 1)), "cudaMalloc(twiddle)") ||
+    // at most (E - 1) / E n entries for the first phase and 1 / E of that for each further one
+    if (cuda_check(ctx, cudaMalloc(&t.tws, sizeof(float2) * (n + 8)), "cudaMalloc(twiddles)") ||
         cuda_check(ctx, cudaMalloc(&t.hbr, sizeof(float) * n), "cudaMalloc(hbr)") ||
         cuda_check(ctx, cudaMalloc(&t.kernel, sizeof(float) * n), "cudaMalloc(kernel)"))
       return FBP_ERR_OUT_OF_MEMORY;
@@ -651,11 +783,10 @@ int ensure_filter_tables(fbp_context* ctx, int n, int filter) {
   }
   double* H = static_cast<double*>(scratch(ctx, sizeof(double) * n));
   if (!H) return FBP_ERR_OUT_OF_MEMORY;
-  int blocks = (n + 127) / 128;
-  response_kernel<<<blocks, 128, 0, ctx->stream>>>(n, filter, H);
-  tables_kernel<<<blocks, 128, 0, ctx->stream>>>(n, ilog2(n), H, t.hbr, t.twiddle, t.kernel);
-  ctx->launches += 1;  // two launches above
-  if (int rc = launched(ctx, "filter tables")) return rc;
+  if (int rc = cuda_check(ctx, launch_tables(n, ilog2(n), filter, H, t.hbr, t.tws, t.kernel, ctx->stream),
+                          "filter tables"))
+    return rc;
+  ctx->launches += 2;
   t.n = n;
   t.filter = filter;
   return FBP_OK;
@@ -667,19 +798,12 @@ int launch_filter_fft(fbp_context* ctx, const RowSet& rs, int n) {
   if (rs.rows == 0) return FBP_OK;
   FilterKArgs a;
   a.rs = rs;
-  a.n = n;
-  a.log2n = ilog2(n);
-  a.pairs_per_cta = std::max(1, std::min(8, 4096 / n));
   a.npairs = (rs.rows + 1) / 2;
-  a.tw = ctx->ftab.twiddle;
+  a.tws = ctx->ftab.tws;
   a.hbr = ctx->ftab.hbr;
-  size_t smem = fft_smem_bytes(n, a.pairs_per_cta);
-  // per device and process-wide: set on every launch (same value from every context)
-  cudaFuncSetAttribute(filter_fft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  long long groups = (a.npairs + a.pairs_per_cta - 1) / a.pairs_per_cta;
-  int grid = (int)std::min<long long>(groups, (long long)ctx->num_sms * 4);
-  filter_fft_kernel<<<grid, 256, smem, ctx->stream>>>(a);
-  return launched(ctx, "filter_fft_kernel");
+  if (int rc = cuda_check(ctx, launch_fft(a, ilog2(n), ctx->num_sms, ctx->stream), "filter_fft_kernel")) return rc;
+  ctx->launches++;
+  return FBP_OK;
 }
 
 int launch_elementwise_pre(fbp_context* ctx, const RowSet& rs) {
@@ -790,11 +914,10 @@ int launch_unpack_rows(fbp_context* ctx, const Stack& s, size_t row0, size_t nro
 
 namespace {
 constexpr int kNoAllocMaxN = 4096;
-constexpr size_t kNoAllocH = 0;                                         // double[4096]
-constexpr size_t kNoAllocTw = kNoAllocH + sizeof(double) * kNoAllocMaxN;  // float2[2048]
-constexpr size_t kNoAllocHbr = kNoAllocTw + sizeof(float2) * (kNoAllocMaxN / 2);  // float[4096]
-constexpr size_t kNoAllocG = kNoAllocHbr + sizeof(float) * kNoAllocMaxN;           // float[4096]
-constexpr size_t kNoAllocBytes = kNoAllocG + sizeof(float) * kNoAllocMaxN;         // 80 KiB
+constexpr size_t kNoAllocH = 0;                                           // double[4096]
+constexpr size_t kNoAllocTw = kNoAllocH + sizeof(double) * kNoAllocMaxN;  // float2[4096]
+constexpr size_t kNoAllocHbr = kNoAllocTw + sizeof(float2) * kNoAllocMaxN;  // float[4096]
+constexpr size_t kNoAllocBytes = kNoAllocHbr + sizeof(float) * kNoAllocMaxN;  // 80 KiB
 }  // namespace
 
 static __device__ __align__(256) unsigned char fbp_noalloc_filter_scratch[kNoAllocBytes];
@@ -837,19 +960,15 @@ extern "C" int fbp2d_filter_sinogram_noalloc(float* sinogram, int bins, int view
   if (e != cudaSuccess) return cuda_check(nullptr, e, "cudaGetSymbolAddress(filter scratch)");
   unsigned char* b = static_cast<unsigned char*>(base);
   double* H = reinterpret_cast<double*>(b + kNoAllocH);
-  float2* tw = reinterpret_cast<float2*>(b + kNoAllocTw);
+  float2* tws = reinterpret_cast<float2*>(b + kNoAllocTw);
   float* hbr = reinterpret_cast<float*>(b + kNoAllocHbr);
-  float* g = reinterpret_cast<float*>(b + kNoAllocG);
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   int dev = 0, sms = 148;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_check(nullptr, e, "cudaGetDevice");
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return cuda_check(nullptr, e, "cudaDeviceGetAttribute(multiprocessor count)");
 
-  const int blocks = (n + 127) / 128;
-  response_kernel<<<blocks, 128, 0, stream>>>(n, filter_type, H);
-  tables_kernel<<<blocks, 128, 0, stream>>>(n, ilog2(n), H, hbr, tw, g);
-  if ((e = cudaGetLastError()) != cudaSuccess)
+  if ((e = launch_tables(n, ilog2(n), filter_type, H, hbr, tws, nullptr, stream)) != cudaSuccess)
     return cuda_check(nullptr, e, "fbp2d_filter_sinogram_noalloc: filter tables");
 
   RowSet rs{};
@@ -868,18 +987,8 @@ extern "C" int fbp2d_filter_sinogram_noalloc(float* sinogram, int bins, int view
   }
   FilterKArgs a;
   a.rs = rs;
-  a.n = n;
-  a.log2n = ilog2(n);
-  a.pairs_per_cta = std::max(1, std::min(8, 4096 / n));
   a.npairs = (rs.rows + 1) / 2;
-  a.tw = tw;
+  a.tws = tws;
   a.hbr = hbr;
-  const size_t smem = fft_smem_bytes(n, a.pairs_per_cta);
-  if ((e = cudaFuncSetAttribute(filter_fft_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024)) !=
-      cudaSuccess)
-    return cuda_check(nullptr, e, "fbp2d_filter_sinogram_noalloc: shared memory attribute");
-  const long long groups = (a.npairs + a.pairs_per_cta - 1) / a.pairs_per_cta;
-  const int grid = (int)std::min<long long>(groups, (long long)sms * 4);
-  filter_fft_kernel<<<grid, 256, smem, stream>>>(a);
-  return cuda_check(nullptr, cudaGetLastError(), "fbp2d_filter_sinogram_noalloc: filter_fft_kernel");
+  return cuda_check(nullptr, launch_fft(a, ilog2(n), sms, stream), "fbp2d_filter_sinogram_noalloc: filter_fft_kernel");
 }

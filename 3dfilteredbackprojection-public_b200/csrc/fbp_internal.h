@@ -89,7 +89,7 @@ struct Stack {
 struct FilterTables {
   int n = 0, filter = -1;
   int cap = 0;                // entries allocated (grow only: no cudaFree between jobs)
-  float2* twiddle = nullptr;  // n/2 entries exp(-2 pi i k / n)
+  float2* tws = nullptr;      // twiddles of the register FFT's phases (fbp_filter.cu)
   float* hbr = nullptr;       // n entries H[bitrev(k)] / n
   float* kernel = nullptr;    // n entries: spatial kernel g = IDFT(H) (circular)
 };

@@ -79,3 +79,54 @@ def test_bp2d_view_sets_and_sizes(fbp, oracle, kind, nx, nz, views, bins, turns)
              sdd=float(np.float32(sod)) + float(np.float32(sdd - sod)))
     ref = (oracle.bp_fan2d if kind == "fan" else oracle.bp_parallel2d)(sino.astype(np.float64), c)
     assert relative_rmse(img, ref) < TOL_BP2D
+
+
+# FP32 transform of n <= 4096 samples and its inverse: rounding 6e-8 per stage,
+# independent over 2 log2 n = 24 stages (3e-7), on white noise whose filtered
+# rows are of its own scale.
+TOL_ROWS = 1e-6
+
+
+@pytest.mark.parametrize("rows", [1, 2, 7, 700])
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 9, 17, 33, 64, 65, 128, 129, 257, 511, 513, 1000, 1025, 2049, 4096])
+def test_fft_filter_every_length(fbp, oracle, m, rows):
+    """Each register-phase split of the row transform, padded and unpadded
+    rows, odd row counts (an unpaired last row), fewer and more pairs than the
+    GPU has SMs; the allocation-free entry point gives the same bits."""
+    import torch
+    x = np.random.default_rng(m * 10 + rows).standard_normal((rows, m)).astype(np.float32)
+    filt = m % 4
+    f2 = fbp.FBP2D(0)
+    got = f2.apply_filter(x.copy(), filt)
+    ref = oracle.filter_rows(x.astype(np.float64), filt)
+    assert relative_rmse(got, ref) < TOL_ROWS
+    d = torch.as_tensor(x, device="cuda")
+    assert fbp.library().fbp2d_filter_sinogram_noalloc(d.data_ptr(), m, rows, filt, 0.0, 0.0, 0, None) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(d.cpu().numpy(), got)
+
+
+@pytest.mark.parametrize("layout", ["projections", "sinograms"])
+@pytest.mark.parametrize("u,v,n", [(70, 1, 5), (70, 2, 3), (130, 3, 5), (301, 4, 6), (9, 5, 7), (600, 7, 3)])
+def test_fft_filter_pair_layout(fbp, oracle, layout, u, v, n):
+    """Rows filtered into the pair layout (a pair inside one view, across two
+    views, at a view's edges) and back, with log and weight in the load."""
+    rng = np.random.default_rng(u)
+    counts = (rng.random((n, v, u)) * 900 + 100).astype(np.float32)
+    s = fbp.FBP3D(0)
+    sod, odd, width = 200.0, 100.0, 150.0
+    if layout == "projections":
+        s.upload_projections(counts)
+        s.log_normalize_projections(1000.0)
+        s.apply_fdk_weights_to_projections(sod, odd, width)
+        s.apply_filter_to_projections(1)
+        got = s.download_projections()
+    else:
+        s.upload_sinograms(np.ascontiguousarray(counts.transpose(1, 0, 2)))
+        s.log_normalize_sinograms(1000.0)
+        s.apply_fdk_weights_to_sinograms(sod, odd, width)
+        s.apply_filter_to_sinograms(1)
+        got = s.download_sinograms(np.empty((v, n, u), np.float32)).transpose(1, 0, 2)
+    s.ctx.close()
+    p = oracle.fdk_weight(oracle.log_normalize(counts.astype(np.float64), 1000.0), sod + odd, width / u, width / u)
+    assert relative_rmse(got, oracle.filter_rows(p, 1)) < TOL_ROWS
