@@ -116,8 +116,12 @@ size_t estimate_bytes(const fbp_request& r) {
     const size_t split = std::min<size_t>((size_t)r.det_rows * r.views, 65536) * (cols4 + 64) * 4;
     return stack + packed + vol + split + (64u << 20);
   }
-  if (r.kind == FBP_JOB_FAN2D || r.kind == FBP_JOB_PARALLEL2D)
-    return cols4 * r.views * 4 * 3 + (size_t)r.vol_h * r.vol_h * 4 + (16u << 20);
+  if (r.kind == FBP_JOB_FAN2D || r.kind == FBP_JOB_PARALLEL2D) {
+    // rows, staged rows, and the larger of the split rows and the
+    // backprojector's packed ones (parallel beam: with their mirror images)
+    const size_t packed = (cols4 + 256) * r.views * 4 * (r.kind == FBP_JOB_PARALLEL2D ? 2 : 1);
+    return cols4 * r.views * 4 * 2 + packed + (size_t)r.vol_h * r.vol_h * 4 + (16u << 20);
+  }
   return 0;
 }
 
