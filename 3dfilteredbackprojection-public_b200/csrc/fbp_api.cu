@@ -75,12 +75,15 @@ cudaMemcpyKind kind_of(bool src_dev, bool dst_dev) {
   return cudaMemcpyHostToHost;
 }
 
-// Device error word -> status (and reset).
+// Waits for ctx's stream, then device error word -> status (and reset). The
+// word comes back through a pinned one behind the stream's work, so a call
+// waits once (a copy to pageable memory waits by itself, and a wait before it
+// makes three).
 int check_device_error(fbp_context* ctx) {
-  int h = 0;
-  FBP_TRY(fbp::cuda_check(ctx, cudaMemcpyAsync(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream),
+  FBP_TRY(fbp::cuda_check(ctx, cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream),
                           "error word readback"));
   FBP_TRY(fbp::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize"));
+  const int h = *ctx->h_err;
   if (h == fbp::kDevOk) return FBP_OK;
   cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream);
   cudaStreamSynchronize(ctx->stream);
@@ -98,9 +101,7 @@ int check_device_error(fbp_context* ctx) {
 }
 
 int sync_host(fbp_context* ctx, bool host_involved) {
-  if (!host_involved) return FBP_OK;
-  FBP_TRY(fbp::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize"));
-  return check_device_error(ctx);
+  return host_involved ? check_device_error(ctx) : FBP_OK;
 }
 
 void free_stack(Stack& s) {
@@ -680,10 +681,12 @@ int fbp_create(fbp_context** out, int device) {
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess ||
       cudaMemset(ctx->d_err, 0, sizeof(int)) != cudaSuccess ||
+      cudaMallocHost(&ctx->h_err, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&ctx->d_minmax, 2 * sizeof(int)) != cudaSuccess) {
     g_thread_error = std::string("context setup failed: ") + cudaGetErrorString(cudaGetLastError());
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     cudaFree(ctx->d_err);
+    cudaFreeHost(ctx->h_err);
     cudaFree(ctx->d_minmax);
     delete ctx;
     return FBP_ERR_CUDA;
@@ -713,7 +716,7 @@ int fbp_destroy(fbp_context* ctx) {
     cudaFree(ctx->ftab.kernel);
     cudaFree(ctx->ttab.th);
     cudaFree(ctx->d_scratch);
-    cudaFreeHost(ctx->h_pinned);
+    cudaFreeHost(ctx->h_err);
     cudaFree(ctx->d_batch);
     cudaFreeHost(ctx->h_batch);
     if (ctx->ev_batch_copy) cudaEventDestroy(ctx->ev_batch_copy);
@@ -748,7 +751,6 @@ int fbp_set_stream(fbp_context* ctx, void* stream) {
 
 int fbp_synchronize(fbp_context* ctx) {
   FBP_CTX(ctx);
-  FBP_TRY(fbp::cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize"));
   return check_device_error(ctx);
 }
 

@@ -420,12 +420,9 @@ cudaError_t launch_fft_cfg(const FilterKArgs& a, int num_sms, cudaStream_t strea
   int groups = (int)std::max<long long>(1, std::min<long long>(MAXG, a.npairs / num_sms));
   if (T * groups < 32) groups = std::min(MAXG, 32 / T);
   const size_t smem = fft_phases(L) > 1 ? sizeof(float2) * ((size_t)groups << L) : 0;
-  auto kern = filter_fft_kernel<L>;
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T * groups, smem);
-  if (e != cudaSuccess) return e;
+  const int per_sm = (fft_ebits(L) == 4 ? 2 : 3) * 256 / (T * groups);  // blocks resident (the launch bounds)
   const long long blocks = (a.npairs + groups - 1) / groups;
-  kern<<<(unsigned)std::min<long long>(blocks, (long long)num_sms * std::max(1, per_sm)), T * groups, smem, stream>>>(a);
+  filter_fft_kernel<L><<<(unsigned)std::min<long long>(blocks, (long long)num_sms * per_sm), T * groups, smem, stream>>>(a);
   return cudaGetLastError();
 }
 

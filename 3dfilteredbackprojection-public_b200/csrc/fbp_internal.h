@@ -100,6 +100,8 @@ struct ToeplitzTables {
   int m = 0, n = 0, filter = -1;
   void* th = nullptr;  // 2 * m * kp BF16 values, then 9 x m FP32 columns T P_j (row baseline basis)
   size_t cap = 0;      // bytes allocated at th (grow only)
+  float ginv[81] = {0};  // inverse Gram matrix of the row baseline basis for rows of gm samples
+  int gm = 0;
 };
 
 }  // namespace fbp
@@ -153,6 +155,7 @@ struct fbp_context {
   fbp::Stack sino;
 
   int* d_err = nullptr;          // device error word
+  int* h_err = nullptr;          // pinned word it is read back into
   int* d_minmax = nullptr;       // volume min / max as order-preserving int keys
   bool minmax_valid = false;     // d_minmax describes the current volume
   double2* d_trig = nullptr;     // per-view (cos, sin) in FP64
@@ -166,8 +169,6 @@ struct fbp_context {
   fbp::ToeplitzTables ttab;
   void* d_scratch = nullptr;     // generic scratch (row shifts, Toeplitz operands)
   size_t scratch_bytes = 0;
-  void* h_pinned = nullptr;      // small pinned staging for per-call tables
-  size_t h_pinned_bytes = 0;
 
   // cached backprojection plans: the largest detector window of any
   // (tile, view) for a geometry (samples, rows including row v + 1); several,

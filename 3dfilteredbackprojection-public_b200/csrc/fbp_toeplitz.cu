@@ -496,7 +496,14 @@ int launch_filter_toeplitz(fbp_context* ctx, const RowSet& rs, int n, int filter
   if (!sp) return FBP_ERR_OUT_OF_MEMORY;
   __nv_bfloat16* xh = reinterpret_cast<__nv_bfloat16*>(sp);
   __nv_bfloat16* xl = reinterpret_cast<__nv_bfloat16*>(sp + sbytes);
-  const BasisGram gram = basis_gram(m);
+  BasisGram gram;
+  if (t.gm != m) {
+    gram = basis_gram(m);
+    std::copy(gram.ginv, gram.ginv + kBasis * kBasis, t.ginv);
+    t.gm = m;
+  } else {
+    std::copy(t.ginv, t.ginv + kBasis * kBasis, gram.ginv);
+  }
   const size_t stage_smem = kp <= 2048 ? sizeof(float) * 8 * (size_t)kp : 0;  // 8 warps x one padded row
   if (stage_smem) {
     // the attribute is process-wide and other contexts launch with other row
