@@ -169,13 +169,10 @@ int flush_pending(fbp_context* ctx, Stack& s) {
   return FBP_OK;
 }
 
-// Bring the content back into the f32 rows (from the filtered buffer) and
-// apply anything pending.
+// The rows are about to be read or replaced: apply anything pending; what
+// follows is no longer the FP32 form's filter output alone.
 int materialize_f32(fbp_context* ctx, Stack& s) {
-  if (s.filtered) {
-    FBP_TRY(fbp::launch_unpack_rows(ctx, s, 0, s.rows(), s.f32, s.pitch));
-    s.filtered = false;
-  }
+  s.filtered = false;
   return flush_pending(ctx, s);
 }
 
@@ -228,21 +225,10 @@ int upload_stack(fbp_context* ctx, Stack& s, const float* src, int u, int v, int
 int download_rows(fbp_context* ctx, Stack& s, size_t row0, size_t nrows, float* dst, int on_dev, size_t row_step = 1) {
   if (!dst) return fbp::set_error(ctx, FBP_ERR_INVALID_ARGUMENT, "null destination pointer");
   FBP_TRY(flush_pending(ctx, s));
-  if (s.filtered) {
-    // unpack just these rows into a scratch f32 block
-    float* tmp = static_cast<float*>(fbp::scratch(ctx, sizeof(float) * nrows * s.pitch));
-    if (!tmp) return FBP_ERR_OUT_OF_MEMORY;
-    FBP_TRY(fbp::launch_unpack_rows(ctx, s, row0, nrows, tmp, s.pitch, (long long)row_step));
-    FBP_TRY(fbp::cuda_check(ctx,
-                            copy_rows(dst, (size_t)s.u * 4, tmp, (size_t)s.pitch * 4, (size_t)s.u * 4, nrows,
-                                              kind_of(true, on_dev), ctx->stream),
-                            "row download"));
-  } else {
-    FBP_TRY(fbp::cuda_check(ctx,
-                            copy_rows(dst, (size_t)s.u * 4, s.f32 + row0 * s.pitch, (size_t)s.pitch * 4 * row_step,
-                                              (size_t)s.u * 4, nrows, kind_of(true, on_dev), ctx->stream),
-                            "row download"));
-  }
+  FBP_TRY(fbp::cuda_check(ctx,
+                          copy_rows(dst, (size_t)s.u * 4, s.f32 + row0 * s.pitch, (size_t)s.pitch * 4 * row_step,
+                                            (size_t)s.u * 4, nrows, kind_of(true, on_dev), ctx->stream),
+                          "row download"));
   return sync_host(ctx, !on_dev);
 }
 
@@ -259,9 +245,7 @@ int upload_rows(fbp_context* ctx, Stack& s, size_t row0, size_t nrows, const flo
   return sync_host(ctx, !on_dev);
 }
 
-// Run weights / log (pending) + filter on a stack; the result goes to the
-// stack's filtered buffer in the backprojector's pair layout (FP32 pairs for
-// the FP32 form, FP16 pairs with a per-view scale for the MIXED form).
+// Run weights / log (pending) + filter on a stack, in place (FP32 rows in every form).
 int filter_stack(fbp_context* ctx, Stack& s, int filter_type) {
   if (filter_type < 0 || filter_type > FBP_FILTER_RAMP_SAMPLED)
     return fbp::set_error(ctx, FBP_ERR_INVALID_ARGUMENT, "unknown filter type");
@@ -275,26 +259,6 @@ int filter_stack(fbp_context* ctx, Stack& s, int filter_type) {
   if (impl == FBP_FILTER_IMPL_AUTO)
     impl = (mixed && fbp::toeplitz_supported(s.u)) ? FBP_FILTER_IMPL_TOEPLITZ : FBP_FILTER_IMPL_FFT;
   fbp::RowSet rs = rowset_of(s);
-  if (!mixed) {
-    // FP32 form: straight into the backprojector's float2 pair layout
-    const int layout = fbp::kLayoutPair32;
-    const int fpitch = round_up(s.u, 4);
-    const size_t need = (size_t)fpitch * s.filt_rows() * Stack::elem_bytes(layout);
-    if (!s.filt || s.filt_bytes < need) {
-      cudaFree(s.filt);
-      s.filt = nullptr;
-      s.filt_bytes = 0;
-      if (fbp::cuda_check(ctx, cudaMalloc(&s.filt, need), "cudaMalloc(filtered views)")) return FBP_ERR_OUT_OF_MEMORY;
-      s.filt_bytes = need;
-    }
-    s.filt_layout = layout;
-    s.filt_pitch = fpitch;
-    rs.out = s.filt;
-    rs.out_layout = layout;
-    rs.out_pitch = fpitch;
-  }
-  // MIXED form: FP32 rows in place; the backprojector packs them to FP16
-  // with per-view scales in the layout of the kernel it selects
   if (impl == FBP_FILTER_IMPL_TOEPLITZ)
     FBP_TRY(fbp::launch_filter_toeplitz(ctx, rs, n, filter_type));
   else
@@ -352,8 +316,8 @@ fbp::BPGeom cone_geom(const Stack& s, float sod, float odd, float det_w, float v
 }
 
 // Autotuner: the first backprojection of a geometry (with autotuning on) times
-// each applicable shape - the four-fold symmetric kernel with 16 voxels per
-// thread along y (one CTA per SM) or 8 (two CTAs per SM), the generic kernel
+// each applicable shape - the four-fold symmetric kernel with its own choice
+// of tile height, with 16 or with 8, the generic kernel
 // with 16 or 8 voxels per thread, each with its full view ring or a 4-stage
 // one - on a central slab of up to 48 y-slices (written into the volume,
 // which the real launch then overwrites) and keeps the fastest for that
@@ -365,7 +329,7 @@ void tune_key(const fbp_context* ctx, const Stack& s, const fbp::BPGeom& g, doub
   const double k[fbp_context::kTuneKey] = {
       (double)g.kind, g.sod, g.sdd, g.du, g.dv, g.vox, g.span, g.offset, (double)g.nu, (double)g.nv,
       (double)g.nviews, (double)g.nx, (double)g.ny, (double)g.nz, (double)ctx->precision,
-      (double)(s.filtered ? s.filt_layout : -1), (double)g.row_off, (double)g.nv_total, (double)g.y_off,
+      (double)(s.filtered ? fbp::kLayoutQuad32 : -1), (double)g.row_off, (double)g.nv_total, (double)g.y_off,
       (double)g.ny_total, (double)s.sinogram, (double)ctx->num_sms, (double)ctx->device_cc};
   std::copy(k, k + fbp_context::kTuneKey, key);
 }
@@ -431,9 +395,10 @@ int autotune_backprojector(fbp_context* ctx, Stack& s, const fbp::BPGeom& g, boo
   gt.y_off = g.y_off + y0;
   gt.ny = nt;
   gt.vol_ystride = g.vol_ystride > 0 ? g.vol_ystride : g.ny;
-  const TuneShape cand[6] = {{FBP_BACKPROJECTOR_SYMMETRIC, 16, 0}, {FBP_BACKPROJECTOR_SYMMETRIC, 8, 0},
-                             {FBP_BACKPROJECTOR_GENERIC, 0, 0},    {FBP_BACKPROJECTOR_GENERIC, 0, 4},
-                             {FBP_BACKPROJECTOR_GENERIC_Y8, 0, 0}, {FBP_BACKPROJECTOR_GENERIC_Y8, 0, 4}};
+  const TuneShape cand[7] = {{FBP_BACKPROJECTOR_SYMMETRIC, 0, 0},  {FBP_BACKPROJECTOR_SYMMETRIC, 16, 0},
+                             {FBP_BACKPROJECTOR_SYMMETRIC, 8, 0},  {FBP_BACKPROJECTOR_GENERIC, 0, 0},
+                             {FBP_BACKPROJECTOR_GENERIC, 0, 4},    {FBP_BACKPROJECTOR_GENERIC_Y8, 0, 0},
+                             {FBP_BACKPROJECTOR_GENERIC_Y8, 0, 4}};
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   FBP_TRY(fbp::cuda_check(ctx, cudaEventCreate(&e0), "event"));
   FBP_TRY(fbp::cuda_check(ctx, cudaEventCreate(&e1), "event"));
@@ -449,7 +414,7 @@ int autotune_backprojector(fbp_context* ctx, Stack& s, const fbp::BPGeom& g, boo
       rc = r;
       break;
     }
-    s.pack_ready = mixed && !s.filtered;  // the timed launch reuses the packed views
+    s.pack_ready = true;  // the timed launch reuses the packed views
     cudaEventRecord(e0, ctx->stream);
     r = fbp::launch_backproject(ctx, gt, s, ctx->vol + (size_t)y0 * g.nx, 0, mixed);
     cudaEventRecord(e1, ctx->stream);
@@ -617,9 +582,9 @@ int make_tensor_map_2d_bf16_sw128(fbp_context* ctx, CUtensorMap* map, void* base
 
 int prepare_packed(fbp_context* ctx, Stack& s, int layout) {
   const bool quad = fbp::is_quad_layout(layout);
-  const int fpitch = quad ? s.u + 1 : round_up(s.u, 4);
-  const size_t need = quad ? (size_t)(s.n / 4) * (s.v + 1) * (size_t)(s.u + 1) * Stack::elem_bytes(layout)
-                           : (size_t)fpitch * s.filt_rows() * Stack::elem_bytes(layout);
+  const int pair = fbp::is_pair_layout(layout) ? 1 : 0;  // one element row (and quad column) more
+  const int fpitch = quad ? s.u + pair : round_up(s.u, 4);
+  const size_t need = (size_t)(quad ? s.n / 4 : s.n) * (s.v + pair) * (size_t)fpitch * Stack::elem_bytes(layout);
   if (!s.filt || s.filt_bytes < need) {
     cudaFree(s.filt);
     s.filt = nullptr;
@@ -638,7 +603,7 @@ int prepare_packed(fbp_context* ctx, Stack& s, int layout) {
   float* scale = s.inv_scale + s.n;
   // the four-term difference of the gradient layout is at most 4 max|value|;
   // the 24-bit layout keeps the FP32 exponent and needs no scale
-  if (layout != kLayoutQuadG24)
+  if (layout != kLayoutQuadG24 && layout != kLayoutQuad32)
     if (int rc = launch_view_scales(ctx, rowset_of(s), quad ? 8192.f : 16384.f, scale, s.inv_scale)) return rc;
   if (int rc = launch_pack(ctx, s, layout, s.filt, fpitch, scale)) return rc;
   s.filt_layout = layout;
@@ -1504,7 +1469,7 @@ int fbp_reconstruct_fdk_to_host(fbp_context* ctx, const float* projections, int 
       apply_shape(ctx, saved);
       rc = fbp::launch_backproject(ctx, gs, s, ctx->vol + (size_t)y0 * h, ylim, mixed);
     }
-    s.pack_ready = mixed && !s.filtered;  // the first slab packed the views: the others reuse them
+    s.pack_ready = true;  // the first slab packed the views: the others reuse them
     if (rc) break;
     if ((rc = fbp::cuda_check(ctx, cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming), "event")) ||
         (rc = fbp::cuda_check(ctx, cudaEventRecord(done[k], ctx->stream), "event")) ||

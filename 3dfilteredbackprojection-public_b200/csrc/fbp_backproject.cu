@@ -13,7 +13,7 @@
 //     rotation axis (y); each consumer thread owns one column segment of NY
 //     voxels and keeps its NY sums in registers across every view, so the
 //     volume is written exactly once (clip epilogue fused into the store).
-//   * Warp specialisation: one producer warp computes, in FP64, the tile's
+//   * Warp specialisation (generic kernel): one producer warp computes, in FP64, the tile's
 //     detector footprint and tile-local projective coefficients for 32 views
 //     at a time (one view per lane), re-based on the tile corner and on the
 //     staged window so that the FP32 coordinates the consumers form stay small
@@ -23,12 +23,12 @@
 //     arrive as zeros from the TMA out-of-bounds fill. Full / empty mbarriers
 //     per stage replace block barriers; consumer warps never wait for one
 //     another.
-//   * Filtered views are stored in a pair layout (element (v, u) holds rows v
-//     and v + 1), so a bilinear tap is two shared-memory loads (8-byte float2
-//     or 4-byte half2). Per view a consumer thread forms 1/D, its detector
-//     column u (constant along the column), the distance weight and the v
-//     step once; per voxel it steps v with one FMA and takes floor / fraction
-//     with the 1.5 * 2^23 rounding constant (no conversion instructions).
+//   * Per view a consumer thread forms 1/D, its detector column u (constant
+//     along the column), the distance weight and the v step once; per voxel it
+//     steps v and takes floor / fraction with the 1.5 * 2^23 rounding constant
+//     (no conversion instructions). FP16 views are staged as row pairs
+//     (element (v, u) holds rows v and v + 1), FP32 views as plain rows along
+//     which the taps march.
 //   * Every mbarrier wait is bounded; on expiry the CTA records an error and
 //     leaves, and every CTA checks the error word before starting.
 
@@ -39,6 +39,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <type_traits>
 #include <vector>
@@ -55,7 +56,7 @@ struct ViewCoef {
   float Nx, Nz, N0;  // u_local * D
   float Vx, Vz, V0;  // v_local * D at the tile's first y
   float wscale;      // extra per-view weight (FP16 views: 1 / scale)
-  int skip;          // tile footprint misses the detector
+  int skip;          // bit 0: tile footprint misses the detector; bit 1: rows advance by less than one per voxel
   int box;           // staged window: width (elements) | rows << 16
 };
 
@@ -252,7 +253,8 @@ __device__ bool tile_view_coef(const BPArgs& a, int k, int ix0, int iy0, int iz0
   vc.Vz = (float)(dv0 * t.Dz);
   vc.V0 = (float)(t.G * t.Yc + dv0 * t.D0);
   vc.wscale = a.inv_scale ? a.inv_scale[k] : 1.0f;
-  vc.skip = skip;
+  // largest row step of the tile (FP32 rounding of the walk stays far below the margin)
+  vc.skip = (skip ? 1 : 0) | (a.dvn < 0.999 * t.dmin ? 2 : 0);
   return skip;
 }
 
@@ -315,6 +317,12 @@ __device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
   return unpack2(d);
 }
 
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(d);
+}
+
 // Value I (0..15) of a kLayoutQuadG24 element held in 12 words: its three
 // bytes sit at byte 3 I, and the float is rebuilt as (bytes << 8) | low byte.
 template <int I>
@@ -347,37 +355,6 @@ __device__ __forceinline__ float fma_f16_f32(__half a, __half b, float c) {
 
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr uint32_t kMagicBits = 0x4B400000u;
-
-// One bilinear update of a voxel whose window-local row coordinate is v >= 0:
-// accum += W * sample(u, v). v + kMagic rounded toward zero is
-// kMagic + floor(v), so its bit pattern minus kMagicBits is the row index and
-// c0 + bits * RB the address of the element at (floor(v), iu) (c0 folds the
-// window base, the column and -kMagicBits * RB); no conversion instructions.
-// wa, wb already carry W for the FP32 layouts.
-template <int LAYOUT>
-__device__ __forceinline__ void tap(float v, uint32_t c0, uint32_t RB, float wa, float wb, float fu, float W,
-                                    float& accum) {
-  const float t = __fadd_rz(v, kMagic);
-  const float fv = v - (t - kMagic);  // in [0, 1)
-  const uint32_t addr = __float_as_uint(t) * RB + c0;
-  if constexpr (LAYOUT == kLayoutRaw32) {
-    const float p00 = lds_f32(addr), p01 = lds_f32(addr + 4);
-    const float p10 = lds_f32(addr + RB), p11 = lds_f32(addr + RB + 4);
-    const float r0 = fmaf(wb, p01, wa * p00);
-    const float r1 = fmaf(wb, p11, wa * p10);
-    accum += fmaf(fv, r1 - r0, r0);
-  } else if constexpr (LAYOUT == kLayoutPair32) {
-    const float2 X = lds_f32x2(addr), Y = lds_f32x2(addr + 8);  // (p00, p10), (p01, p11)
-    const float r0 = fmaf(wb, Y.x, wa * X.x);
-    const float r1 = fmaf(wb, Y.y, wa * X.y);
-    accum += fmaf(fv, r1 - r0, r0);
-  } else {
-    // element = (row v, row v + 1 minus row v); the u-lerp of both in FP32
-    const float2 x = __half22float2(lds_h2(addr)), y = __half22float2(lds_h2(addr + 4));
-    const float2 ag = ffma2(make_float2(fu, fu), fsub2(y, x), x);
-    accum = fmaf(W, fmaf(fv, ag.y, ag.x), accum);
-  }
-}
 
 template <int LAYOUT, int TX, int TZ, int NY>
 __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constant__ BoxMaps maps, const BPArgs a) {
@@ -450,15 +427,13 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
             mbar_arrive(&full[s]);
           } else {
             const CUtensorMap* m = &maps.map[mi];
-            const uint32_t bytes = (uint32_t)(maps.w[mi / kNH] * maps.h[mi % kNH] * (LAYOUT == kLayoutPair32 ? 8 : 4));
-            mbar_arrive_expect_tx(&full[s], bytes);
-            const int x = LAYOUT == kLayoutPair32 ? 2 * cu0 : cu0;  // float2 elements are two floats
-            const int e0 = cv0 + a.pair_rows;                      // pair layouts: row v is element row v + 1
+            mbar_arrive_expect_tx(&full[s], (uint32_t)(maps.w[mi / kNH] * maps.h[mi % kNH] * 4));
+            const int e0 = cv0 + a.pair_rows;  // pair layout: row v is element row v + 1
             void* dst = smem + (size_t)s * a.box_bytes;
             if (a.sino_layout)
-              tma_load_3d(dst, m, x, kk, e0, &full[s]);
+              tma_load_3d(dst, m, cu0, kk, e0, &full[s]);
             else
-              tma_load_3d(dst, m, x, e0, kk, &full[s]);
+              tma_load_3d(dst, m, cu0, e0, kk, &full[s]);
           }
         }
         __syncwarp();
@@ -475,8 +450,8 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
   const int tx = (warp % WX) * 8 + (lane & 7);
   const int tz = (warp / WX) * 4 + (lane >> 3);
   const float fx = (float)tx, fz = (float)tz;
-  constexpr int ESZ = LAYOUT == kLayoutPair32 ? 8 : 4;
-  // rows of a window usable as floor(v): all for pair layouts, all but the
+  constexpr int ESZ = 4;
+  // rows of a window usable as floor(v): all for the pair layout, all but the
   // last for the raw layout (it also reads row v + 1)
   constexpr int kRowTail = LAYOUT == kLayoutRaw32 ? 1 : 0;
 
@@ -493,9 +468,9 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
       break;
     }
     const ViewCoef g = coef[s];
-    if (!g.skip) {
+    if (!(g.skip & 1)) {
       const float D = fmaf(g.Dx, fx, fmaf(g.Dz, fz, g.D0));
-      const float rD = __frcp_rn(D);
+      const float rD = rcp_approx(D);
       const float ul = fmaf(g.Nx, fx, fmaf(g.Nz, fz, g.N0)) * rD;
       const float vl = fmaf(g.Vx, fx, fmaf(g.Vz, fz, g.V0)) * rD;
       const float dvv = a.dvn * rD;
@@ -511,10 +486,61 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
       // the rounded row index can never pass the last staged row
       const float vmax_ok = (float)(BV - kRowTail) - (float)(kSlack / 2);
       if (iu >= 0 && iu <= BU - 2 && vl >= 0.f && vlast < vmax_ok) {
-        const float wa = W - W * fu, wb = W * fu;
         const uint32_t c0 = smem_u32(smem + (size_t)s * a.box_bytes) + (uint32_t)(iu * ESZ) - kMagicBits * RB;
+        // floor and fraction of v with the rounding constant: v + kMagic toward
+        // zero is kMagic + floor(v), whose bit pattern times RB plus c0 is the
+        // element's address; two voxels at a time in packed FP32, stepped by 2 dvv
+        float2 v2 = make_float2(vl, vl + dvv);
+        const float2 step2 = make_float2(2.f * dvv, 2.f * dvv), magic2 = make_float2(kMagic, kMagic);
+        if constexpr (LAYOUT == kLayoutRaw32) {
+          // march along the column: a voxel's upper row, interpolated in u (the
+          // distance weight folded in), is the next voxel's lower row when the
+          // rows advance by one, so a voxel reads one new row (8 bytes) or two
+          const float wb = W * fu, wa = W - wb;
+          auto load = [&](uint32_t at) { return fmaf(wb, lds_f32(at + 4), wa * lds_f32(at)); };
+          auto march = [&](auto shortc) {
+            constexpr bool SHORT = decltype(shortc)::value;
+            float lo = 0.f, hi = 0.f;
+            uint32_t before = 0;
 #pragma unroll
-        for (int j = 0; j < NY; ++j) tap<LAYOUT>(fmaf((float)j, dvv, vl), c0, RB, wa, wb, fu, W, acc[j]);
+            for (int j = 0; j < NY; j += 2) {
+              if (j) v2 = fadd2(v2, step2);
+              const float2 t2 = fadd2_rz(v2, magic2);
+              const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
+#pragma unroll
+              for (int p = 0; p < 2 && j + p < NY; ++p) {
+                const uint32_t bits = __float_as_uint(p ? t2.y : t2.x);
+                const uint32_t at = bits * RB + c0;
+                if (j + p == 0) {
+                  lo = load(at);
+                } else {
+                  lo = bits == before ? lo : hi;
+                  if (!SHORT && bits - before > 1u) lo = load(at);
+                }
+                hi = load(at + RB);
+                acc[j + p] += fmaf(p ? fv2.y : fv2.x, hi - lo, lo);
+                before = bits;
+              }
+            }
+          };
+          if (g.skip & 2) march(std::true_type{});
+          else march(std::false_type{});
+        } else {
+          // element = (row v, row v + 1 minus row v); the u-lerp of both in FP32
+#pragma unroll
+          for (int j = 0; j < NY; j += 2) {
+            if (j) v2 = fadd2(v2, step2);
+            const float2 t2 = fadd2_rz(v2, magic2);
+            const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
+#pragma unroll
+            for (int p = 0; p < 2 && j + p < NY; ++p) {
+              const uint32_t at = __float_as_uint(p ? t2.y : t2.x) * RB + c0;
+              const float2 x = __half22float2(lds_h2(at)), y = __half22float2(lds_h2(at + 4));
+              const float2 ag = ffma2(make_float2(fu, fu), fsub2(y, x), x);
+              acc[j + p] = fmaf(W, fmaf(p ? fv2.y : fv2.x, ag.y, ag.x), acc[j + p]);
+            }
+          }
+        }
       } else {
         bad = true;  // cannot happen when the footprint pass is right; recorded below
       }
@@ -556,41 +582,91 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
 // degrees, (-Z, X), at view k + K/4 project to the same detector coordinate
 // (t = X cos + Z sin and s = -X sin + Z cos are unchanged). A CTA therefore
 // owns an orbit of four 16 x 16 x NY tiles (a tile of the lower-left quadrant
-// and its three rotations) and walks all K views m of the representative
-// tile: the producer computes the tile footprint and coefficients once per m
-// and stages the windows of views m + r K/4 (mod K), r = 0..3 (same origin
-// and box), which feed the r-th rotated tile; each consumer thread forms its
-// detector column, weights and v steps once per m and applies every
-// floor / fraction / address to four accumulator sets. Windows live in a byte ring
-// (entries of variable size, freed in order), so typical small windows keep
-// several quads in flight while the largest still fits.
+// and its three rotations) and walks all K views of the representative tile:
+// one warp computes the tile footprint and coefficients once per view k, a
+// second one stages one window of the interleaved stack, whose element holds the
+// samples of the views g + s K/4 (g = k mod K/4) in slots s = 0 .. 3; each
+// consumer thread forms its detector column, weights and v steps once per view
+// and applies every floor / fraction / address to four accumulator sets.
+// Rotation r of the tile reads slot (m + r) mod 4 at view k = g + m K/4: the
+// sums stay in slot order and are turned by one slot whenever the walk passes
+// from one quarter turn to the next, so one copy of the tap code serves all
+// quarters. Windows live in a byte ring (entries of variable size, freed in
+// order), so typical small windows keep several views in flight while the
+// largest still fits.
+//
+// Layouts: FP16 and 24-bit gradient quads (MIXED, MIXED24), whose element
+// carries everything a tap needs, and plain FP32 quads (FP32 form), where a
+// tap needs two rows of two columns. A column's voxels share u, so the FP32
+// taps march along it: the row above the previous voxel's becomes this
+// voxel's lower row, already interpolated in u, and each voxel reads one new
+// row (two 16-byte loads, 8 bytes an update, against 16 for the four samples)
+// as long as the rows advance by at most one per voxel, and a second one where
+// they advance by more.
+//
+// Bound: FP32, the load / store unit (80% busy: 2 to 3 wavefronts per 32
+// updates); MIXED, the FMA pipes' dependent chains (29 FMA-pipe operations per
+// four updates; 64% of issue slots at 16 consumer warps); 24-bit, both.
+// Measured, backprojection with its packing, before = four row-pair windows
+// (FP32) or the quarters unrolled (MIXED), 8 consumer warps, one producer warp:
+//            256^3 x 360     512^3 x 720     480^3 x 480*    768^3 x 1024
+//   FP32     3.59 -> 2.47    55.6 -> 37.0    23.8 -> 17.6    264.6 -> 174.0 ms
+//   MIXED    2.66 -> 2.52    39.4 -> 36.6    15.9 -> 14.8    185.5 -> 165.4 ms
+//   24-bit   3.63 -> 3.32    52.8 -> 46.4    20.9 -> 19.7    247.5 -> 214.3 ms
+// (* the 1440^3 geometry at a third). Tried and slower: fetching a view's record
+// and projection before the previous view's taps (and two windows held at once
+// can need more than the ring), 16 voxels a thread for FP32.
 
 constexpr int kQuadEntries = 8;  // outstanding view-quads per CTA
 
 // Quad record flags.
 constexpr int kQSkip = 1;    // the tile footprint misses the detector (or failed a check): no taps
-constexpr int kQDirect = 2;  // interleaved layout: window not staged, consumers gather it from global memory
+constexpr int kQDirect = 2;  // window not staged, consumers gather it from global memory
 constexpr int kQFirst = 4;   // first quad of a work item (a tile orbit and y-slab of one job)
 constexpr int kQLast = 8;    // last quad of a work item: the consumers store its voxels next
 constexpr int kQExit = 16;   // multi-job launch: the queue is empty, the CTA leaves
+constexpr int kQTurn = 32;   // last view of a quarter turn: the sums move on by one slot
+constexpr int kQShort = 64;  // rows advance by less than one per voxel everywhere in the tile
 
-// 16-byte aligned so that consumers read a record with vector loads (96 bytes)
+// 16-byte aligned so that consumers read a record with vector loads: four for
+// every layout, the fifth (weights) for the FP16 views, the last for windows
+// that are not staged and for the next item
 struct alignas(16) QuadCoef {
-  float Dx, Dz, D0, Nx, Nz, N0, Vx, Vz, V0;
-  float ws[4];  // per-view extra weight of the four views (FP16 views: 1 / scale)
-  int flags;    // kQ* bits
-  int sub;      // bytes between the entry's four windows
-  int u0, e0;   // direct: element column / element row of the window origin
+  float Dx, Dz, D0, Nx;
+  float Nz, N0, Vx, Vz;
+  float V0;
+  float dvn;       // the job's v step per voxel times D
+  float vmax;      // exclusive bound on the window-local v of a tap
+  int flags;       // kQ* bits
   // consumer constants of the window, formed once by the producer
   uint32_t cbase;  // ring address of element column 0 minus kMagicBits element rows
   uint32_t rb;     // bytes per staged element row
-  uint32_t plane;  // interleaved layout: bytes between the 16-byte planes of an element row
   int bu2;         // last element column a tap may start at (box width - 2)
-  float vmax;      // exclusive bound on the window-local v of a tap
-  float dvn;       // the job's v step per voxel times D
+  uint32_t plane;  // bytes between the 16-byte planes of an element row
+  float ws[4];     // per-view extra weight of the four slots (FP16 views: 1 / scale)
+  int grp;         // view group
+  int u0, e0;      // direct: element column / element row of the window origin
   int item;        // work item of this quad
 };
 static_assert(sizeof(QuadCoef) == 96, "six 16-byte loads per record");
+
+// A quad from the geometry warp to the issuing warp: the consumers' record
+// (its ring address still open) and its copy.
+struct alignas(16) QuadStage {
+  QuadCoef qc;
+  int need, tx_bytes;  // ring bytes, bytes of the copy (0, -: nothing to copy)
+  int x, y, grp, mi;   // tensor coordinates and box
+  int pad[2];
+};
+constexpr int kGeoQuads = 32;  // quads per block between the two (one a lane)
+static_assert(sizeof(QuadStage) == 128, "stage records");
+
+__device__ __forceinline__ void named_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 
 // Multi-job launch (several reconstructions in one persistent launch): one
 // entry per job in global memory; work item item0 + i of job j is the job's
@@ -634,12 +710,11 @@ __device__ __forceinline__ const BoxMaps& job_maps(const BoxMaps& m, const QuadQ
   else return m;
 }
 
-// Tile of a work item and the first view (group) of its walk. The walk starts
-// at an offset advanced by about K views per `resident` CTAs in tile order
-// (interleaved layout: by view groups): tiles that run at the same time then
-// read the same views (their windows share L2) instead of all starting at view
-// 0. The offset depends only on the tile, so results are the same whichever
-// CTA, launch or batch computes it.
+// Tile of a work item and the first view of its walk. The walk starts at an
+// offset advanced by about K views per `resident` CTAs in tile order: tiles
+// that run at the same time then read the same views (their windows share L2)
+// instead of all starting at view 0. The offset depends only on the tile, so
+// results are the same whichever CTA, launch or batch computes it.
 //
 // Tile order within a y-slab: bands of `band` orbit rows along z, walked
 // column by column along x, so the ~`resident` tiles that run at once form a
@@ -648,9 +723,9 @@ __device__ __forceinline__ const BoxMaps& job_maps(const BoxMaps& m, const QuadQ
 // tiles would, and DRAM reads of the filtered views fall in proportion.
 struct ItemTile {
   int ix0, iy0, iz0;
-  int g0, k0;
+  int k0;
 };
-template <bool QG, int NY>
+template <int NY>
 __device__ __forceinline__ ItemTile item_tile(const BPArgs& ja, long long t, int nbh) {
   ItemTile it;
   const long long per = (long long)nbh * nbh;
@@ -665,17 +740,27 @@ __device__ __forceinline__ ItemTile item_tile(const BPArgs& ja, long long t, int
   it.iz0 = bz * 16;
   it.iy0 = by * NY;
   const int K = ja.nviews;
-  it.g0 = QG ? (int)((t * (K >> 2) / max(1, ja.resident)) % (K >> 2)) : 0;
-  it.k0 = QG ? 0 : (int)((t * K / max(1, ja.resident)) % K);
+  it.k0 = (int)((t * K / max(1, ja.resident)) % K);
   return it;
 }
 
-// 288 threads. OCC = 2 CTAs per SM: 9 warps each put 5 warps on some SM
-// sub-partitions (16K registers each), so at most 96 registers per thread,
-// and each CTA gets half of the shared memory. OCC = 1: up to 168 registers
-// and all of the shared memory, for 16 voxels per thread along y (64
-// accumulators a thread, the window staged once for twice the voxels).
-//
+// Shapes. A CTA's representative tile is 16 x 16 columns x TY = NY YW voxels:
+// eight consumer warps, or two times eight one above the other (YW = 2), of 32
+// columns x NY voxels (4 NY sums a thread), then the issuing warp and the
+// geometry warp. What separates the shapes is how many consumer warps a
+// scheduler has to hide the taps' chains behind one another (8 of NY = 16: two;
+// 16 of NY = 8 or 12: four) against the registers they leave (168, 96 .. 112)
+// and the work per view and thread, which is the same for any NY (about a fifth
+// of the instructions at NY = 16, a third at 8). Launches give every warp the
+// same registers; the shapes that need more for their consumers get whole
+// warpgroups (four warps, two of them idle) of producers and move the
+// producers' surplus with setmaxnreg: 640 x 96 = 512 x 112 + 128 x 32, 384 x 80
+// = 256 x 104 + 128 x 32.
+constexpr bool quad_moves_regs(int layout, int NY, int YW) { return YW == 2 || (layout == kLayoutQuad32 && NY == 12); }
+constexpr int quad_threads(int layout, int NY, int YW) {
+  return 256 * YW + (quad_moves_regs(layout, NY, YW) ? 128 : 64);
+}
+
 // MULTI = false: one job, one work item (tile orbit and y-slab) per CTA, from
 // the block index. MULTI = true: a persistent launch of OCC CTAs per SM over
 // the work items of several jobs (uneven sizes, each with its own geometry,
@@ -685,33 +770,31 @@ __device__ __forceinline__ ItemTile item_tile(const BPArgs& ja, long long t, int
 // first quad and store its voxels after its last. An item's arithmetic and
 // view order do not depend on the launch, so a job's volume is the same bits
 // alone or batched with others.
-template <int LAYOUT, int NY, int OCC, bool MULTI>
-__global__ void __launch_bounds__(256 + 32, OCC)
+template <int LAYOUT, int NY, int YW, int OCC, bool MULTI>
+__global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
     bp_quad_kernel(const __grid_constant__ BoxMaps maps, const __grid_constant__ BPArgs a,
                    const __grid_constant__ QuadQueue qq) {
-  constexpr int TX = 16, TZ = 16, NCW = 8, E = kQuadEntries;
-  // QG: the four views of a quad come interleaved in one window (one copy,
-  // two 16-byte loads per voxel step feed all four taps). The quads are
-  // walked group-major, q = g + m K/4 for m = 0..3, so the slot of rotation
-  // r, (m + r) mod 4, is a compile-time index in each of the four unrolled steps.
-  // QG24: the same with three 16-byte planes of 24-bit values and no scale.
-  constexpr bool QG24 = LAYOUT == kLayoutQuadG24;
-  constexpr bool QG = LAYOUT == kLayoutQuadG16 || QG24;
-  constexpr int ESZ = QG24 ? 48 : QG ? 32 : LAYOUT == kLayoutPair32 ? 8 : 4;
-  constexpr int NPL = QG24 ? 3 : 2;  // 16-byte planes per element row
-  constexpr int kRowTail = LAYOUT == kLayoutRaw32 ? 1 : 0;
+  constexpr int TX = 16, TZ = 16, TY = NY * YW, NCW = 8 * YW, E = kQuadEntries;
+  constexpr bool Q24 = LAYOUT == kLayoutQuadG24;
+  constexpr bool Q32 = LAYOUT == kLayoutQuad32;
+  constexpr int NPL = Q24 ? 3 : Q32 ? 1 : 2;  // 16-byte planes per element row
+  constexpr int ESZ = 16 * NPL;
+  constexpr int kRowTail = Q32 ? 1 : 0;  // a tap also reads the next element row
+  constexpr int kCol0 = Q32 ? 0 : 1;     // element column of detector column 0 (gradient elements start at -1)
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int R = MULTI ? qq.ring : a.box_bytes;  // ring bytes
   int* const err = MULTI ? qq.err : a.err;
 
   QuadCoef* coef = reinterpret_cast<QuadCoef*>(smem + R);
-  uint64_t* full = reinterpret_cast<uint64_t*>(coef + E);
+  QuadStage* stage = reinterpret_cast<QuadStage*>(coef + E);  // two blocks
+  uint64_t* full = reinterpret_cast<uint64_t*>(stage + 2 * kGeoQuads);
   uint64_t* empty = full + E;
   // end_pos: ring byte position (64-bit: a persistent CTA allocates far more
   // than 2^31 bytes over its items) where each entry's windows end
   long long* end_pos = reinterpret_cast<long long*>(empty + E);
   volatile int* s_abort = reinterpret_cast<volatile int*>(end_pos + E);
+  volatile int* hdr = s_abort + 1;  // per block: quads (-1: no more), job
 
   if (tid == 0) {
     *s_abort = *(volatile int*)err != 0;
@@ -725,15 +808,19 @@ __global__ void __launch_bounds__(256 + 32, OCC)
   __syncthreads();
   if (*s_abort) return;
 
-  if (warp == NCW) {
-    // ---------------------------------------------------------------- producer
-    // head / tail: ring bytes allocated / freed; hpos = head mod R; oldest:
-    // first quad not yet known to be released; seq: quads issued since the
-    // launch (all items)
-    long long head = 0, tail = 0;
-    int hpos = 0, oldest = 0, seq = 0;
-    bool more = true, first = true;
-    while (more && !*s_abort) {
+  // Named barriers between the two producer warps: block b full, block b free
+  constexpr int kBarFull = 1, kBarFree = 3;
+  if (warp >= NCW) {
+    if constexpr (quad_moves_regs(LAYOUT, NY, YW)) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    if (warp > NCW + 1) return;
+  }
+  if (warp == NCW + 1) {
+    // ---------------------------------------------------------------- geometry
+    // one quad a lane, a block ahead of the issuing warp: its FP64 chains and
+    // (at 32 registers) spills stay off the ring's path
+    int b = 0, blocks = 0;
+    bool first = true;
+    while (!*s_abort) {
       // the next work item: this CTA's tile, or the queue's next item
       long long item;
       if constexpr (MULTI) {
@@ -750,24 +837,19 @@ __global__ void __launch_bounds__(256 + 32, OCC)
       const BPArgs& ja = job_args<MULTI>(a, qq, jb);
       const BoxMaps& jm = job_maps<MULTI>(maps, qq, jb);
       const long long t_local = MULTI ? item - qq.jobs[jb].item0 + qq.jobs[jb].t0 : item;
-      const ItemTile til = item_tile<QG, NY>(ja, t_local, MULTI ? qq.jobs[jb].nbh : ja.ntx >> 1);
+      const ItemTile til = item_tile<TY>(ja, t_local, MULTI ? qq.jobs[jb].nbh : ja.ntx >> 1);
       const int K = ja.nviews, Q = K >> 2;
-      for (int kb = 0; kb < K && !*s_abort; kb += 32) {
-        const int it = kb + lane;  // quad of the item (ring entry order)
-        // view of the representative tile; rotation r uses view (k + r Q) mod K
-        const int gq = QG ? ((it >> 2) + til.g0) % Q : 0;  // view group of quad it
-        const int k = QG ? gq + (it & 3) * Q : (it + til.k0) % K;
-        QuadCoef qc;
-        int u0 = 0, v0 = 0, mi = 0, need = 0, sub = 0, tx_bytes = 0;
-        bool skip = true, direct = false;
-        qc.flags = kQSkip;
-        qc.rb = 0;
+      for (int kb = 0; kb < K && !*s_abort; kb += kGeoQuads) {
+        if (blocks >= 2) named_sync(kBarFree + b, 64);
+        const int it = kb + lane;         // quad of the item (ring entry order)
+        const int k = (it + til.k0) % K;  // view of the representative tile
         if (it < K) {
+          QuadStage& st = stage[b * kGeoQuads + lane];
           ViewCoef vc;
           bool overflow = false, behind = false;
-          int need_u = 0, need_v = 0;
-          skip = tile_view_coef(ja, k, til.ix0, til.iy0, til.iz0, TX - 1, NY - 1, TZ - 1, vc, u0, v0, need_u,
-                                need_v, overflow, behind);
+          int u0, v0, need_u = 0, need_v = 0;
+          bool skip = tile_view_coef(ja, k, til.ix0, til.iy0, til.iz0, TX - 1, TY - 1, TZ - 1, vc, u0, v0, need_u,
+                                     need_v, overflow, behind);
           // checks of the job's geometry go to the job's error word
           if (overflow) atomicCAS(ja.err, 0, kDevFootprint);
           if (behind) atomicCAS(ja.err, 0, kDevGeometry);
@@ -776,24 +858,29 @@ __global__ void __launch_bounds__(256 + 32, OCC)
           const int rows = need_v - ja.pair_rows;
           while (wi < kNW - 1 && jm.w[wi] < need_u) ++wi;
           while (hi < kNH - 1 && jm.h[hi] < rows) ++hi;
-          mi = wi * kNH + hi;
-          tx_bytes = jm.w[wi] * jm.h[hi] * ESZ;
-          sub = (tx_bytes + 127) & ~127;
-          // interleaved layout: a window wider than the widest box or larger than
-          // the ring (rare near-source tiles) is read from global memory instead
-          direct = QG && !skip && (need_u > jm.w[kNW - 1] || rows > jm.h[kNH - 1] || sub > R);
-          need = (skip || direct) ? 0 : (QG ? sub : 4 * sub);
+          const int tx_bytes = jm.w[wi] * jm.h[hi] * ESZ;
+          const int bytes = (tx_bytes + 127) & ~127;
+          // a window wider than the widest box or larger than the ring (rare
+          // near-source tiles) is read from global memory instead
+          const bool direct = !skip && (need_u > jm.w[kNW - 1] || rows > jm.h[kNH - 1] || bytes > R);
+          st.need = (skip || direct) ? 0 : bytes;
+          st.tx_bytes = tx_bytes;
+          st.x = 2 * (u0 + kCol0);
+          st.y = v0 + ja.pair_rows;
+          st.grp = k % Q;
+          st.mi = wi * kNH + hi;
+          QuadCoef& qc = st.qc;
           qc.Dx = vc.Dx; qc.Dz = vc.Dz; qc.D0 = vc.D0;
           qc.Nx = vc.Nx; qc.Nz = vc.Nz; qc.N0 = vc.N0;
           qc.Vx = vc.Vx; qc.Vz = vc.Vz; qc.V0 = vc.V0;
 #pragma unroll
-          for (int r = 0; r < 4; ++r) qc.ws[r] = ja.inv_scale ? ja.inv_scale[(k + r * Q) % K] : 1.0f;
+          for (int r = 0; r < 4; ++r) qc.ws[r] = ja.inv_scale ? ja.inv_scale[k % Q + r * Q] : 1.0f;
           qc.flags = (skip ? kQSkip : 0) | (direct ? kQDirect : 0) | (it == 0 ? kQFirst : 0) |
-                     (it == K - 1 ? kQLast : 0);
+                     (it == K - 1 ? kQLast : 0) | ((k + 1) % Q == 0 ? kQTurn : 0) | (vc.skip & 2 ? kQShort : 0);
           // window: width (elements) and rows
           const int BU = direct ? need_u : jm.w[wi], BV = direct ? rows : jm.h[hi];
-          qc.sub = sub;
-          qc.u0 = u0 + 1;
+          qc.grp = k % Q;
+          qc.u0 = u0 + kCol0;
           qc.e0 = v0 + ja.pair_rows;
           qc.rb = (uint32_t)(BU * ESZ);
           qc.plane = (uint32_t)(BU * 16);
@@ -802,73 +889,80 @@ __global__ void __launch_bounds__(256 + 32, OCC)
           qc.dvn = ja.dvn;
           qc.item = (int)item;
         }
-        const int nb = min(32, K - kb);
-        for (int i = 0; i < nb; ++i) {
-          const int q = seq + i;  // ring sequence number
-          const int e = q % E;
-          const int qneed = __shfl_sync(0xffffffffu, need, i);
-          // allocate qneed contiguous ring bytes: wrap to 0 when the tail end is too short
-          const bool wrap = hpos + qneed > R;
-          const long long start = wrap ? head + (R - hpos) : head;
-          bool ok = true;
-          while (oldest < q && (oldest <= q - E || start + qneed - tail > R)) {
-            if (!mbar_wait(&empty[oldest % E], (oldest / E) & 1, err)) {
-              ok = false;
-              break;
-            }
-            tail = end_pos[oldest % E];
-            ++oldest;
-          }
-          if (!ok) {
-            *s_abort = 1;
-            more = false;
+        if (lane == 0) {
+          hdr[2 * b] = min(kGeoQuads, K - kb);
+          hdr[2 * b + 1] = jb;
+        }
+        __syncwarp();
+        named_arrive(kBarFull + b, 64);
+        b ^= 1;
+        ++blocks;
+      }
+    }
+    if (blocks >= 2) named_sync(kBarFree + b, 64);
+    if (lane == 0) hdr[2 * b] = -1;
+    __syncwarp();
+    named_arrive(kBarFull + b, 64);
+    if (blocks >= 1) named_sync(kBarFree + (b ^ 1), 64);  // the last block's release: no arrival is left pending
+    return;
+  }
+  if (warp == NCW) {
+    // ----------------------------------------------------------------- issuing
+    // head / tail: ring bytes allocated / freed; hpos = head mod R; oldest:
+    // first quad not yet known to be released; seq: quads issued since the
+    // launch (all items)
+    long long head = 0, tail = 0;
+    int hpos = 0, oldest = 0, seq = 0;
+    for (int b = 0;; b ^= 1) {
+      named_sync(kBarFull + b, 64);
+      const int nb = hdr[2 * b];
+      if (nb < 0) break;
+      const BoxMaps& jm = job_maps<MULTI>(maps, qq, MULTI ? hdr[2 * b + 1] : 0);
+      for (int i = 0; i < nb && !*s_abort; ++i) {  // after an abort the blocks are only handed back
+        const QuadStage& st = stage[b * kGeoQuads + i];
+        const int q = seq, e = q % E;  // ring sequence number and entry
+        const int qneed = st.need;
+        // allocate qneed contiguous ring bytes: wrap to 0 when the tail end is too short
+        const bool wrap = hpos + qneed > R;
+        const long long start = wrap ? head + (R - hpos) : head;
+        bool ok = true;
+        while (oldest < q && (oldest <= q - E || start + qneed - tail > R)) {
+          if (!mbar_wait(&empty[oldest % E], (oldest / E) & 1, err)) {
+            ok = false;
             break;
           }
-          if (oldest == q) tail = start;  // nothing outstanding: the whole ring is free
-          const int off = wrap ? 0 : hpos;  // start mod R
-          if (lane == i) {
-            qc.cbase = smem_u32(smem) + (uint32_t)off - kMagicBits * qc.rb;
-            coef[e] = qc;
-          }
-          if (lane == 0) end_pos[e] = start + qneed;
-          head = start + qneed;
-          hpos = off + qneed == R ? 0 : off + qneed;
-          const int sk = __shfl_sync(0xffffffffu, (int)(skip || direct), i);
-          const int cu0 = __shfl_sync(0xffffffffu, u0, i), cv0 = __shfl_sync(0xffffffffu, v0, i);
-          const int cmi = __shfl_sync(0xffffffffu, mi, i), csub = __shfl_sync(0xffffffffu, sub, i);
-          const int ctx = __shfl_sync(0xffffffffu, tx_bytes, i);
-          // view of the representative tile at quad kb + i (the interleaved layout addresses its group)
-          const int ck = QG ? 0 : __shfl_sync(0xffffffffu, k, i);
-          __syncwarp();
-          if (lane == 0) {
-            if (sk) {
-              mbar_arrive(&full[e]);
-            } else if (QG) {
-              // group gq, slots = views gq + s Q; element column u0 + 1 holds columns u0, u0 + 1
-              mbar_arrive_expect_tx(&full[e], (uint32_t)ctx);
-              tma_load_4d(smem + off, &jm.map[cmi], 2 * (cu0 + 1), 0, cv0 + ja.pair_rows,
-                          (((kb + i) >> 2) + til.g0) % Q, &full[e]);
-            } else {
-              mbar_arrive_expect_tx(&full[e], (uint32_t)(4 * ctx));
-              const CUtensorMap* m = &jm.map[cmi];
-              const int x = LAYOUT == kLayoutPair32 ? 2 * cu0 : cu0;
-              const int e0 = cv0 + ja.pair_rows;
-#pragma unroll
-              for (int r = 0; r < 4; ++r) {
-                void* dst = smem + off + r * csub;
-                const int kv = (ck + r * Q) % K;
-                if (ja.sino_layout)
-                  tma_load_3d(dst, m, x, kv, e0, &full[e]);
-                else
-                  tma_load_3d(dst, m, x, e0, kv, &full[e]);
-              }
-            }
-          }
-          __syncwarp();
+          tail = end_pos[oldest % E];
+          ++oldest;
         }
-        if (!more) break;
-        seq += nb;
+        if (!ok) {
+          *s_abort = 1;
+          break;
+        }
+        if (oldest == q) tail = start;    // nothing outstanding: the whole ring is free
+        const int off = wrap ? 0 : hpos;  // start mod R
+        // the record, one word a lane, its ring address filled in
+        constexpr int kWords = sizeof(QuadCoef) / 4, kBaseWord = offsetof(QuadCoef, cbase) / 4;
+        if (lane < kWords) {
+          uint32_t w = reinterpret_cast<const uint32_t*>(&st.qc)[lane];
+          if (lane == kBaseWord) w = smem_u32(smem) + (uint32_t)off - kMagicBits * st.qc.rb;
+          reinterpret_cast<uint32_t*>(&coef[e])[lane] = w;
+        }
+        if (lane == 0) end_pos[e] = start + qneed;
+        head = start + qneed;
+        hpos = off + qneed == R ? 0 : off + qneed;
+        __syncwarp();
+        if (lane == 0) {
+          if (qneed == 0) {
+            mbar_arrive(&full[e]);
+          } else {
+            mbar_arrive_expect_tx(&full[e], (uint32_t)st.tx_bytes);
+            tma_load_4d(smem + off, &jm.map[st.mi], st.x, 0, st.y, st.grp, &full[e]);
+          }
+        }
+        __syncwarp();
+        ++seq;
       }
+      named_arrive(kBarFree + b, 64);
     }
     if (MULTI && !*s_abort) {
       // queue empty: one record that tells the consumers to leave
@@ -897,17 +991,28 @@ __global__ void __launch_bounds__(256 + 32, OCC)
     return;
   }
 
+  if constexpr (YW == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+  else if constexpr (quad_moves_regs(LAYOUT, NY, YW)) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
   // ------------------------------------------------------------------ consumers
-  // a warp owns 8 x 4 columns; for the interleaved layout each quarter-warp
-  // (one shared-memory phase of 16-byte loads) is a compact 4 x 2 patch, whose
-  // detector columns stay within 8 elements (no bank conflicts)
-  const int tx = QG ? (warp & 1) * 8 + ((lane >> 3) & 1) * 4 + (lane & 3) : (warp & 1) * 8 + (lane & 7);
-  const int tz = QG ? (warp >> 1) * 4 + (lane >> 4) * 2 + ((lane >> 2) & 1) : (warp >> 1) * 4 + (lane >> 3);
+  // a warp owns 8 x 4 columns; each quarter-warp (one shared-memory phase of
+  // 16-byte loads) is a compact 4 x 2 patch, whose detector columns stay
+  // within 8 elements (no bank conflicts)
+  const int tx = (warp & 1) * 8 + ((lane >> 3) & 1) * 4 + (lane & 3);
+  const int tz = ((warp >> 1) & 3) * 4 + (lane >> 4) * 2 + ((lane >> 2) & 1);
+  const int ty = (warp >> 3) * NY;  // first of this warp's voxels along y
   const float fx = (float)tx, fz = (float)tz;
-  // plain FP32 sums: four rotations x NY voxels in registers (a
-  // compensated sum was measured to change no digit of the MIXED form's
-  // error, which the FP16 views set, and cost 5% at C4)
+  // plain FP32 sums: four slots x NY voxels in registers (a compensated sum
+  // was measured to change no digit of the MIXED form's error, which the
+  // FP16 views set, and cost 5% at C4)
   float acc[4][NY];
+  // the next quarter turn: its slot s belongs to the rotation of slot s - 1
+  auto turn = [&]() {
+#pragma unroll
+    for (int j = 0; j < NY; ++j) {
+      const float t = acc[3][j];
+      acc[3][j] = acc[2][j], acc[2][j] = acc[1][j], acc[1][j] = acc[0][j], acc[0][j] = t;
+    }
+  };
   // a new work item: zero every sum of this thread
   auto reset = [&]() {
 #pragma unroll
@@ -918,40 +1023,37 @@ __global__ void __launch_bounds__(256 + 32, OCC)
   reset();
   int e = 0;
   uint32_t ph = 0;
-  bool bad = false, stop = false, last = false, leave = false;
-  int grp = 0;        // interleaved layout: view group of the current four quads
+  bool bad = false, stop = false, last = false, leave = false, turned = false;
   long long item = -1;  // work item being accumulated
   int jb = 0;         // its job
   // one quad: wait for its window, apply it to the 4 x NY voxels, release it
-  auto step = [&](auto mc) {
-    constexpr int M = decltype(mc)::value;
+  auto step = [&]() {
     if (!mbar_wait(&full[e], ph, err)) {
       *s_abort = 1;
       stop = true;
       return;
     }
-    const QuadCoef g = coef[e];
+    const QuadCoef g = coef[e];  // all of it at once: one latency
+    const int flags = g.flags;
     if constexpr (MULTI) {  // one job's single item: set up before the loop, the loop counts its quads
-      if (g.flags & (kQExit | kQFirst)) {
-        if (g.flags & kQExit) {  // no more items (always at a group start)
+      if (flags & (kQExit | kQFirst)) {
+        if (flags & kQExit) {  // no more items
           leave = true;
         } else {
           item = g.item;
           jb = find_job(qq, item);
-          const BPArgs& ja = qq.jobs[jb].a;
-          const ItemTile til = item_tile<QG, NY>(ja, item - qq.jobs[jb].item0 + qq.jobs[jb].t0, qq.jobs[jb].nbh);
-          grp = til.g0;
         }
       }
-      last = (g.flags & kQLast) != 0;
+      last = (flags & kQLast) != 0;
     }
-    if (!(g.flags & kQSkip)) {
+    if (!(flags & kQSkip)) {
       // explicit roundings (no contraction): the same bits in every instantiation
       const float D = fmaf(g.Dx, fx, fmaf(g.Dz, fz, g.D0));
       const float rD = rcp_approx(D);
       const float ul = __fmul_rn(fmaf(g.Nx, fx, fmaf(g.Nz, fz, g.N0)), rD);
-      const float vl = __fmul_rn(fmaf(g.Vx, fx, fmaf(g.Vz, fz, g.V0)), rD);
       const float dvv = __fmul_rn(g.dvn, rD);
+      const float vl0 = __fmul_rn(fmaf(g.Vx, fx, fmaf(g.Vz, fz, g.V0)), rD);
+      const float vl = YW == 1 ? vl0 : fmaf((float)ty, dvv, vl0);
       const float W = __fmul_rn(rD, rD);
       const float fuf = floorf(ul);
       const int iu = (int)fuf;
@@ -959,45 +1061,129 @@ __global__ void __launch_bounds__(256 + 32, OCC)
       const float vlast = fmaf((float)(NY - 1), dvv, vl);
       const uint32_t RB = g.rb;
       if (iu >= 0 && iu <= g.bu2 && vl >= 0.f && vlast < g.vmax) {
-        const uint32_t c0 = g.cbase + (uint32_t)(iu * (QG ? 16 : ESZ));
-        const __half2 fu2 = __float2half2_rn(fu);
-        if constexpr (QG) {
+        const uint32_t c0 = g.cbase + (uint32_t)(iu * 16);
+        // v of voxels j and j + 1, stepped by 2 dvv from (vl, vl + dvv): no
+        // per-pair constants (a few ulps of v from the repeated additions);
+        // floor and fraction of the pair with packed FP32 ops
+        static_assert(NY % 2 == 0, "voxels stepped in pairs");
+        const float2 magic2 = make_float2(kMagic, kMagic);
+        const float dv2 = 2.f * dvv;
+        const float2 step2 = make_float2(dv2, dv2);
+        float2 v2 = make_float2(vl, vl + dvv);
+        if constexpr (Q32) {
+          // weights of the two columns, the distance weight folded in
+          const float wbs = __fmul_rn(W, fu), was = __fsub_rn(W, wbs);
+          const float2 wa = make_float2(was, was), wb = make_float2(wbs, wbs);
+          // an element row at this thread's detector position: the four slots, interpolated in u
+          auto blend = [&](const uint4& A, const uint4& B, float2 (&q)[2]) {
+            q[0] = ffma2(wb, make_float2(__uint_as_float(B.x), __uint_as_float(B.y)),
+                         fmul2(wa, make_float2(__uint_as_float(A.x), __uint_as_float(A.y))));
+            q[1] = ffma2(wb, make_float2(__uint_as_float(B.z), __uint_as_float(B.w)),
+                         fmul2(wa, make_float2(__uint_as_float(A.z), __uint_as_float(A.w))));
+          };
+          auto add = [&](const float2 (&lo)[2], const float2 (&hi)[2], float fv, int j) {
+            const float fl = 1.f - fv;
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+              const float2 d = ffma2(make_float2(fv, fv), hi[p],
+                                     ffma2(make_float2(fl, fl), lo[p], make_float2(acc[2 * p][j], acc[2 * p + 1][j])));
+              acc[2 * p][j] = d.x;
+              acc[2 * p + 1][j] = d.y;
+            }
+          };
+          if (!(flags & kQDirect)) {
+            auto load = [&](uint32_t at, float2 (&q)[2]) { blend(lds_u4(at), lds_u4(at + 16), q); };
+            auto march = [&](auto shortc) {
+              constexpr bool SHORT = decltype(shortc)::value;
+              float2 lo[2], hi[2];
+              uint32_t before = 0;  // bit pattern of the previous voxel's row
+#pragma unroll
+              for (int j = 0; j < NY; j += 2) {
+                if (j) v2 = fadd2(v2, step2);
+                const float2 t2 = fadd2_rz(v2, magic2);
+                const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                  const uint32_t bits = __float_as_uint(p ? t2.y : t2.x);
+                  const uint32_t at = bits * RB + c0;
+                  if (j + p == 0) {
+                    load(at, lo);
+                  } else {
+                    const bool same = bits == before;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                      lo[i].x = same ? lo[i].x : hi[i].x;
+                      lo[i].y = same ? lo[i].y : hi[i].y;
+                    }
+                    if (!SHORT && bits - before > 1u) load(at, lo);
+                  }
+                  load(at + RB, hi);
+                  add(lo, hi, p ? fv2.y : fv2.x, j + p);
+                  before = bits;
+                }
+              }
+            };
+            if (flags & kQShort) march(std::true_type{});
+            else march(std::false_type{});
+          } else {
+            // window not staged: read the elements from global memory (zero
+            // outside the stored extent, as the TMA fill would give)
+            const BPArgs& ja = job_args<MULTI>(a, qq, jb);
+            const int col = g.u0 + iu;
+            auto load = [&](int row, float2 (&q)[2]) {
+              const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+              const uint4* p = ja.qg + ((size_t)g.grp * ja.qg_rows + row) * ja.qg_pitch + col;
+              const bool in = row >= 0 && row < ja.qg_rows;
+              blend(in && col >= 0 && col < ja.qg_pitch ? __ldg(p) : zero,
+                    in && col + 1 >= 0 && col + 1 < ja.qg_pitch ? __ldg(p + 1) : zero, q);
+            };
+#pragma unroll
+            for (int j = 0; j < NY; ++j) {
+              const float v = fmaf((float)j, dvv, vl);
+              const float t = __fadd_rz(v, kMagic);
+              const int row = g.e0 + (int)(__float_as_uint(t) - kMagicBits);
+              float2 lo[2], hi[2];
+              load(row, lo);
+              load(row + 1, hi);
+              add(lo, hi, v - (t - kMagic), j);
+            }
+          }
+        } else {
+          const __half2 fu2 = __float2half2_rn(fu);
           float Wr[4];
 #pragma unroll
           for (int r = 0; r < 4; ++r) Wr[r] = __fmul_rn(W, g.ws[r]);
-          // (A, G) of the four rotations at one voxel from the 2 x 16 bytes of
-          // its element (slot of rotation r: (M + r) mod 4): A = u-lerp of row
-          // e - 1, G = u-lerp of the row difference
+          // (A, G) of the four slots at one voxel from the 16-byte planes of
+          // its element: A = u-lerp of row e - 1, G = u-lerp of the row difference
           auto decode = [&](const uint4& L0, const uint4& L1, const uint4& L2, float (&A)[4], float (&G)[4]) {
-            if constexpr (QG24) {
+            if constexpr (Q24) {
               const uint32_t wv[12] = {L0.x, L0.y, L0.z, L0.w, L1.x, L1.y, L1.z, L1.w, L2.x, L2.y, L2.z, L2.w};
-              // (A, G) = (a, b - a) + fu (c' - a, d - c' - b + a) for the slot of rotation r
-              auto slot = [&](auto slc, float& Ar, float& Gr) {
+              // (A, G) = (a, b - a) + fu (c' - a, d - c' - b + a) of slot SL
+              auto slot = [&](auto slc) {
                 constexpr int SL = decltype(slc)::value;
                 const float2 ag = ffma2(make_float2(fu, fu), make_float2(dec24<4 * SL + 2>(wv), dec24<4 * SL + 3>(wv)),
                                         make_float2(dec24<4 * SL>(wv), dec24<4 * SL + 1>(wv)));
-                Ar = ag.x;
-                Gr = ag.y;
+                A[SL] = ag.x;
+                G[SL] = ag.y;
               };
-              slot(std::integral_constant<int, (M + 0) & 3>{}, A[0], G[0]);
-              slot(std::integral_constant<int, (M + 1) & 3>{}, A[1], G[1]);
-              slot(std::integral_constant<int, (M + 2) & 3>{}, A[2], G[2]);
-              slot(std::integral_constant<int, (M + 3) & 3>{}, A[3], G[3]);
+              slot(std::integral_constant<int, 0>{});
+              slot(std::integral_constant<int, 1>{});
+              slot(std::integral_constant<int, 2>{});
+              slot(std::integral_constant<int, 3>{});
             } else {
               const uint32_t wv[8] = {L0.x, L0.y, L0.z, L0.w, L1.x, L1.y, L1.z, L1.w};
 #pragma unroll
-              for (int r = 0; r < 4; ++r) {
-                const int sl = (M + r) & 3;
+              for (int sl = 0; sl < 4; ++sl) {
                 const __half2 X1 = *reinterpret_cast<const __half2*>(&wv[2 * sl]);      // (a, b - a)
                 const __half2 X2 = *reinterpret_cast<const __half2*>(&wv[2 * sl + 1]);  // (c' - a, d - c' - b + a)
                 const float2 P = __half22float2(X1);
-                A[r] = fma_f16_f32(__low2half(fu2), __low2half(X2), P.x);
-                G[r] = fma_f16_f32(__low2half(fu2), __high2half(X2), P.y);
+                A[sl] = fma_f16_f32(__low2half(fu2), __low2half(X2), P.x);
+                G[sl] = fma_f16_f32(__low2half(fu2), __high2half(X2), P.y);
               }
             }
           };
-          // rotation pairs (0, 1), (2, 3) of one voxel: v-lerp and weighted sum as packed pairs
-          auto rot_pairs = [&](const float (&A)[4], const float (&G)[4], float fv, int j) {
+          // slot pairs (0, 1), (2, 3) of one voxel: v-lerp and weighted sum as packed pairs
+          auto slot_pairs = [&](const float (&A)[4], const float (&G)[4], float fv, int j) {
 #pragma unroll
             for (int pr = 0; pr < 2; ++pr) {
               float& d0 = acc[2 * pr][j];
@@ -1009,29 +1195,21 @@ __global__ void __launch_bounds__(256 + 32, OCC)
               d1 = d.y;
             }
           };
-          if (!(g.flags & kQDirect)) {
+          if (!(flags & kQDirect)) {
             const uint32_t plane = g.plane;
-            static_assert(NY % 2 == 0, "voxels stepped in pairs");
-            const float2 magic2 = make_float2(kMagic, kMagic);
-            // v of voxels j and j + 1, stepped by 2 dvv from (vl, vl + dvv): no
-            // per-pair constants (a few ulps of v from the repeated additions)
-            const float dv2 = 2.f * dvv;
-            const float2 step2 = make_float2(dv2, dv2);
-            float2 v2 = make_float2(vl, vl + dvv);
 #pragma unroll
             for (int j = 0; j < NY; j += 2) {
-              // floor and fraction of voxels j and j + 1 with packed FP32 ops
               if (j) v2 = fadd2(v2, step2);
               const float2 t2 = fadd2_rz(v2, magic2);
               const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
               const uint32_t a0 = __float_as_uint(t2.x) * RB + c0, a1 = __float_as_uint(t2.y) * RB + c0;
-              // slots 0, 1 | slots 2, 3 (QG24: the 48 bytes of the element)
+              // slots 0, 1 | slots 2, 3 (24-bit: the 48 bytes of the element)
               const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
               float A0[4], G0[4];
-              decode(lds_u4(a0), lds_u4(a0 + plane), QG24 ? lds_u4(a0 + 2 * plane) : z4, A0, G0);
-              rot_pairs(A0, G0, fv2.x, j);
-              decode(lds_u4(a1), lds_u4(a1 + plane), QG24 ? lds_u4(a1 + 2 * plane) : z4, A0, G0);
-              rot_pairs(A0, G0, fv2.y, j + 1);
+              decode(lds_u4(a0), lds_u4(a0 + plane), Q24 ? lds_u4(a0 + 2 * plane) : z4, A0, G0);
+              slot_pairs(A0, G0, fv2.x, j);
+              decode(lds_u4(a1), lds_u4(a1 + plane), Q24 ? lds_u4(a1 + 2 * plane) : z4, A0, G0);
+              slot_pairs(A0, G0, fv2.y, j + 1);
             }
           } else {
             // window not staged: read the elements from global memory (zero
@@ -1048,32 +1226,15 @@ __global__ void __launch_bounds__(256 + 32, OCC)
               const int row = g.e0 + (int)(__float_as_uint(t) - kMagicBits);
               uint4 L0 = zero, L1 = zero, L2 = zero;
               if (col_ok && row >= 0 && row < ja.qg_rows) {
-                const uint4* p = ja.qg + ((size_t)grp * ja.qg_rows + row) * NPL * ja.qg_pitch + col;
+                const uint4* p = ja.qg + ((size_t)g.grp * ja.qg_rows + row) * NPL * ja.qg_pitch + col;
                 L0 = __ldg(p);
                 L1 = __ldg(p + ja.qg_pitch);
-                if (QG24) L2 = __ldg(p + 2 * ja.qg_pitch);
+                if (Q24) L2 = __ldg(p + 2 * ja.qg_pitch);
               }
               float A[4], G[4];
               decode(L0, L1, L2, A, G);
-              rot_pairs(A, G, fv, j);
+              slot_pairs(A, G, fv, j);
             }
-          }
-        } else {
-          const uint32_t sub = (uint32_t)g.sub;
-          float wa[4], wb[4], Wr[4];
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            Wr[r] = __fmul_rn(W, g.ws[r]);
-            wb[r] = __fmul_rn(Wr[r], fu);
-            wa[r] = __fsub_rn(Wr[r], wb[r]);
-          }
-#pragma unroll
-          for (int j = 0; j < NY; ++j) {
-            const float v = fmaf((float)j, dvv, vl);
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-              tap<LAYOUT>(v, c0 + r * sub, RB, wa[r], wb[r], fu, Wr[r],
-                          acc[r][j]);
           }
         }
       } else {
@@ -1086,13 +1247,17 @@ __global__ void __launch_bounds__(256 + 32, OCC)
       e = 0;
       ph ^= 1;
     }
+    turned = (flags & kQTurn) != 0;
   };
   // the item's sums into its voxels: four rotated columns,
   // (x, z) -> (n-1-z, x) -> (n-1-x, n-1-z) -> (z, n-1-x)
   auto store = [&]() {
     const BPArgs& ja = job_args<MULTI>(a, qq, jb);
-    const ItemTile til = item_tile<QG, NY>(ja, MULTI ? item - qq.jobs[jb].item0 + qq.jobs[jb].t0 : item,
-                                           MULTI ? qq.jobs[jb].nbh : a.ntx >> 1);
+    const ItemTile til = item_tile<TY>(ja, MULTI ? item - qq.jobs[jb].item0 + qq.jobs[jb].t0 : item,
+                                       MULTI ? qq.jobs[jb].nbh : a.ntx >> 1);
+    // four turns bring the sums back to the first view's slots, where rotation
+    // r sits in slot r + its quarter: move it to slot r
+    for (int i = (4 - til.k0 / (ja.nviews >> 2)) & 3; i > 0; --i) turn();
     const int n = ja.nx;
     const int ix = til.ix0 + tx, iz = til.iz0 + tz;
     const int cx[4] = {ix, n - 1 - iz, n - 1 - ix, iz};
@@ -1106,7 +1271,7 @@ __global__ void __launch_bounds__(256 + 32, OCC)
       float* out = vol + ((size_t)cz[r] * ystride) * n + cx[r];
 #pragma unroll
       for (int j = 0; j < NY; ++j) {
-        const int iy = til.iy0 + j;
+        const int iy = til.iy0 + ty + j;
         if (iy < ny) {
           float val = acc[r][j] * scale;
           if (iy < ylim) val = fmaxf(val, 0.f);
@@ -1122,25 +1287,15 @@ __global__ void __launch_bounds__(256 + 32, OCC)
     // one work item, K quads (as many as views): a loop of known length
     item = (long long)blockIdx.y * gridDim.x + blockIdx.x;
     const int K = a.nviews;
-    if constexpr (QG) {
-      grp = item_tile<QG, NY>(a, item, a.ntx >> 1).g0;
-      const int Q = K >> 2;
-      for (int q = 0; q < K; q += 4) {
-        step(std::integral_constant<int, 0>{});
-        if (stop) break;
-        step(std::integral_constant<int, 1>{});
-        if (stop) break;
-        step(std::integral_constant<int, 2>{});
-        if (stop) break;
-        step(std::integral_constant<int, 3>{});
-        if (stop) break;
-        if (++grp == Q) grp = 0;
-      }
-    } else {
-      for (int q = 0; q < K; ++q) {
-        step(std::integral_constant<int, 0>{});
-        if (stop) break;
-      }
+    // the four quarter turns, the first one entered at its view k0 mod Q and
+    // finished at the end (the turns stay out of the inner loop)
+    const int Q = K >> 2, first = Q - item_tile<TY>(a, item, a.ntx >> 1).k0 % Q;
+    int left = K;
+    for (int n = first; left > 0 && !stop; n = min(Q, left)) {
+      left -= n;
+#pragma unroll 2
+      for (int q = 0; q < n; ++q) { step(); if (stop) break; }
+      if (turned) turn();
     }
     if (bad) atomicCAS(a.err, 0, kDevFootprint);
     if (stop || *s_abort) return;
@@ -1148,22 +1303,10 @@ __global__ void __launch_bounds__(256 + 32, OCC)
     return;
   }
   for (;;) {
-    if constexpr (QG) {
-      // a group of four quads (an item's quads come in whole groups)
-      step(std::integral_constant<int, 0>{});
-      if (stop || leave) break;
-      step(std::integral_constant<int, 1>{});
-      if (stop) break;
-      step(std::integral_constant<int, 2>{});
-      if (stop) break;
-      step(std::integral_constant<int, 3>{});
-      if (stop) break;
-      const int Qj = job_args<MULTI>(a, qq, jb).nviews >> 2;
-      if (++grp == Qj) grp = 0;
-    } else {
-      step(std::integral_constant<int, 0>{});
-      if (stop || leave) break;
-    }
+    do step();
+    while (!(stop || leave || turned || last));
+    if (stop || leave) break;
+    if (turned) turn();
     if (last) {
       if (bad) atomicCAS(job_args<MULTI>(a, qq, jb).err, 0, kDevFootprint);
       bad = false;
@@ -1284,46 +1427,64 @@ cudaError_t launch_cfg(const BoxMaps& maps, const BPArgs& a, size_t smem, cudaSt
   return cudaGetLastError();
 }
 
-template <int LAYOUT, int NY, int OCC>
+template <int LAYOUT, int NY, int YW, int OCC>
 cudaError_t launch_quad_cfg(const BoxMaps& maps, const BPArgs& a, size_t smem, cudaStream_t stream) {
-  auto kern = bp_quad_kernel<LAYOUT, NY, OCC, false>;
+  auto kern = bp_quad_kernel<LAYOUT, NY, YW, OCC, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   if (e != cudaSuccess) return e;
   // all of L1 as shared memory, so that two CTAs of up to 113 KB share an SM
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  dim3 grid((a.ntx / 2) * (a.ntz / 2), (a.ny + NY - 1) / NY);
-  kern<<<grid, 256 + 32, smem, stream>>>(maps, a, QuadQueue{});
+  dim3 grid((a.ntx / 2) * (a.ntz / 2), (a.ny + NY * YW - 1) / (NY * YW));
+  kern<<<grid, quad_threads(LAYOUT, NY, YW), smem, stream>>>(maps, a, QuadQueue{});
   return cudaGetLastError();
 }
 
-template <int NY, int OCC>
-cudaError_t launch_quad_ny(int layout, const BoxMaps& maps, const BPArgs& a, size_t smem, cudaStream_t stream) {
-  switch (layout) {
-    case kLayoutPair32:
-      return launch_quad_cfg<kLayoutPair32, NY, OCC>(maps, a, smem, stream);
-    case kLayoutPair16:
-      return launch_quad_cfg<kLayoutPair16, NY, OCC>(maps, a, smem, stream);
-    case kLayoutQuadG16:
-      return launch_quad_cfg<kLayoutQuadG16, NY, OCC>(maps, a, smem, stream);
-    case kLayoutQuadG24:
-      return launch_quad_cfg<kLayoutQuadG24, NY, OCC>(maps, a, smem, stream);
-    default:
-      return launch_quad_cfg<kLayoutRaw32, NY, OCC>(maps, a, smem, stream);
+// The kernel shape of a staged layout and tile height (quad_tile_ny's values).
+#define FBP_QUAD_SHAPES(LAUNCH)                                                              \
+  switch (layout) {                                                                          \
+    case kLayoutQuadG16:                                                                     \
+      return ny_tile == 8    ? LAUNCH(kLayoutQuadG16, 8, 1, 2)                               \
+             : ny_tile == 16 ? LAUNCH(kLayoutQuadG16, 8, 2, 1)                               \
+                             : LAUNCH(kLayoutQuadG16, 12, 2, 1);                             \
+    case kLayoutQuadG24:                                                                     \
+      return ny_tile == 8    ? LAUNCH(kLayoutQuadG24, 8, 1, 2)                               \
+             : ny_tile == 12 ? LAUNCH(kLayoutQuadG24, 12, 1, 2)                              \
+                             : LAUNCH(kLayoutQuadG24, 16, 1, 1);                             \
+    default:                                                                                 \
+      return ny_tile == 8    ? LAUNCH(kLayoutQuad32, 8, 1, 2)                                \
+             : ny_tile == 12 ? LAUNCH(kLayoutQuad32, 12, 1, 2)                               \
+                             : LAUNCH(kLayoutQuad32, 16, 1, 1);                              \
   }
-}
 
 cudaError_t launch_quad(int layout, int ny_tile, const BoxMaps& maps, const BPArgs& a, size_t smem,
                         cudaStream_t stream) {
-  return ny_tile == 16 ? launch_quad_ny<16, 1>(layout, maps, a, smem, stream)
-                       : launch_quad_ny<8, 2>(layout, maps, a, smem, stream);
+#define FBP_LAUNCH(L, NY, YW, OCC) launch_quad_cfg<L, NY, YW, OCC>(maps, a, smem, stream)
+  FBP_QUAD_SHAPES(FBP_LAUNCH)
+#undef FBP_LAUNCH
+}
+
+int quad_occ(int ny_tile) { return ny_tile == 8 || ny_tile == 12 ? 2 : 1; }
+
+// Tile height of a symmetric backprojection: the caller's (8 or 16), or the one
+// with the least work on the fullest SM, ceil(tiles / SMs) x height, times what
+// a voxel costs in that shape on a large volume (512^3, 720 views; 480^3 at the
+// 1440^3 geometry). MIXED: 24 0.94 of 16 (36.6 against 37.3 ms; 14.7 against
+// 16.2); FP32 and 24-bit: 12 0.95 of 8 (37.2 against 38.1 and 46.7 against 49.3
+// ms; 17.6 against 18.9 and 19.7 against 20.2).
+int quad_tile_height(int asked, int layout, int orbits, int ny, int num_sms) {
+  if (asked) return asked;
+  auto cost = [&](int h, double rel) {
+    const long long tiles = (long long)orbits * ((ny + h - 1) / h);
+    return (double)((tiles + num_sms - 1) / num_sms) * h * rel;
+  };
+  if (layout == kLayoutQuadG16) return cost(24, 0.94) < cost(16, 1.0) ? 24 : 16;
+  return cost(12, 0.95) < cost(8, 1.0) ? 12 : 8;
 }
 
 template <int TX, int TZ, int NY>
 cudaError_t launch_layout(int layout, const BoxMaps& maps, const BPArgs& a, size_t smem, cudaStream_t stream) {
   switch (layout) {
-    case kLayoutPair32:
-      return launch_cfg<kLayoutPair32, TX, TZ, NY>(maps, a, smem, stream);
     case kLayoutPair16:
       return launch_cfg<kLayoutPair16, TX, TZ, NY>(maps, a, smem, stream);
     default:
@@ -1509,11 +1670,12 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     return set_error(ctx, FBP_ERR_UNSUPPORTED,
                      "the four-fold symmetric backprojector needs nx == nz (a multiple of 32), views % 4 == 0 and "
                      "views over one full turn");
-  // MIXED forms over f32 rows: packed for the selected kernel below
-  const bool packed = mixed && !st.filtered && (quad || !c24);
-  const int layout = st.filtered ? st.filt_layout
-                     : packed    ? (quad ? (c24 ? kLayoutQuadG24 : kLayoutQuadG16) : kLayoutPair16)
-                                 : kLayoutRaw32;
+  // what the selected kernel reads: interleaved quads (symmetric), FP16 pairs
+  // (MIXED) or the FP32 rows themselves
+  const bool packed = quad || (mixed && !c24);
+  const int layout = quad ? (!mixed ? kLayoutQuad32 : c24 ? kLayoutQuadG24 : kLayoutQuadG16)
+                     : packed ? kLayoutPair16
+                              : kLayoutRaw32;
   const int esize = Stack::elem_bytes(layout);
   BPArgs a{};
   a.vol = vol;
@@ -1545,9 +1707,9 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   a.inv_scale = (layout == kLayoutPair16 || layout == kLayoutQuadG16) ? st.inv_scale : nullptr;
   // TMA: x * element size must be a multiple of 16 bytes (the interleaved
   // layouts' x counts 8-byte words, two per 16-byte plane element: always even)
-  a.align = is_quad_layout(layout) ? 1 : layout == kLayoutPair32 ? 2 : 4;
+  a.align = is_quad_layout(layout) ? 1 : 4;
   a.sino_layout = st.sinogram ? 1 : 0;
-  a.pair_rows = layout == kLayoutRaw32 ? 0 : 1;
+  a.pair_rows = is_pair_layout(layout) ? 1 : 0;
   a.clip_ylimit = clip_ylimit;
   a.err = ctx->d_err;
 
@@ -1556,11 +1718,10 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   a.trig = ctx->d_trig;
 
   // tile configuration: 16 x 16 columns, NY voxels along y (1 for 2D)
-  // symmetric kernel: 16 voxels per thread along y with one CTA per SM, or 8
-  // with two (a per-context choice; 0 = 16)
-  const int quad_ny = ctx->quad_tile_ny == 8 ? 8 : 16;
-  const int TX = 16, TZ = 16,
-            NY = is2d ? 1 : quad ? quad_ny : (ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC_Y8 ? 8 : 16);
+  const int TX = 16, TZ = 16, orbits = (g.nx / 32) * (g.nx / 32);
+  const int NY = is2d   ? 1
+                 : quad ? quad_tile_height(ctx->quad_tile_ny, layout, orbits, g.ny, ctx->num_sms)
+                        : (ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC_Y8 ? 8 : 16);
   a.ntx = (g.nx + TX - 1) / TX;
   a.ntz = (g.nz + TZ - 1) / TZ;
   const int nty = (g.ny + NY - 1) / NY;
@@ -1605,7 +1766,11 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     // few blocks: each adds its whole shared histogram to the global one
     const int blocks = (int)std::max(1LL, std::min<long long>((ntiles + 7) / 8, (long long)ctx->num_sms * 2));
     const size_t hist_smem = sizeof(unsigned) * kBoxHist * kBoxHist;
-    auto fk = is2d ? footprint_kernel<16, 16, 1> : NY == 8 ? footprint_kernel<16, 16, 8> : footprint_kernel<16, 16, 16>;
+    auto fk = is2d       ? footprint_kernel<16, 16, 1>
+              : NY == 8  ? footprint_kernel<16, 16, 8>
+              : NY == 12 ? footprint_kernel<16, 16, 12>
+              : NY == 16 ? footprint_kernel<16, 16, 16>
+                         : footprint_kernel<16, 16, 24>;
     if (cuda_check(ctx, cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_smem),
                    "footprint_kernel shared memory"))
       return FBP_ERR_CUDA;
@@ -1631,27 +1796,36 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   }
   const int bu = (plan.box_u + a.align - 1) / a.align * a.align;
   // a pair element carries row v + 1 with it: one row less to stage
-  const int bv = layout == kLayoutRaw32 ? plan.box_v : std::max(1, plan.box_v - 1);
-  if (!is_quad_layout(layout) && ((layout == kLayoutPair32 ? 2 * bu : bu) > 256 || bv > 256))
+  const int bv = a.pair_rows ? std::max(1, plan.box_v - 1) : plan.box_v;
+  // Limits of the FP32 form: windows of filtered rows up to 128 x 257 samples,
+  // of other rows up to 256 x 256 (what a staged box of them holds), the
+  // symmetric kernel's four together at most the ring
+  const bool fp32 = layout == kLayoutRaw32 || layout == kLayoutQuad32;
+  const int fu = st.filtered ? (plan.box_u + 1) / 2 * 2 : (plan.box_u + 3) / 4 * 4;
+  const int fv = st.filtered ? std::max(1, plan.box_v - 1) : plan.box_v;
+  if ((fp32 && ((st.filtered ? 2 * fu : fu) > 256 || fv > 256)) || (!is_quad_layout(layout) && (bu > 256 || bv > 256)))
     return set_error(ctx, FBP_ERR_UNSUPPORTED,
                      "detector footprint of a voxel tile exceeds the 256-element TMA box; geometry magnification "
                      "too large for the staged backprojector");
   a.box_u = bu;
   a.box_v = bv;
-  // two CTAs per SM: each gets half of the 228 KB shared memory; the
-  // symmetric kernel with 16 voxels per thread runs one CTA per SM
-  const int occ = (quad && NY == 16) ? 1 : 2;
+  // two CTAs per SM: each gets half of the 228 KB shared memory
+  const int occ = quad ? quad_occ(NY) : 2;
   const size_t smem_cap = occ == 1 ? (size_t)kMaxDynamicSmem : 113 * 1024;
   const size_t max_box = (size_t)(bu * bv * esize + 127) / 128 * 128;
   size_t smem = 0;
   bool use_quad = quad;
   if (use_quad) {
     // byte ring for the windows + entry records
-    const size_t fixed = kQuadEntries * (sizeof(QuadCoef) + 2 * sizeof(uint64_t) + sizeof(long long)) + 64;
+    const size_t fixed = kQuadEntries * (sizeof(QuadCoef) + 2 * sizeof(uint64_t) + sizeof(long long)) +
+                         2 * kGeoQuads * sizeof(QuadStage) + 64;
     const size_t ring = (smem_cap - fixed) / 128 * 128;
-    // the interleaved layout gathers windows that do not fit from global memory
-    const size_t entry = is_quad_layout(layout) ? 0 : 4 * max_box;
-    if (entry > ring) {
+    // Windows that do not fit are gathered from global memory; the FP32 form
+    // keeps to the generic kernel where four separate windows of its rows
+    // (pairs of rows when filtered) would not fit an SM (half, tile height 8)
+    const size_t entry = fp32 ? 4 * (((size_t)fu * fv * (st.filtered ? 8 : 4) + 127) / 128 * 128) : 0;
+    const size_t limit = ((ctx->quad_tile_ny == 8 ? 113 * 1024 : (size_t)kMaxDynamicSmem) - 1024) / 128 * 128;
+    if (entry > limit) {
       use_quad = false;  // the largest quad does not fit: generic path
       if (ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC)
         return set_error(ctx, FBP_ERR_UNSUPPORTED, "detector windows too large for the symmetric backprojector");
@@ -1687,15 +1861,14 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   if (is_quad_layout(layout)) {
     a.qg = static_cast<const uint4*>(st.filt);
     a.qg_pitch = st.filt_pitch;
-    a.qg_rows = st.v + 1;
+    a.qg_rows = st.v + a.pair_rows;
   }
-  // the grid of boxes over the filtered stack (4-byte elements; float2 as two floats)
-  const bool from_filt = st.filtered || packed;
-  const void* base = from_filt ? st.filt : (const void*)st.f32;
-  const int pitch_el = from_filt ? st.filt_pitch : st.pitch;
+  // the grid of boxes over the staged views (4-byte elements, or 16-byte planes)
+  const void* base = packed ? st.filt : (const void*)st.f32;
+  const int pitch_el = packed ? st.filt_pitch : st.pitch;
   const uint64_t pitch_bytes = (uint64_t)pitch_el * esize;
-  const uint64_t ux = layout == kLayoutPair32 ? 2ull * st.u : (uint64_t)st.u;
-  const uint64_t rows_v = layout == kLayoutRaw32 ? (uint64_t)st.v : (uint64_t)st.v + 1;  // element rows per view
+  const uint64_t ux = (uint64_t)st.u;
+  const uint64_t rows_v = (uint64_t)st.v + a.pair_rows;  // element rows per view
   BoxMaps maps;
   // interleaved layout: boxes of at most 128 x 256 elements (TMA: 256 words per
   // box row) and at most the ring; larger windows are gathered directly
@@ -1713,9 +1886,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   if (!(plan.sel_layout == layout && plan.sel_u == mbu && plan.sel_v == mbv)) {
     // the interleaved layouts take the boxes fitted to the histogram (C4: the
     // MIXED backprojection 1405 -> 1289 ms); the others keep the quarter steps
-    // of the largest window, measured faster for the FP32 pairs (1835 vs 1884
-    // ms at C4: their shared-memory row stride, 8 bytes x the box width, meets
-    // bank conflicts at some fitted widths)
+    // of the largest window
     static const std::vector<unsigned> no_hist;
     choose_boxes(is_quad_layout(layout) ? plan.hist : no_hist, mbu, mbv, a.align, a.pair_rows, planes, plan.sel_w,
                  plan.sel_h);
@@ -1737,7 +1908,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
           return rc;
         continue;
       }
-      const uint32_t box_x = layout == kLayoutPair32 ? 2 * maps.w[i] : maps.w[i];  // in 4-byte elements
+      const uint32_t box_x = maps.w[i];
       uint64_t dims[3], strides[2];
       uint32_t box[3];
       if (st.sinogram) {  // [v][view][u]
@@ -1811,31 +1982,24 @@ long long bp_plan_batch_key(const BPLaunchPlan& p) {
 
 namespace {
 
-template <int LAYOUT, int NY, int OCC>
+template <int LAYOUT, int NY, int YW, int OCC>
 cudaError_t launch_quad_multi_cfg(const QuadQueue& qq, size_t smem, int grid, cudaStream_t stream) {
-  auto kern = bp_quad_kernel<LAYOUT, NY, OCC, true>;
+  auto kern = bp_quad_kernel<LAYOUT, NY, YW, OCC, true>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   static const BoxMaps no_maps{};
   static const BPArgs no_args{};
-  kern<<<grid, 256 + 32, smem, stream>>>(no_maps, no_args, qq);
+  kern<<<grid, quad_threads(LAYOUT, NY, YW), smem, stream>>>(no_maps, no_args, qq);
   return cudaGetLastError();
 }
 
-template <int NY, int OCC>
-cudaError_t launch_quad_multi_ny(int layout, const QuadQueue& qq, size_t smem, int grid, cudaStream_t stream) {
-  switch (layout) {
-    case kLayoutPair32:
-      return launch_quad_multi_cfg<kLayoutPair32, NY, OCC>(qq, smem, grid, stream);
-    case kLayoutQuadG16:
-      return launch_quad_multi_cfg<kLayoutQuadG16, NY, OCC>(qq, smem, grid, stream);
-    case kLayoutQuadG24:
-      return launch_quad_multi_cfg<kLayoutQuadG24, NY, OCC>(qq, smem, grid, stream);
-    default:
-      return cudaErrorInvalidValue;  // other layouts run one launch per job
-  }
+cudaError_t launch_quad_multi(int layout, int ny_tile, const QuadQueue& qq, size_t smem, int grid,
+                              cudaStream_t stream) {
+#define FBP_LAUNCH(L, NY, YW, OCC) launch_quad_multi_cfg<L, NY, YW, OCC>(qq, smem, grid, stream)
+  FBP_QUAD_SHAPES(FBP_LAUNCH)
+#undef FBP_LAUNCH
 }
 
 }  // namespace
@@ -1854,8 +2018,6 @@ int launch_bp_batch(fbp_context* L, BPLaunchPlan* const* plans, int n, const lon
   const BPLaunchPlan& p0 = *plans[0];
   const long long key = bp_plan_batch_key(p0);
   if (key == 0) return set_error(L, FBP_ERR_INVALID_ARGUMENT, "backprojection plan cannot run in a batch");
-  if (p0.layout != kLayoutPair32 && p0.layout != kLayoutQuadG16 && p0.layout != kLayoutQuadG24)
-    return set_error(L, FBP_ERR_UNSUPPORTED, "batched backprojection supports FP32 pairs and interleaved quads");
   const size_t jobs_bytes = (sizeof(QuadJob) * n + 63) / 64 * 64;
   const size_t maps_bytes = sizeof(BoxMaps) * n;
   const size_t bytes = jobs_bytes + maps_bytes + 64;
@@ -1916,8 +2078,7 @@ int launch_bp_batch(fbp_context* L, BPLaunchPlan* const* plans, int n, const lon
   qq.err = L->d_err;
   qq.ring = p0.a.box_bytes;
   const int grid = (int)std::min<long long>(items, (long long)p0.occ * L->num_sms);
-  cudaError_t e = p0.ny_tile == 16 ? launch_quad_multi_ny<16, 1>(p0.layout, qq, p0.smem, grid, L->stream)
-                                   : launch_quad_multi_ny<8, 2>(p0.layout, qq, p0.smem, grid, L->stream);
+  cudaError_t e = launch_quad_multi(p0.layout, p0.ny_tile, qq, p0.smem, grid, L->stream);
   if (e == cudaSuccess) L->launches++;
   return cuda_check(L, e, "bp_quad_kernel (batch)");
 }

@@ -378,37 +378,12 @@ __global__ void __launch_bounds__(256, fft_ebits(L) == 4 ? 2 : 3) filter_fft_ker
     for (int i = 0; i < E; ++i) x[i] = make_float2(x[i].x * h[i], x[i].y * h[i]);
     dit_regs<E, REM>(x);
     fft_inverse<L, NP - 2>(x, a.tws, t, at, sync);
-    const int v0 = rs.out_layout == kLayoutPair32 ? (int)(r0 % rs.n_v) : 0;
-    if (rs.out_layout == kLayoutPair32 && !rs.sinogram && two && v0 + 1 < rs.n_v) {
-      // rows v0, v0 + 1 of one view: element v0 + 1 whole, the near halves of its neighbours
-      float2* o0 = static_cast<float2*>(rs.out) + pair_row(rs, (int)(r0 / rs.n_v), v0) * rs.out_pitch + t;
-      float2 *o1 = o0 + rs.out_pitch, *o2 = o1 + rs.out_pitch;
-      const bool first = v0 == 0, last = v0 + 1 == rs.n_v - 1;
+    float* d0 = rs.data + r0 * rs.pitch + t;
 #pragma unroll
-      for (int i = 0; i < E; ++i) {
-        if (i * T >= left) continue;
-        o1[i * T] = x[i];
-        o0[i * T].y = x[i].x;
-        o2[i * T].x = x[i].y;
-        if (first) o0[i * T].x = 0.f;
-        if (last) o2[i * T].y = 0.f;
-      }
-    } else if (rs.out_layout == kLayoutRaw32) {
-      float* d0 = rs.data + r0 * rs.pitch + t;
-#pragma unroll
-      for (int i = 0; i < E; ++i) {
-        if (i * T >= left) continue;
-        d0[i * T] = x[i].x;
-        if (two) d0[rs.pitch + i * T] = x[i].y;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < E; ++i) {
-        const int c = t + i * T;
-        if (c >= rs.m) continue;
-        store_row_sample(rs, r0, c, x[i].x);
-        if (two) store_row_sample(rs, r0 + 1, c, x[i].y);
-      }
+    for (int i = 0; i < E; ++i) {
+      if (i * T >= left) continue;
+      d0[i * T] = x[i].x;
+      if (two) d0[rs.pitch + i * T] = x[i].y;
     }
   }
 }
@@ -664,6 +639,26 @@ __global__ void pack_quadg24_kernel(const float* src, long long spitch, int m, i
   }
 }
 
+// f32 rows -> kLayoutQuad32: the four views' samples of one detector pixel as
+// one 16-byte element. Grid: x over columns, y over detector rows, z over view
+// groups. 4 bytes read and 4 written per sample.
+__global__ void __launch_bounds__(256) pack_quad32_kernel(const float* __restrict__ src, long long spitch, int m,
+                                                          int n_views, int n_v, bool sinogram,
+                                                          float4* __restrict__ out) {
+  const int Q = n_views >> 2, g = blockIdx.z, c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m) return;
+  for (int iv = blockIdx.y; iv < n_v; iv += gridDim.y) {
+    float v[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int view = g + s * Q;
+      const long long r = sinogram ? (long long)iv * n_views + view : (long long)view * n_v + iv;
+      v[s] = __ldg(src + r * spitch + c);
+    }
+    out[((long long)g * n_v + iv) * m + c] = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
 // Natural-order complex FFT of rows (FFFT::fft_radix2 / inverse_fft_radix2,
 // FastFourierTransformGPU.cpp:3-36): inverse = conj, FFT, conj, divide by n.
 __global__ void __launch_bounds__(256) fft_rows_kernel(float2* data, int n, int log2n, int rows,
@@ -716,28 +711,6 @@ __global__ void fft_shift_kernel(float2* data, int n, int rows, int shift) {
       int j = (int)((((long long)i + shift) % n + n) % n);
       row[j] = buf[i];
     }
-  }
-}
-
-__global__ void unpack_rows_kernel(const void* src, int layout, long long spitch, const float* inv_scale,
-                                   int n_views, int n_v, bool sinogram, long long row0, long long row_step,
-                                   long long nrows, int m, float* dst, long long dpitch) {
-  long long total = nrows * m;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    long long r = e / m;
-    int i = (int)(e - r * m);
-    long long gr = row0 + r * row_step;
-    const int view = sinogram ? (int)(gr % n_views) : (int)(gr / n_v);
-    const int iv = sinogram ? (int)(gr / n_views) : (int)(gr % n_v);
-    // row iv is the .x half of element iv + 1
-    const long long er = sinogram ? (long long)(iv + 1) * n_views + view : (long long)view * (n_v + 1) + iv + 1;
-    float x;
-    if (layout == kLayoutPair32)
-      x = static_cast<const float2*>(src)[er * spitch + i].x;
-    else
-      x = __half2float(static_cast<const __half2*>(src)[er * spitch + i].x) * inv_scale[view];
-    dst[r * dpitch + i] = x;
   }
 }
 
@@ -851,6 +824,14 @@ int launch_pack(fbp_context* ctx, const Stack& s, int layout, void* out, long lo
                                                        static_cast<uint4*>(out));
     return launched(ctx, "pack_quadg24_kernel");
   }
+  if (layout == kLayoutQuad32) {
+    if (s.n % 4) return set_error(ctx, FBP_ERR_UNSUPPORTED, "the interleaved layout needs a multiple of 4 views");
+    if (s.n / 4 > 65535) return set_error(ctx, FBP_ERR_UNSUPPORTED, "the interleaved layout takes up to 262140 views");
+    const dim3 grid((s.u + 255) / 256, std::min(s.v, 65535), s.n / 4);
+    pack_quad32_kernel<<<grid, 256, 0, ctx->stream>>>(s.f32, s.pitch, s.u, s.n, s.v, s.sinogram,
+                                                      static_cast<float4*>(out));
+    return launched(ctx, "pack_quad32_kernel");
+  }
   return set_error(ctx, FBP_ERR_INVALID_ARGUMENT, "unknown packed layout");
 }
 
@@ -877,15 +858,6 @@ int launch_fft_shift_rows(fbp_context* ctx, float2* data, int n, int rows, int s
   fft_shift_kernel<<<std::min(rows, ctx->num_sms * 4), 256, sizeof(float2) * n, ctx->stream>>>(data, n, rows,
                                                                                                 shift);
   return launched(ctx, "fft_shift_kernel");
-}
-
-int launch_unpack_rows(fbp_context* ctx, const Stack& s, size_t row0, size_t nrows, float* dst,
-                       long long dst_pitch, long long row_step) {
-  if (nrows == 0) return FBP_OK;
-  unpack_rows_kernel<<<grid_for(ctx, (long long)nrows * s.u, 256), 256, 0, ctx->stream>>>(
-      s.filt, s.filt_layout, s.filt_pitch, s.inv_scale, s.n, s.v, s.sinogram, (long long)row0, row_step,
-      (long long)nrows, s.u, dst, dst_pitch);
-  return launched(ctx, "unpack_rows_kernel");
 }
 
 }  // namespace fbp

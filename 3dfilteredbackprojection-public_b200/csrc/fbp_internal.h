@@ -21,13 +21,13 @@ enum DeviceError : int {
   kDevGeometry = 3,   // a voxel lies at or behind the source plane
 };
 
-// Layout of filtered views kept for the backprojector. A pair layout has
+// Layout of the views as the backprojector stages them. The pair layout has
 // nv + 1 element rows per view; element e at column u holds the samples of
-// detector rows e - 1 and e (zero outside the detector), so one
-// shared-memory load yields both rows of a bilinear tap for v in [e-1, e).
+// detector rows e - 1 and e (zero outside the detector), so one shared-memory
+// load yields both rows of a bilinear tap for v in [e-1, e).
 enum FiltLayout : int {
-  kLayoutRaw32 = 0,   // plain FP32 rows (unfiltered data, 2D staging)
-  kLayoutPair32 = 1,  // float2 (8 bytes / sample), FP32 form
+  kLayoutRaw32 = 0,   // plain FP32 rows (FP32 form off the symmetric kernel, unfiltered data)
+  // 1 was FP32 row pairs
   kLayoutPair16 = 2,  // half2 (4 bytes / sample) with a per-view scale, MIXED form
   // Four views interleaved per detector element, for the four-fold symmetric
   // backprojector (MIXED form). Views k = g + s K/4 (s = 0..3) form group g;
@@ -46,29 +46,35 @@ enum FiltLayout : int {
   // bits. No scale (the FP32 exponent is kept). 4 slots x 4 values x 3 bytes
   // = 48 bytes per element, three 16-byte planes per element row.
   kLayoutQuadG24 = 4,
+  // Four views interleaved per detector sample (FP32 form): element (g, v, u)
+  // holds the FP32 samples of views g + s K/4, s = 0..3. 16 bytes per element,
+  // one plane; a tap reads two columns of two rows.
+  kLayoutQuad32 = 5,
 };
 
-constexpr bool is_quad_layout(int layout) { return layout == kLayoutQuadG16 || layout == kLayoutQuadG24; }
+constexpr bool is_quad_layout(int layout) { return layout >= kLayoutQuadG16; }
+// Layouts whose element carries its neighbours (one element row more than detector rows).
+constexpr bool is_pair_layout(int layout) { return layout == kLayoutPair16 || layout == kLayoutQuadG16 || layout == kLayoutQuadG24; }
 
 // A stack of detector rows. Projections are [view][v][u] (rows ordered view
 // major), sinograms [v][view][u] (rows ordered v major). Rows of u samples
 // are padded to `pitch` elements so that every row starts 16-byte aligned.
-// After filtering, the stack's content is the filtered buffer `filt` (in a
-// pair layout) and f32 still holds the unfiltered input.
+// The rows are filtered in place; the backprojection call packs them into
+// `filt` in the layout of the kernel it selects.
 struct Stack {
   float* f32 = nullptr;
   int u = 0, v = 0, n = 0;
   int pitch = 0;  // f32 row pitch in elements (multiple of 4)
   bool sinogram = false;
-  bool filtered = false;          // content lives in filt
+  bool filtered = false;          // the rows went through the FP32 form's filter
   void* filt = nullptr;
   size_t filt_bytes = 0;
-  int filt_layout = kLayoutPair32;
+  int filt_layout = kLayoutRaw32;
   int filt_pitch = 0;             // elements per row of filt (multiple of 4)
   float* inv_scale = nullptr;     // per view (x2: [inv | scale]) for the FP16 layouts
   int scale_cap = 0;              // views inv_scale has room for
   size_t f32_cap = 0;             // bytes allocated at f32 (buffers only grow: no cudaFree between jobs)
-  bool pack_ready = false;        // filt already holds the packed FP16 views of f32 (slabs of one reconstruction)
+  bool pack_ready = false;        // filt already holds f32 packed as filt_layout (slabs of one reconstruction)
   // Log normalisation and FDK weights recorded by their calls and applied
   // inside the filter kernel's load (log first, then weight), or by a
   // standalone pass when something else reads the rows first.
@@ -80,10 +86,8 @@ struct Stack {
   size_t rows() const { return (size_t)v * n; }
   size_t bytes32() const { return (size_t)pitch * rows() * sizeof(float); }
   static int elem_bytes(int layout) {
-    return layout == kLayoutQuadG24 ? 48 : layout == kLayoutQuadG16 ? 32 : layout == kLayoutPair32 ? 8 : 4;
+    return layout == kLayoutQuadG24 ? 48 : layout == kLayoutQuadG16 ? 32 : layout == kLayoutQuad32 ? 16 : 4;
   }
-  // element rows of the filtered buffer (pair layouts carry one extra row per view)
-  size_t filt_rows() const { return (size_t)(v + 1) * n; }
 };
 
 struct FilterTables {
@@ -122,7 +126,7 @@ struct fbp_context {
   int pad_len = 0;
   int clip_after_bp = 1;
   int bp_variant = FBP_BACKPROJECTOR_AUTO;
-  int quad_tile_ny = 0;  // symmetric backprojector: voxels per thread along y (8 or 16; 0 = 16)
+  int quad_tile_ny = 0;  // symmetric backprojector: tile height along y (8 or 16; 0 = by volume size and form)
   int det_row_off = 0, det_rows_total = 0;  // fbp_set_detector_rows (0 rows: the whole detector)
   int slab_y0 = 0, slab_ny = 0;             // fbp_set_volume_slab (0 slices: the whole volume)
   int last_bp[5] = {-1, -1, 0, 0, 0};  // variant, layout, box_u, box_v, tile height of the last backprojection
@@ -132,7 +136,7 @@ struct fbp_context {
   static constexpr int kTuneKey = 23;  // geometry, form, layout, slab, GPU
   struct TuneShape {
     int variant = FBP_BACKPROJECTOR_AUTO;
-    int quad_ny = 0;  // symmetric: voxels per thread along y
+    int quad_ny = 0;  // symmetric: tile height along y
     int stages = 0;   // generic: view ring stages
   };
   struct TuneEntry {
@@ -208,7 +212,7 @@ void* scratch(fbp_context* ctx, size_t bytes);
 
 // ---- filter (fbp_filter.cu) ----
 struct RowSet {
-  float* data;          // f32 rows (input; also output when out16 == nullptr)
+  float* data;          // f32 rows, filtered in place
   long long pitch;      // elements
   long long rows;
   int m;                // samples per row
@@ -221,11 +225,6 @@ struct RowSet {
   bool weight = false;
   float w_sdd = 0, w_du = 0, w_dv = 0;
   float w_voff = 0;  // detector-centre offset of the rows (row band of a taller detector)
-  // output: in place into `data` (out == nullptr) or into a pair layout
-  void* out = nullptr;
-  int out_layout = kLayoutRaw32;
-  long long out_pitch = 0;            // elements
-  const float* view_scale = nullptr;  // kLayoutPair16: values are multiplied by it before rounding
 };
 int ensure_filter_tables(fbp_context* ctx, int n, int filter);
 int launch_filter_fft(fbp_context* ctx, const RowSet& rs, int n);
@@ -236,14 +235,10 @@ int launch_elementwise_pre(fbp_context* ctx, const RowSet& rs);  // weight / log
 int launch_view_scales(fbp_context* ctx, const RowSet& rs, float limit, float* view_scale, float* inv_scale);
 // Pack the stack's f32 rows into a compact backprojector layout: kLayoutPair16
 // with row pitch `pitch` elements or kLayoutQuadG16 (FP16 with the per-view
-// scales view_scale), or kLayoutQuadG24 (24-bit, no scale).
+// scales view_scale), kLayoutQuadG24 (24-bit) or kLayoutQuad32 (no scale).
 int launch_pack(fbp_context* ctx, const Stack& s, int layout, void* out, long long pitch, const float* view_scale);
 int launch_fft_rows(fbp_context* ctx, float2* data, int n, int rows, int inverse);
 int launch_fft_shift_rows(fbp_context* ctx, float2* data, int n, int rows, int shift);
-// Copy filtered rows [row0, row0 + nrows) of a pair layout back to FP32 rows.
-// rows row0, row0 + row_step, ... (nrows of them) of the filtered buffer, as FP32 rows of dst
-int launch_unpack_rows(fbp_context* ctx, const Stack& s, size_t row0, size_t nrows, float* dst, long long dst_pitch,
-                       long long row_step = 1);
 bool toeplitz_supported(int m);
 
 // ---- backprojection (fbp_backproject.cu) ----
@@ -260,9 +255,9 @@ struct BPGeom {
   int y_off = 0, ny_total = 0;
   int vol_ystride = 0;  // y-slices between z planes of the output (0: ny); a slab of a whole volume
 };
-// Backproject the stack's content (filt when filtered, else f32 rows). In
-// the MIXED form (`mixed`) f32 content is first packed into the FP16 layout
-// the selected kernel reads (prepare_packed); sums are FP32 in every form.
+// Backproject the stack's rows, packed first into the layout that the
+// selected kernel reads (prepare_packed) where that is not the rows
+// themselves; `mixed`: the reduced layouts. Sums are FP32 in every form.
 int launch_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, int clip_ylimit, bool mixed);
 // The same in two steps: plan (footprint pass, packing, tensor maps; work on
 // ctx's stream) and launch. Plans with the same non-zero batch key can also run

@@ -28,9 +28,8 @@
 // tcgen05.mma.cta_group::1.kind::f16 (M 128, N 256, K 16: 12 per K block), and
 // frees stages with tcgen05.commit; warps 4..7 (one warpgroup, each reading its
 // 32 TMEM lanes) load the FP32 accumulators with tcgen05.ld, stage them
-// through shared memory and write the backprojector's pair layout (FP16 with
-// the per-view scale) with row-contiguous stores. All waits are bounded and
-// TMEM is always released.
+// through shared memory and write the rows in place with row-contiguous
+// stores. All waits are bounded and TMEM is always released.
 
 #include "fbp_internal.h"
 #include "fbp_rows.cuh"
@@ -118,7 +117,7 @@ __device__ __forceinline__ void mma_commit(uint64_t* b) {
 }
 
 struct GemmArgs {
-  RowSet rs;        // output mapping (pair layout) of the whole stack
+  RowSet rs;        // the whole stack's rows (output in place)
   long long row0;   // first stack row of this chunk
   int nrows;        // rows in this chunk
   int m;            // samples per row (N and K extent)
@@ -243,7 +242,7 @@ __global__ void __launch_bounds__(256, 1) toeplitz_gemm_kernel(const __grid_cons
       if (ok && !*s_abort && col < g.m) {
         for (int r = w; r < BM; r += 4) {
           const int lr = rowt + r;
-          if (lr < g.nrows) store_row_sample(g.rs, g.row0 + lr, col, stage[r * kEpiStride + lane]);
+          if (lr < g.nrows) g.rs.data[(g.row0 + lr) * g.rs.pitch + col] = stage[r * kEpiStride + lane];
         }
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");

@@ -422,13 +422,13 @@ class FBP3D:
         """Kernel, staged layout and window box of the last backprojection."""
         v, l, bu, bv, ny = C.c_int(), C.c_int(), C.c_int(), C.c_int(), C.c_int()
         self.ctx.call("fbp_last_backprojection", C.byref(v), C.byref(l), C.byref(bu), C.byref(bv), C.byref(ny))
-        names = {0: "rows32", 1: "pairs32", 2: "pairs16", 3: "quads16", 4: "quads24"}
+        names = {0: "rows32", 2: "pairs16", 3: "quads16", 4: "quads24", 5: "quads32"}
         kernels = {Backprojector.SYMMETRIC: "symmetric", Backprojector.GENERIC_Y8: "generic_y8"}
         return {"kernel": kernels.get(v.value, "generic"),
                 "layout": names.get(l.value, str(l.value)), "box": (bu.value, bv.value), "tile_ny": ny.value}
 
     def set_symmetric_tile(self, voxels_per_thread_y: int) -> None:
-        """Voxels per thread along y of the symmetric backprojector (8, 16; 0 = 16)."""
+        """Tile height along y of the symmetric backprojector (8, 16; 0 = the library's choice)."""
         self.ctx.call("fbp_set_symmetric_tile", int(voxels_per_thread_y))
 
     def set_autotune_cache(self, path) -> None:

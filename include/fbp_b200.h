@@ -53,8 +53,7 @@ extern "C" {
 /* MIXED24: split-BF16 Toeplitz filter, 24-bit filtered views (FP32 with   */
 /*        the low byte dropped: 16 significant bits, FP32 exponent) for the  */
 /*        four-fold symmetric backprojector (FP32 views otherwise), FP32     */
-/*        accumulation. 12 bytes of shared-memory gathers per update (FP32   */
-/*        16, MIXED 8), for inputs whose noise leaves FP16 storage short of  */
+/*        accumulation. For inputs whose noise leaves FP16 storage short of  */
 /*        1e-4 relative error.                                              */
 #define FBP_PRECISION_FP32 0
 #define FBP_PRECISION_MIXED 1
@@ -128,8 +127,9 @@ int fbp_set_backprojector(fbp_context* ctx, int variant);
  * reference, whose backprojection is one fixed shader. */
 int fbp_set_autotune(fbp_context* ctx, int enable);
 /* With autotuning on: the shapes the tuner times are the symmetric kernel
- * with 16 or 8 voxels per thread along y and the generic kernel with 16 or 8
- * voxels per thread, each with its full view ring or a 4-stage one. A cache
+ * with its own choice of tile height, with 16 and with 8, and the generic
+ * kernel with 16 or 8 voxels per thread, each with its full view ring or a
+ * 4-stage one. A cache
  * file (path; NULL or "" = none) keeps the choices across processes: they are
  * read from it on the first tuning and each new choice is appended as one
  * line (key of geometry, form, layout, slab and GPU; shape; time), so another
@@ -140,19 +140,19 @@ int fbp_set_autotune_cache(fbp_context* ctx, const char* path);
 int fbp_autotune_stats(const fbp_context* ctx, int* timed, int* from_cache);
 /* View ring stages of the generic backprojector (2..8; 0 = as many as fit). */
 int fbp_set_view_ring(fbp_context* ctx, int stages);
-/* Voxels per thread along y of the four-fold symmetric backprojector: 16
- * (one CTA per SM, 64 accumulators a thread) or 8 (two CTAs per SM); 0 (the
- * default) = 16. No counterpart in the reference. */
+/* Tile height along y of the four-fold symmetric backprojector: 16 or 8; 0
+ * (the default) = the library's choice by volume size and form (8, 12, 16 or
+ * 24). No counterpart in the reference. */
 int fbp_set_symmetric_tile(fbp_context* ctx, int voxels_per_thread_y);
 /* Device bytes held by ctx's buffers. */
 int fbp_memory_in_use(const fbp_context* ctx, size_t* bytes);
 /* What the last backprojection ran (no counterpart in the reference, whose
  * backprojection is one fixed shader): *variant = FBP_BACKPROJECTOR_GENERIC,
  * _GENERIC_Y8 or _SYMMETRIC; *layout = staged view layout (0 FP32 rows,
- * 1 FP32 row pairs, 2 FP16 row pairs, 3 FP16 four-view gradient quads,
- * 4 24-bit four-view gradient quads);
+ * 2 FP16 row pairs, 3 FP16 four-view gradient quads, 4 24-bit four-view
+ * gradient quads, 5 FP32 four-view quads);
  * *box_u x *box_v = largest staged detector window in elements; *tile_ny =
- * voxels per thread along y. Any output pointer may be NULL. FBP_ERR_STATE
+ * tile height along y. Any output pointer may be NULL. FBP_ERR_STATE
  * before the first backprojection. */
 int fbp_last_backprojection(const fbp_context* ctx, int* variant, int* layout, int* box_u, int* box_v,
                             int* tile_ny);

@@ -130,3 +130,71 @@ def test_fft_filter_pair_layout(fbp, oracle, layout, u, v, n):
     s.ctx.close()
     p = oracle.fdk_weight(oracle.log_normalize(counts.astype(np.float64), 1000.0), sod + odd, width / u, width / u)
     assert relative_rmse(got, oracle.filter_rows(p, 1)) < TOL_ROWS
+
+
+# Backprojection of white noise (no filter): the sum over views is as
+# incoherent as the taps' errors, so the relative error is one tap's. FP32:
+# position rounding, as TOL_BP2D. 24-bit views: 16 significant bits, 2^-17 RMS
+# a value, four values a tap. FP16 views: 2^-12 a value (2.4e-4).
+TOL_BP = {"FP32": 3e-5, "MIXED24": 5e-5, "MIXED": 4e-4}
+
+
+def _noise_bp(fbp, oracle, c, precision, variant, tile=0, sinograms=False):
+    rng = np.random.default_rng(c["nx"] + 7 * c["nviews"])
+    proj = rng.standard_normal((c["nviews"], c["nv"], c["nu"])).astype(np.float32)
+    s = fbp.FBP3D(0)
+    s.set_clip_after_backprojection(False)
+    s.set_precision(getattr(fbp.Precision, precision))
+    s.set_backprojector(getattr(fbp.Backprojector, variant))
+    if tile:
+        s.set_symmetric_tile(tile)
+    args = (c["sod"], c["sdd"] - c["sod"], c["nu"] * c["du"], c["nx"] * c["vox"], c["span"] / (2 * math.pi),
+            c["nx"], c["ny"], c["offset"])
+    if sinograms:
+        s.upload_sinograms(np.ascontiguousarray(proj.transpose(1, 0, 2)))
+        s.project_backward_cone_fdk_from_sinograms(*args)
+    else:
+        s.upload_projections(proj)
+        s.project_backward_cone_fdk_from_projections(*args)
+    got, info = s.read_volume(), s.last_backprojection()
+    s.ctx.close()
+    ref = oracle.bp_cone(proj.astype(np.float64), c)
+    return relative_rmse(got, ref), info
+
+
+@pytest.mark.parametrize("precision", ["FP32", "MIXED", "MIXED24"])
+@pytest.mark.parametrize("tile", [0, 8, 16])
+@pytest.mark.parametrize("n,ny,views,du", [(32, 2, 4, 1.5), (32, 25, 8, 2.25), (64, 13, 12, 1.5), (64, 47, 20, 0.75),
+                                           (96, 24, 36, 0.5), (64, 12, 132, 1.5)])
+def test_symmetric_tile_heights(fbp, oracle, precision, tile, n, ny, views, du):
+    """Every tile height the symmetric kernel has, volumes that end inside a
+    tile, walks shorter than a block of quads, rows that advance by less than
+    one, about one, two and three per voxel."""
+    c = dict(sod=3.0 * n, sdd=4.5 * n, du=du, dv=du, span=2 * math.pi, offset=0.0, nu=int(2.4 * n / du), nv=int(2 * n / du),
+             nviews=views, nx=n, ny=ny, nz=n, vox=1.0)
+    err, info = _noise_bp(fbp, oracle, c, precision, "SYMMETRIC", tile, sinograms=ny == 13)
+    assert info["kernel"] == "symmetric" and (not tile or info["tile_ny"] == tile)
+    assert err < TOL_BP[precision]
+
+
+def test_symmetric_fp32_unstaged_windows(fbp, oracle):
+    """High magnification: windows wider than the widest box (128 elements) are
+    gathered from global memory (zero outside the detector)."""
+    c = dict(sod=120.0, sdd=360.0, du=0.6, dv=0.6, span=2 * math.pi, offset=0.0, nu=330, nv=300, nviews=48, nx=64,
+             ny=40, nz=64, vox=1.0)
+    err, info = _noise_bp(fbp, oracle, c, "FP32", "SYMMETRIC")
+    assert info["kernel"] == "symmetric" and info["layout"] == "quads32"
+    assert info["box"][0] > 128
+    assert err < TOL_BP["FP32"]
+
+
+@pytest.mark.parametrize("precision", ["FP32", "MIXED", "MIXED24"])
+@pytest.mark.parametrize("variant", ["GENERIC", "GENERIC_Y8"])
+@pytest.mark.parametrize("n,ny,views,du", [(17, 1, 3, 1.5), (33, 25, 9, 2.25), (50, 47, 21, 0.75), (30, 16, 35, 0.5)])
+def test_generic_row_steps(fbp, oracle, precision, variant, n, ny, views, du):
+    """The generic kernel's march for every row step, off the symmetric sizes."""
+    c = dict(sod=3.0 * n, sdd=4.5 * n, du=du, dv=du, span=2 * math.pi, offset=0.0, nu=int(2.4 * n / du), nv=int(2 * n / du),
+             nviews=views, nx=n, ny=ny, nz=n, vox=1.0)
+    err, info = _noise_bp(fbp, oracle, c, precision, variant, sinograms=ny == 47)
+    assert info["kernel"] == (variant.lower() if ny > 1 else "generic")  # one slice: the 2D tile
+    assert err < TOL_BP["FP32" if precision == "MIXED24" else precision]
