@@ -580,11 +580,13 @@ int make_tensor_map_2d_bf16_sw128(fbp_context* ctx, CUtensorMap* map, void* base
                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 
-int prepare_packed(fbp_context* ctx, Stack& s, int layout) {
+int prepare_packed(fbp_context* ctx, Stack& s, int layout, const Orbits& o) {
   const bool quad = fbp::is_quad_layout(layout);
-  const int pair = fbp::is_pair_layout(layout) ? 1 : 0;  // one element row (and quad column) more
-  const int fpitch = quad ? s.u + pair : round_up(s.u, 4);
-  const size_t need = (size_t)(quad ? s.n / 4 : s.n) * (s.v + pair) * (size_t)fpitch * Stack::elem_bytes(layout);
+  const int pair = fbp::is_pair_layout(layout) ? 1 : 0;  // one element row more
+  // rows of 16-byte multiples (two 8-byte elements, four 4-byte ones)
+  const int esize = Stack::elem_bytes(layout);
+  const int fpitch = fbp::is_grad_layout(layout) ? s.u + 1 : round_up(s.u, std::max(1, 16 / esize));
+  const size_t need = (size_t)(quad ? o.groups : s.n) * (s.v + pair) * (size_t)fpitch * esize;
   if (!s.filt || s.filt_bytes < need) {
     cudaFree(s.filt);
     s.filt = nullptr;
@@ -603,9 +605,10 @@ int prepare_packed(fbp_context* ctx, Stack& s, int layout) {
   float* scale = s.inv_scale + s.n;
   // the four-term difference of the gradient layout is at most 4 max|value|;
   // the 24-bit layout keeps the FP32 exponent and needs no scale
-  if (layout != kLayoutQuadG24 && layout != kLayoutQuad32)
-    if (int rc = launch_view_scales(ctx, rowset_of(s), quad ? 8192.f : 16384.f, scale, s.inv_scale)) return rc;
-  if (int rc = launch_pack(ctx, s, layout, s.filt, fpitch, scale)) return rc;
+  if (layout == kLayoutQuadG16 || fbp::is_p16_layout(layout))
+    if (int rc = launch_view_scales(ctx, rowset_of(s), layout == kLayoutQuadG16 ? 8192.f : 16384.f, scale, s.inv_scale))
+      return rc;
+  if (int rc = launch_pack(ctx, s, layout, o, s.filt, fpitch, scale)) return rc;
   s.filt_layout = layout;
   s.filt_pitch = fpitch;
   return FBP_OK;

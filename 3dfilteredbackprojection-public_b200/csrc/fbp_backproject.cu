@@ -95,6 +95,10 @@ struct BPArgs {
   // 16-byte entries, [group][element row][plane][element column]
   const uint4* qg;
   int qg_pitch, qg_rows;  // element columns per plane row, element rows per group
+  // orbits of the interleaved layouts (struct Orbits) and their representative
+  // tiles; wrap: slots the sums move by from the last phase back to the first
+  int groups, mirror, wrap;
+  int nbx, nbz;
   int resident;           // CTAs resident on the GPU at once (view-group skew of the interleaved walk)
   int band;               // tile orbits along z in one band of the symmetric kernel's tile order
   int* minmax;            // fold the stored values' min / max into this pair (or nullptr)
@@ -493,9 +497,10 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
         float2 v2 = make_float2(vl, vl + dvv);
         const float2 step2 = make_float2(2.f * dvv, 2.f * dvv), magic2 = make_float2(kMagic, kMagic);
         if constexpr (LAYOUT == kLayoutRaw32) {
-          // march along the column: a voxel's upper row, interpolated in u (the
-          // distance weight folded in), is the next voxel's lower row when the
-          // rows advance by one, so a voxel reads one new row (8 bytes) or two
+          // where the rows advance by less than one per voxel, march along the
+          // column: a voxel's upper row, interpolated in u (the distance weight
+          // folded in), is the next voxel's lower row or its upper one again,
+          // so a voxel reads one new row (8 bytes) instead of two
           const float wb = W * fu, wa = W - wb;
           auto load = [&](uint32_t at) { return fmaf(wb, lds_f32(at + 4), wa * lds_f32(at)); };
           auto march = [&](auto shortc) {
@@ -511,12 +516,8 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
               for (int p = 0; p < 2 && j + p < NY; ++p) {
                 const uint32_t bits = __float_as_uint(p ? t2.y : t2.x);
                 const uint32_t at = bits * RB + c0;
-                if (j + p == 0) {
-                  lo = load(at);
-                } else {
-                  lo = bits == before ? lo : hi;
-                  if (!SHORT && bits - before > 1u) lo = load(at);
-                }
+                if (j + p == 0 || !SHORT) lo = load(at);
+                else lo = bits == before ? lo : hi;
                 hi = load(at + RB);
                 acc[j + p] += fmaf(p ? fv2.y : fv2.x, hi - lo, lo);
                 before = bits;
@@ -626,6 +627,7 @@ constexpr int kQFirst = 4;   // first quad of a work item (a tile orbit and y-sl
 constexpr int kQLast = 8;    // last quad of a work item: the consumers store its voxels next
 constexpr int kQExit = 16;   // multi-job launch: the queue is empty, the CTA leaves
 constexpr int kQTurn = 32;   // last view of a quarter turn: the sums move on by one slot
+constexpr int kQWrap = 128;  // .. from the last phase back to the first
 constexpr int kQShort = 64;  // rows advance by less than one per voxel everywhere in the tile
 
 // 16-byte aligned so that consumers read a record with vector loads: four for
@@ -676,8 +678,6 @@ struct QuadJob {
   BPArgs a;
   long long item0;  // first work item of the job in this launch
   long long t0;     // its tile
-  int nbh;          // representative tiles per axis
-  int nty;          // y-slabs
 };
 struct QuadQueue {
   const QuadJob* jobs;    // sorted by item0
@@ -726,15 +726,15 @@ struct ItemTile {
   int k0;
 };
 template <int NY>
-__device__ __forceinline__ ItemTile item_tile(const BPArgs& ja, long long t, int nbh) {
+__device__ __forceinline__ ItemTile item_tile(const BPArgs& ja, long long t) {
   ItemTile it;
-  const long long per = (long long)nbh * nbh;
+  const long long per = (long long)ja.nbx * ja.nbz;
   const int by = (int)(t / per);
   const int rem = (int)(t - (long long)by * per);
-  const int H = min(max(1, ja.band), nbh);
-  const int b = rem / (H * nbh);
-  const int hb = min(H, nbh - b * H);  // orbit rows in this band (the last may be short)
-  const int r2 = rem - b * H * nbh;
+  const int H = min(max(1, ja.band), ja.nbz);
+  const int b = rem / (H * ja.nbx);
+  const int hb = min(H, ja.nbz - b * H);  // orbit rows in this band (the last may be short)
+  const int r2 = rem - b * H * ja.nbx;
   const int bx = r2 / hb, bz = b * H + (r2 - bx * hb);
   it.ix0 = bx * 16;
   it.iz0 = bz * 16;
@@ -776,11 +776,15 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
                    const __grid_constant__ QuadQueue qq) {
   constexpr int TX = 16, TZ = 16, TY = NY * YW, NCW = 8 * YW, E = kQuadEntries;
   constexpr bool Q24 = LAYOUT == kLayoutQuadG24;
-  constexpr bool Q32 = LAYOUT == kLayoutQuad32;
-  constexpr int NPL = Q24 ? 3 : Q32 ? 1 : 2;  // 16-byte planes per element row
-  constexpr int ESZ = 16 * NPL;
+  constexpr bool Q32 = LAYOUT == kLayoutQuad32 || LAYOUT == kLayoutDuo32;
+  constexpr bool P16 = is_p16_layout(LAYOUT);
+  constexpr bool GRAD = is_grad_layout(LAYOUT);
+  constexpr int S = slots_of(LAYOUT);
+  constexpr int NPL = Q24 ? 3 : GRAD ? 2 : 1;  // planes per element row
+  constexpr int CB = S == 4 ? 16 : 8;          // bytes per column of a plane
+  constexpr int ESZ = CB * NPL;
   constexpr int kRowTail = Q32 ? 1 : 0;  // a tap also reads the next element row
-  constexpr int kCol0 = Q32 ? 0 : 1;     // element column of detector column 0 (gradient elements start at -1)
+  constexpr int kCol0 = GRAD ? 1 : 0;    // element column of detector column 0 (gradient elements start at -1)
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int R = MULTI ? qq.ring : a.box_bytes;  // ring bytes
@@ -837,8 +841,8 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
       const BPArgs& ja = job_args<MULTI>(a, qq, jb);
       const BoxMaps& jm = job_maps<MULTI>(maps, qq, jb);
       const long long t_local = MULTI ? item - qq.jobs[jb].item0 + qq.jobs[jb].t0 : item;
-      const ItemTile til = item_tile<TY>(ja, t_local, MULTI ? qq.jobs[jb].nbh : ja.ntx >> 1);
-      const int K = ja.nviews, Q = K >> 2;
+      const ItemTile til = item_tile<TY>(ja, t_local);
+      const int K = ja.nviews, Q = ja.groups;
       for (int kb = 0; kb < K && !*s_abort; kb += kGeoQuads) {
         if (blocks >= 2) named_sync(kBarFree + b, 64);
         const int it = kb + lane;         // quad of the item (ring entry order)
@@ -865,7 +869,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
           const bool direct = !skip && (need_u > jm.w[kNW - 1] || rows > jm.h[kNH - 1] || bytes > R);
           st.need = (skip || direct) ? 0 : bytes;
           st.tx_bytes = tx_bytes;
-          st.x = 2 * (u0 + kCol0);
+          st.x = CB / 8 * (u0 + kCol0);
           st.y = v0 + ja.pair_rows;
           st.grp = k % Q;
           st.mi = wi * kNH + hi;
@@ -874,16 +878,18 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
           qc.Nx = vc.Nx; qc.Nz = vc.Nz; qc.N0 = vc.N0;
           qc.Vx = vc.Vx; qc.Vz = vc.Vz; qc.V0 = vc.V0;
 #pragma unroll
-          for (int r = 0; r < 4; ++r) qc.ws[r] = ja.inv_scale ? ja.inv_scale[k % Q + r * Q] : 1.0f;
+          for (int r = 0; r < S; ++r)
+            qc.ws[r] = ja.inv_scale ? ja.inv_scale[k % Q + (r < ja.mirror ? r : r - ja.mirror) * Q] : 1.0f;
           qc.flags = (skip ? kQSkip : 0) | (direct ? kQDirect : 0) | (it == 0 ? kQFirst : 0) |
-                     (it == K - 1 ? kQLast : 0) | ((k + 1) % Q == 0 ? kQTurn : 0) | (vc.skip & 2 ? kQShort : 0);
+                     (it == K - 1 ? kQLast : 0) | ((k + 1) % Q == 0 ? kQTurn : 0) | (k == K - 1 ? kQWrap : 0) |
+                     (vc.skip & 2 ? kQShort : 0);
           // window: width (elements) and rows
           const int BU = direct ? need_u : jm.w[wi], BV = direct ? rows : jm.h[hi];
           qc.grp = k % Q;
           qc.u0 = u0 + kCol0;
           qc.e0 = v0 + ja.pair_rows;
           qc.rb = (uint32_t)(BU * ESZ);
-          qc.plane = (uint32_t)(BU * 16);
+          qc.plane = (uint32_t)(BU * CB);
           qc.bu2 = BU - 2;
           qc.vmax = (float)(BV - kRowTail) - (float)(kSlack / 2);
           qc.dvn = ja.dvn;
@@ -1004,26 +1010,29 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
   // plain FP32 sums: four slots x NY voxels in registers (a compensated sum
   // was measured to change no digit of the MIXED form's error, which the
   // FP16 views set, and cost 5% at C4)
-  float acc[4][NY];
-  // the next quarter turn: its slot s belongs to the rotation of slot s - 1
+  float acc[S][NY];
+  // the next phase: its slot s belongs to the rotation of slot s - 1
   auto turn = [&]() {
 #pragma unroll
     for (int j = 0; j < NY; ++j) {
-      const float t = acc[3][j];
-      acc[3][j] = acc[2][j], acc[2][j] = acc[1][j], acc[1][j] = acc[0][j], acc[0][j] = t;
+      const float t = acc[S - 1][j];
+#pragma unroll
+      for (int s = S - 1; s > 0; --s) acc[s][j] = acc[s - 1][j];
+      acc[0][j] = t;
     }
   };
   // a new work item: zero every sum of this thread
   auto reset = [&]() {
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < S; ++r)
 #pragma unroll
       for (int j = 0; j < NY; ++j) acc[r][j] = 0.f;
   };
   reset();
   int e = 0;
   uint32_t ph = 0;
-  bool bad = false, stop = false, last = false, leave = false, turned = false;
+  bool bad = false, stop = false, last = false, leave = false;
+  int turned = 0;  // slots the sums move by after this view
   long long item = -1;  // work item being accumulated
   int jb = 0;         // its job
   // one quad: wait for its window, apply it to the 4 x NY voxels, release it
@@ -1061,7 +1070,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
       const float vlast = fmaf((float)(NY - 1), dvv, vl);
       const uint32_t RB = g.rb;
       if (iu >= 0 && iu <= g.bu2 && vl >= 0.f && vlast < g.vmax) {
-        const uint32_t c0 = g.cbase + (uint32_t)(iu * 16);
+        const uint32_t c0 = g.cbase + (uint32_t)(iu * CB);
         // v of voxels j and j + 1, stepped by 2 dvv from (vl, vl + dvv): no
         // per-pair constants (a few ulps of v from the repeated additions);
         // floor and fraction of the pair with packed FP32 ops
@@ -1074,17 +1083,12 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
           // weights of the two columns, the distance weight folded in
           const float wbs = __fmul_rn(W, fu), was = __fsub_rn(W, wbs);
           const float2 wa = make_float2(was, was), wb = make_float2(wbs, wbs);
-          // an element row at this thread's detector position: the four slots, interpolated in u
-          auto blend = [&](const uint4& A, const uint4& B, float2 (&q)[2]) {
-            q[0] = ffma2(wb, make_float2(__uint_as_float(B.x), __uint_as_float(B.y)),
-                         fmul2(wa, make_float2(__uint_as_float(A.x), __uint_as_float(A.y))));
-            q[1] = ffma2(wb, make_float2(__uint_as_float(B.z), __uint_as_float(B.w)),
-                         fmul2(wa, make_float2(__uint_as_float(A.z), __uint_as_float(A.w))));
-          };
-          auto add = [&](const float2 (&lo)[2], const float2 (&hi)[2], float fv, int j) {
+          // an element row at this thread's detector position: the slots' pairs, interpolated in u
+          auto blend = [&](const float2& A, const float2& B) { return ffma2(wb, B, fmul2(wa, A)); };
+          auto add = [&](const float2 (&lo)[S / 2], const float2 (&hi)[S / 2], float fv, int j) {
             const float fl = 1.f - fv;
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
+            for (int p = 0; p < S / 2; ++p) {
               const float2 d = ffma2(make_float2(fv, fv), hi[p],
                                      ffma2(make_float2(fl, fl), lo[p], make_float2(acc[2 * p][j], acc[2 * p + 1][j])));
               acc[2 * p][j] = d.x;
@@ -1092,10 +1096,20 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
             }
           };
           if (!(flags & kQDirect)) {
-            auto load = [&](uint32_t at, float2 (&q)[2]) { blend(lds_u4(at), lds_u4(at + 16), q); };
+            auto load = [&](uint32_t at, float2 (&q)[S / 2]) {
+              if constexpr (S == 4) {
+                const uint4 A = lds_u4(at), B = lds_u4(at + CB);
+                q[0] = blend(make_float2(__uint_as_float(A.x), __uint_as_float(A.y)),
+                             make_float2(__uint_as_float(B.x), __uint_as_float(B.y)));
+                q[S / 2 - 1] = blend(make_float2(__uint_as_float(A.z), __uint_as_float(A.w)),
+                                     make_float2(__uint_as_float(B.z), __uint_as_float(B.w)));
+              } else {
+                q[0] = blend(lds_f32x2(at), lds_f32x2(at + CB));
+              }
+            };
             auto march = [&](auto shortc) {
               constexpr bool SHORT = decltype(shortc)::value;
-              float2 lo[2], hi[2];
+              float2 lo[S / 2], hi[S / 2];
               uint32_t before = 0;  // bit pattern of the previous voxel's row
 #pragma unroll
               for (int j = 0; j < NY; j += 2) {
@@ -1111,7 +1125,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
                   } else {
                     const bool same = bits == before;
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) {
+                    for (int i = 0; i < S / 2; ++i) {
                       lo[i].x = same ? lo[i].x : hi[i].x;
                       lo[i].y = same ? lo[i].y : hi[i].y;
                     }
@@ -1130,22 +1144,80 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
             // outside the stored extent, as the TMA fill would give)
             const BPArgs& ja = job_args<MULTI>(a, qq, jb);
             const int col = g.u0 + iu;
-            auto load = [&](int row, float2 (&q)[2]) {
-              const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-              const uint4* p = ja.qg + ((size_t)g.grp * ja.qg_rows + row) * ja.qg_pitch + col;
+            auto load = [&](int row, float2 (&q)[S / 2]) {
+              const float2* p = reinterpret_cast<const float2*>(ja.qg) +
+                                (((size_t)g.grp * ja.qg_rows + row) * ja.qg_pitch + col) * (S / 2);
               const bool in = row >= 0 && row < ja.qg_rows;
-              blend(in && col >= 0 && col < ja.qg_pitch ? __ldg(p) : zero,
-                    in && col + 1 >= 0 && col + 1 < ja.qg_pitch ? __ldg(p + 1) : zero, q);
+              const bool inA = in && col >= 0 && col < ja.qg_pitch, inB = in && col + 1 >= 0 && col + 1 < ja.qg_pitch;
+#pragma unroll
+              for (int i = 0; i < S / 2; ++i)
+                q[i] = blend(inA ? __ldg(p + i) : make_float2(0.f, 0.f), inB ? __ldg(p + S / 2 + i) : make_float2(0.f, 0.f));
             };
 #pragma unroll
             for (int j = 0; j < NY; ++j) {
               const float v = fmaf((float)j, dvv, vl);
               const float t = __fadd_rz(v, kMagic);
               const int row = g.e0 + (int)(__float_as_uint(t) - kMagicBits);
-              float2 lo[2], hi[2];
+              float2 lo[S / 2], hi[S / 2];
               load(row, lo);
               load(row + 1, hi);
               add(lo, hi, v - (t - kMagic), j);
+            }
+          }
+        } else if constexpr (P16) {
+          // slots' (row v, row v + 1 minus row v): the u-lerp of both in FP32
+          float Wr[S];
+#pragma unroll
+          for (int r = 0; r < S; ++r) Wr[r] = __fmul_rn(W, g.ws[r]);
+          auto tap = [&](const uint32_t (&X)[S], const uint32_t (&Y)[S], float fv, int j) {
+#pragma unroll
+            for (int r = 0; r < S; ++r) {
+              const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&X[r]));
+              const float2 y = __half22float2(*reinterpret_cast<const __half2*>(&Y[r]));
+              const float2 ag = ffma2(make_float2(fu, fu), fsub2(y, x), x);
+              acc[r][j] = fmaf(Wr[r], fmaf(fv, ag.y, ag.x), acc[r][j]);
+            }
+          };
+          if (!(flags & kQDirect)) {
+            auto load = [&](uint32_t at, uint32_t (&X)[S]) {
+              if constexpr (S == 4) {
+                const uint4 q = lds_u4(at);
+                X[0] = q.x, X[1] = q.y, X[S - 2] = q.z, X[S - 1] = q.w;
+              } else {
+                const float2 q = lds_f32x2(at);
+                X[0] = __float_as_uint(q.x), X[1] = __float_as_uint(q.y);
+              }
+            };
+#pragma unroll
+            for (int j = 0; j < NY; j += 2) {
+              if (j) v2 = fadd2(v2, step2);
+              const float2 t2 = fadd2_rz(v2, magic2);
+              const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
+#pragma unroll
+              for (int p = 0; p < 2; ++p) {
+                const uint32_t at = __float_as_uint(p ? t2.y : t2.x) * RB + c0;
+                uint32_t X[S], Y[S];
+                load(at, X);
+                load(at + CB, Y);
+                tap(X, Y, p ? fv2.y : fv2.x, j + p);
+              }
+            }
+          } else {
+            const BPArgs& ja = job_args<MULTI>(a, qq, jb);
+            const int col = g.u0 + iu;
+#pragma unroll
+            for (int j = 0; j < NY; ++j) {
+              const float v = fmaf((float)j, dvv, vl);
+              const float t = __fadd_rz(v, kMagic);
+              const int row = g.e0 + (int)(__float_as_uint(t) - kMagicBits);
+              const uint32_t* p = reinterpret_cast<const uint32_t*>(ja.qg) +
+                                  (((size_t)g.grp * ja.qg_rows + row) * ja.qg_pitch + col) * S;
+              const bool in = row >= 0 && row < ja.qg_rows;
+              const bool inA = in && col >= 0 && col < ja.qg_pitch, inB = in && col + 1 >= 0 && col + 1 < ja.qg_pitch;
+              uint32_t X[S], Y[S];
+#pragma unroll
+              for (int r = 0; r < S; ++r) X[r] = inA ? __ldg(p + r) : 0u, Y[r] = inB ? __ldg(p + S + r) : 0u;
+              tap(X, Y, v - (t - kMagic), j);
             }
           }
         } else {
@@ -1247,27 +1319,32 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
       e = 0;
       ph ^= 1;
     }
-    turned = (flags & kQTurn) != 0;
+    turned = flags & kQTurn ? (flags & kQWrap ? (MULTI ? 1 : a.wrap) : 1) : 0;
   };
-  // the item's sums into its voxels: four rotated columns,
-  // (x, z) -> (n-1-z, x) -> (n-1-x, n-1-z) -> (z, n-1-x)
+  // the item's sums into its voxels: the rotated columns, (x, z) ->
+  // (n-1-z, x) -> (n-1-x, n-1-z) -> (z, n-1-x), or (x, z) -> (n-1-x, n-1-z)
   auto store = [&]() {
     const BPArgs& ja = job_args<MULTI>(a, qq, jb);
-    const ItemTile til = item_tile<TY>(ja, MULTI ? item - qq.jobs[jb].item0 + qq.jobs[jb].t0 : item,
-                                       MULTI ? qq.jobs[jb].nbh : a.ntx >> 1);
-    // four turns bring the sums back to the first view's slots, where rotation
-    // r sits in slot r + its quarter: move it to slot r
-    for (int i = (4 - til.k0 / (ja.nviews >> 2)) & 3; i > 0; --i) turn();
-    const int n = ja.nx;
+    const ItemTile til = item_tile<TY>(ja, MULTI ? item - qq.jobs[jb].item0 + qq.jobs[jb].t0 : item);
+    // a whole walk brings the sums back to the first view's slots, where
+    // rotation r sits in slot r + its phase: move it to slot r
+    for (int i = (S - til.k0 / ja.groups % S) % S; i > 0; --i) turn();
+    // representative columns: four slots, x < n - h and z < h (h = n / 2) and
+    // the centre of an odd size; two slots, z < h and an odd size's middle
+    // row; columns that are their own image are rotation 0's alone
+    const int n = ja.nx, h = n >> 1;
     const int ix = til.ix0 + tx, iz = til.iz0 + tz;
-    const int cx[4] = {ix, n - 1 - iz, n - 1 - ix, iz};
-    const int cz[4] = {iz, ix, n - 1 - iz, n - 1 - ix};
+    const bool mid = (n & 1) && iz == h && (S == 2 || ix == h);
+    const bool own = (S == 4 ? ix < n - h : ix < n) && (iz < h || mid);
+    const int cx[4] = {ix, S == 4 ? n - 1 - iz : n - 1 - ix, n - 1 - ix, iz};
+    const int cz[4] = {iz, S == 4 ? ix : n - 1 - iz, n - 1 - iz, n - 1 - ix};
     float* const vol = ja.vol;
     const int ystride = ja.vol_ystride, ny = ja.ny, ylim = ja.clip_ylimit;
     const float scale = ja.scale;
     float lo = __int_as_float(0x7f800000), hi = -lo;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < S; ++r) {
+      if (!own || (mid && r > 0)) continue;
       float* out = vol + ((size_t)cz[r] * ystride) * n + cx[r];
 #pragma unroll
       for (int j = 0; j < NY; ++j) {
@@ -1287,15 +1364,15 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
     // one work item, K quads (as many as views): a loop of known length
     item = (long long)blockIdx.y * gridDim.x + blockIdx.x;
     const int K = a.nviews;
-    // the four quarter turns, the first one entered at its view k0 mod Q and
-    // finished at the end (the turns stay out of the inner loop)
-    const int Q = K >> 2, first = Q - item_tile<TY>(a, item, a.ntx >> 1).k0 % Q;
+    // the phases, the first one entered at its view k0 mod Q and finished at
+    // the end (the turns stay out of the inner loop)
+    const int Q = a.groups, first = Q - item_tile<TY>(a, item).k0 % Q;
     int left = K;
     for (int n = first; left > 0 && !stop; n = min(Q, left)) {
       left -= n;
 #pragma unroll 2
       for (int q = 0; q < n; ++q) { step(); if (stop) break; }
-      if (turned) turn();
+      for (int i = 0; i < turned; ++i) turn();
     }
     if (bad) atomicCAS(a.err, 0, kDevFootprint);
     if (stop || *s_abort) return;
@@ -1306,7 +1383,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
     do step();
     while (!(stop || leave || turned || last));
     if (stop || leave) break;
-    if (turned) turn();
+    for (int i = 0; i < turned; ++i) turn();
     if (last) {
       if (bad) atomicCAS(job_args<MULTI>(a, qq, jb).err, 0, kDevFootprint);
       bad = false;
@@ -1435,51 +1512,67 @@ cudaError_t launch_quad_cfg(const BoxMaps& maps, const BPArgs& a, size_t smem, c
   // all of L1 as shared memory, so that two CTAs of up to 113 KB share an SM
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  dim3 grid((a.ntx / 2) * (a.ntz / 2), (a.ny + NY * YW - 1) / (NY * YW));
+  dim3 grid(a.nbx * a.nbz, (a.ny + NY * YW - 1) / (NY * YW));
   kern<<<grid, quad_threads(LAYOUT, NY, YW), smem, stream>>>(maps, a, QuadQueue{});
   return cudaGetLastError();
 }
 
 // The kernel shape of a staged layout and tile height (quad_tile_ny's values).
-#define FBP_QUAD_SHAPES(LAUNCH)                                                              \
-  switch (layout) {                                                                          \
-    case kLayoutQuadG16:                                                                     \
-      return ny_tile == 8    ? LAUNCH(kLayoutQuadG16, 8, 1, 2)                               \
-             : ny_tile == 16 ? LAUNCH(kLayoutQuadG16, 8, 2, 1)                               \
-                             : LAUNCH(kLayoutQuadG16, 12, 2, 1);                             \
-    case kLayoutQuadG24:                                                                     \
-      return ny_tile == 8    ? LAUNCH(kLayoutQuadG24, 8, 1, 2)                               \
-             : ny_tile == 12 ? LAUNCH(kLayoutQuadG24, 12, 1, 2)                              \
-                             : LAUNCH(kLayoutQuadG24, 16, 1, 1);                             \
-    default:                                                                                 \
-      return ny_tile == 8    ? LAUNCH(kLayoutQuad32, 8, 1, 2)                                \
-             : ny_tile == 12 ? LAUNCH(kLayoutQuad32, 12, 1, 2)                               \
-                             : LAUNCH(kLayoutQuad32, 16, 1, 1);                              \
-  }
+#define FBP_SYMMETRIC_SHAPES(LAUNCH)                                                         \
+  case kLayoutQuadG16:                                                                       \
+    return ny_tile == 8    ? LAUNCH(kLayoutQuadG16, 8, 1, 2)                                 \
+           : ny_tile == 16 ? LAUNCH(kLayoutQuadG16, 8, 2, 1)                                 \
+                           : LAUNCH(kLayoutQuadG16, 12, 2, 1);                               \
+  case kLayoutQuadG24:                                                                       \
+    return ny_tile == 8    ? LAUNCH(kLayoutQuadG24, 8, 1, 2)                                 \
+           : ny_tile == 12 ? LAUNCH(kLayoutQuadG24, 12, 1, 2)                                \
+                           : LAUNCH(kLayoutQuadG24, 16, 1, 1);                               \
+  default:                                                                                   \
+    return ny_tile == 8    ? LAUNCH(kLayoutQuad32, 8, 1, 2)                                  \
+           : ny_tile == 12 ? LAUNCH(kLayoutQuad32, 12, 1, 2)                                 \
+                           : LAUNCH(kLayoutQuad32, 16, 1, 1);
 
 cudaError_t launch_quad(int layout, int ny_tile, const BoxMaps& maps, const BPArgs& a, size_t smem,
                         cudaStream_t stream) {
 #define FBP_LAUNCH(L, NY, YW, OCC) launch_quad_cfg<L, NY, YW, OCC>(maps, a, smem, stream)
-  FBP_QUAD_SHAPES(FBP_LAUNCH)
+  switch (layout) {
+    case kLayoutDuo32:
+      return FBP_LAUNCH(kLayoutDuo32, 16, 1, 2);
+    case kLayoutQuadP16:
+      return FBP_LAUNCH(kLayoutQuadP16, 8, 1, 2);
+    case kLayoutDuoP16:
+      return FBP_LAUNCH(kLayoutDuoP16, 16, 1, 2);
+      FBP_SYMMETRIC_SHAPES(FBP_LAUNCH)
+  }
 #undef FBP_LAUNCH
 }
 
-int quad_occ(int ny_tile) { return ny_tile == 8 || ny_tile == 12 ? 2 : 1; }
+int quad_occ(int layout, int ny_tile) {
+  return ny_tile == 8 || ny_tile == 12 || layout == kLayoutDuo32 || layout == kLayoutDuoP16 ? 2 : 1;
+}
 
 // Tile height of a symmetric backprojection: the caller's (8 or 16), or the one
-// with the least work on the fullest SM, ceil(tiles / SMs) x height, times what
-// a voxel costs in that shape on a large volume (512^3, 720 views; 480^3 at the
-// 1440^3 geometry). MIXED: 24 0.94 of 16 (36.6 against 37.3 ms; 14.7 against
-// 16.2); FP32 and 24-bit: 12 0.95 of 8 (37.2 against 38.1 and 46.7 against 49.3
-// ms; 17.6 against 18.9 and 19.7 against 20.2).
+// with the least time by a fit to volumes of 96^3 to 384^3 (ms for 360 views;
+// shapes with two CTAs a SM against the waves of tiles W = tiles / (2 SMs),
+// those with one against the tiles on the fullest SM). At 96^3, 128^3, 192^3,
+// 384^3: MIXED 8 high 0.29, 0.45, 1.18, 8.1; 16 high 0.42, 0.44, 1.16, 8.1; 24
+// high 0.56, 0.59, 1.11, 7.6. FP32 and 24-bit take 12 from 36 waves on
+// (about 440^3): 8 and 12 high 0.31 and 0.47, 0.50 and 0.77, 1.40 and 1.48, 9.8
+// and 10.1 at those sizes, then 18.9 and 17.6 at 480 x 490 x 480 (480 views),
+// 38.1 and 37.2 at 512^3 (720 views; 24-bit 49.3 and 46.4).
 int quad_tile_height(int asked, int layout, int orbits, int ny, int num_sms) {
   if (asked) return asked;
-  auto cost = [&](int h, double rel) {
-    const long long tiles = (long long)orbits * ((ny + h - 1) / h);
-    return (double)((tiles + num_sms - 1) / num_sms) * h * rel;
-  };
-  if (layout == kLayoutQuadG16) return cost(24, 0.94) < cost(16, 1.0) ? 24 : 16;
-  return cost(12, 0.95) < cost(8, 1.0) ? 12 : 8;
+  if (layout == kLayoutDuo32 || layout == kLayoutDuoP16) return 16;
+  if (layout == kLayoutQuadP16) return 8;
+  auto tiles = [&](int h) { return (long long)orbits * ((ny + h - 1) / h); };
+  auto waves = [&](int h) { return (double)tiles(h) / (2.0 * num_sms); };
+  auto fullest = [&](int h) { return (double)((tiles(h) + num_sms - 1) / num_sms); };
+  if (layout == kLayoutQuadG16) {
+    const double c8 = 0.345 * (std::max(0.5, waves(8)) + 0.45);
+    const double c16 = 0.36 * (fullest(16) + 0.15), c24 = 0.47 * (fullest(24) + 0.2);
+    return c8 < c16 && c8 < c24 ? 8 : c16 < c24 ? 16 : 24;
+  }
+  return waves(8) >= 36.0 ? 12 : 8;
 }
 
 template <int TX, int TZ, int NY>
@@ -1639,6 +1732,44 @@ static void choose_boxes(const std::vector<unsigned>& hist, int mbu, int mbv, in
   }
 }
 
+// The orbits of a view set; four slots only where the volume is square.
+static Orbits find_orbits(bool cone, double turns, int K, bool square) {
+  const long long whole = llround(turns), halves = llround(2.0 * turns);
+  const bool full_turn = fabs(turns - (double)whole) < 1e-9;
+  const bool half_turn = !full_turn && fabs(2.0 * turns - (double)halves) < 1e-9;  // an odd number of halves
+  if (square && full_turn && whole % 4 == 1 && K % 4 == 0) return {4, K / 4, 4, 4};
+  if (square && !cone && half_turn && halves % 4 == 1 && K % 2 == 0) return {4, K / 2, 2, 2};
+  if (full_turn && (whole % 2 == 1 || whole % 2 == -1) && K % 2 == 0) return {2, K / 2, 2, 2};
+  if (!cone) return {2, K, 1, 1};
+  return {1, K, 1, 1};
+}
+
+// Whether a volume off the symmetric kernel runs on rotational orbits, and on
+// which: the least of (tiles on the fullest SM + 0.4) x the cost of a tile,
+// with the costs measured in units of the plain kernel's 16 x 16 x 16 tile
+// (300 x 251 x 300, 450 to 452 views; 256^3 parallel; the 0.4 is what a SM's
+// last tiles lose by running alone, 100 x 80 x 100). FP32: four slots 1.13 (8
+// high) or 1.76 (12 high), two slots 1.42; FP16 pairs: 1.36 and 1.44.
+static bool choose_orbits(const BPGeom& g, double turns, bool p16, int num_sms, Orbits* orb) {
+  const bool cone = g.kind == FBP_GEOMETRY_CONE;
+  const int t16 = (g.nx + 15) / 16, half = ((g.nx + 1) / 2 + 15) / 16;
+  auto cost = [&](long long columns, int height, double rel) {
+    const long long tiles = columns * ((g.ny + height - 1) / height);
+    return rel * ((double)((tiles + num_sms - 1) / num_sms) + 0.4);
+  };
+  double best = cost((long long)t16 * t16, 16, 1.0);
+  bool any = false;
+  const Orbits four = find_orbits(cone, turns, g.nviews, true), two = find_orbits(cone, turns, g.nviews, false);
+  if (four.slots == 4) {
+    const double c = p16 ? cost((long long)half * half, 8, 1.36)
+                         : std::min(cost((long long)half * half, 8, 1.13), cost((long long)half * half, 12, 1.76));
+    if (c < best) best = c, *orb = four, any = true;
+  }
+  if (two.slots == 2 && cost((long long)t16 * half, 16, p16 ? 1.44 : 1.42) < best) *orb = two, any = true;
+  if (!any) *orb = Orbits{1, g.nviews, 1, 1};
+  return any;
+}
+
 // A planned backprojection: everything a launch needs (arguments, tensor
 // maps, shared memory) after the footprint pass and the packing.
 struct BPLaunchPlan {
@@ -1647,13 +1778,14 @@ struct BPLaunchPlan {
   size_t smem = 0;
   int layout = 0, ny_tile = 0, occ = 2;
   bool use_quad = false, is2d = false;
+  bool orbit = false;  // the quad kernel on an orbit of the generic backprojector's geometries
 };
 
 BPLaunchPlan* new_bp_plan() { return new BPLaunchPlan(); }
 void free_bp_plan(BPLaunchPlan* p) { delete p; }
 
 int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, int clip_ylimit, bool mixed,
-                     BPLaunchPlan* plan_out) {
+                     BPLaunchPlan* plan_out, bool plain) {
   const double pi = 3.14159265358979323846;
   // MIXED24: 24-bit views for the symmetric kernel (FP32 rows otherwise)
   const bool c24 = mixed && ctx->precision == FBP_PRECISION_MIXED24;
@@ -1664,18 +1796,28 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   const long long iturns = llround(turns);
   const bool symmetric = !is2d && g.nx == g.nz && g.nx % 32 == 0 && g.nviews % 4 == 0 &&
                          fabs(turns - (double)iturns) < 1e-9 && iturns % 4 == 1;
-  const bool quad = symmetric && (ctx->bp_variant == FBP_BACKPROJECTOR_AUTO ||
-                                  ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC);
+  const bool quad = symmetric && !plain &&
+                    (ctx->bp_variant == FBP_BACKPROJECTOR_AUTO || ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC);
   if (ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC && !symmetric)
     return set_error(ctx, FBP_ERR_UNSUPPORTED,
                      "the four-fold symmetric backprojector needs nx == nz (a multiple of 32), views % 4 == 0 and "
                      "views over one full turn");
-  // what the selected kernel reads: interleaved quads (symmetric), FP16 pairs
-  // (MIXED) or the FP32 rows themselves
-  const bool packed = quad || (mixed && !c24);
-  const int layout = quad ? (!mixed ? kLayoutQuad32 : c24 ? kLayoutQuadG24 : kLayoutQuadG16)
-                     : packed ? kLayoutPair16
-                              : kLayoutRaw32;
+  // The generic backprojector's geometries that still have rotational orbits
+  // (any size; half turns, parallel beam) run on the same kernel, four or two
+  // voxels to a tap position, where that is faster; an explicit view ring is
+  // the plain kernel's.
+  const bool p16 = mixed && !c24;
+  Orbits orb = find_orbits(g.kind == FBP_GEOMETRY_CONE, turns, g.nviews, g.nx == g.nz);
+  const bool orbit = !quad && !is2d && !plain && g.nx == g.nz && ctx->bp_stages == 0 &&
+                     (ctx->bp_variant == FBP_BACKPROJECTOR_AUTO || ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC) &&
+                     choose_orbits(g, turns, p16, ctx->num_sms, &orb);
+  // what the selected kernel reads: interleaved views (symmetric, orbits), FP16
+  // pairs (MIXED) or the FP32 rows themselves
+  const bool packed = quad || orbit || p16;
+  const int layout = quad    ? (!mixed ? kLayoutQuad32 : c24 ? kLayoutQuadG24 : kLayoutQuadG16)
+                     : orbit ? (orb.slots == 4 ? (p16 ? kLayoutQuadP16 : kLayoutQuad32) : p16 ? kLayoutDuoP16 : kLayoutDuo32)
+                     : p16   ? kLayoutPair16
+                             : kLayoutRaw32;
   const int esize = Stack::elem_bytes(layout);
   BPArgs a{};
   a.vol = vol;
@@ -1704,10 +1846,15 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     a.dvn = (float)(g.vox / g.dv);
     a.scale = (float)(pi / g.nviews / g.du);
   }
-  a.inv_scale = (layout == kLayoutPair16 || layout == kLayoutQuadG16) ? st.inv_scale : nullptr;
+  a.groups = orb.groups;
+  a.mirror = orb.mirror;
+  a.wrap = (orb.slots - orb.phases + 1) % orb.slots;
+  const int half = ((g.nx + 1) / 2 + 15) / 16;
+  a.nbx = orb.slots == 4 ? half : (g.nx + 15) / 16;
+  a.nbz = orb.slots == 1 ? (g.nx + 15) / 16 : half;
   // TMA: x * element size must be a multiple of 16 bytes (the interleaved
   // layouts' x counts 8-byte words, two per 16-byte plane element: always even)
-  a.align = is_quad_layout(layout) ? 1 : 4;
+  a.align = !is_quad_layout(layout) ? 4 : esize == 8 ? 2 : 1;
   a.sino_layout = st.sinogram ? 1 : 0;
   a.pair_rows = is_pair_layout(layout) ? 1 : 0;
   a.clip_ylimit = clip_ylimit;
@@ -1718,10 +1865,11 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   a.trig = ctx->d_trig;
 
   // tile configuration: 16 x 16 columns, NY voxels along y (1 for 2D)
-  const int TX = 16, TZ = 16, orbits = (g.nx / 32) * (g.nx / 32);
-  const int NY = is2d   ? 1
-                 : quad ? quad_tile_height(ctx->quad_tile_ny, layout, orbits, g.ny, ctx->num_sms)
-                        : (ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC_Y8 ? 8 : 16);
+  const int TX = 16, TZ = 16;
+  const int NY = is2d    ? 1
+                 : quad  ? quad_tile_height(ctx->quad_tile_ny, layout, a.nbx * a.nbz, g.ny, ctx->num_sms)
+                 : orbit ? quad_tile_height(0, layout, a.nbx * a.nbz, g.ny, ctx->num_sms)
+                         : (ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC_Y8 ? 8 : 16);
   a.ntx = (g.nx + TX - 1) / TX;
   a.ntz = (g.nz + TZ - 1) / TZ;
   const int nty = (g.ny + NY - 1) / NY;
@@ -1742,7 +1890,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   }
   // a plan made without the histogram (not a symmetric candidate then) is
   // redone in place when the symmetric kernel may now run
-  const bool redo = found && quad && found->hist.empty();
+  const bool redo = found && (quad || orbit) && found->hist.empty();
   const bool hit = found != nullptr && !redo;
   fbp_context::BPPlan& plan = found ? *found : ctx->plans[ctx->plan_next];
   if (!hit) {
@@ -1760,7 +1908,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     }
     // the window histogram only for the symmetric kernel (its interleaved
     // layouts fit their boxes to it); the other plans take quarter steps
-    unsigned* d_hist = quad ? reinterpret_cast<unsigned*>(ctx->d_span + 4) : nullptr;
+    unsigned* d_hist = quad || orbit ? reinterpret_cast<unsigned*>(ctx->d_span + 4) : nullptr;
     cudaMemsetAsync(ctx->d_span, 0, (d_hist ? kSpanWords : 4) * sizeof(int), ctx->stream);
     const long long ntiles = (long long)a.ntx * a.ntz * nty;
     // few blocks: each adds its whole shared histogram to the global one
@@ -1800,21 +1948,30 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   // Limits of the FP32 form: windows of filtered rows up to 128 x 257 samples,
   // of other rows up to 256 x 256 (what a staged box of them holds), the
   // symmetric kernel's four together at most the ring
-  const bool fp32 = layout == kLayoutRaw32 || layout == kLayoutQuad32;
+  const bool fp32 = layout == kLayoutRaw32 || layout == kLayoutQuad32 || layout == kLayoutDuo32;
   const int fu = st.filtered ? (plan.box_u + 1) / 2 * 2 : (plan.box_u + 3) / 4 * 4;
   const int fv = st.filtered ? std::max(1, plan.box_v - 1) : plan.box_v;
-  if ((fp32 && ((st.filtered ? 2 * fu : fu) > 256 || fv > 256)) || (!is_quad_layout(layout) && (bu > 256 || bv > 256)))
+  if ((fp32 && ((st.filtered ? 2 * fu : fu) > 256 || fv > 256)) ||
+      (is_p16_layout(layout) && ((plan.box_u + 3) / 4 * 4 > 256 || bv > 256)))
     return set_error(ctx, FBP_ERR_UNSUPPORTED,
                      "detector footprint of a voxel tile exceeds the 256-element TMA box; geometry magnification "
                      "too large for the staged backprojector");
   a.box_u = bu;
   a.box_v = bv;
   // two CTAs per SM: each gets half of the 228 KB shared memory
-  const int occ = quad ? quad_occ(NY) : 2;
+  const int occ = quad || orbit ? quad_occ(layout, NY) : 2;
   const size_t smem_cap = occ == 1 ? (size_t)kMaxDynamicSmem : 113 * 1024;
   const size_t max_box = (size_t)(bu * bv * esize + 127) / 128 * 128;
   size_t smem = 0;
-  bool use_quad = quad;
+  bool use_quad = quad || orbit;
+  if (orbit) {
+    // what the plain kernel refuses stays refused: two windows of its ring
+    // (16-voxel tiles; rows, or pairs of filtered FP32 rows) in half an SM
+    const int rows16 = ((p16 ? bv : fv) - 2) * 16 / NY + 2;
+    const size_t box = ((size_t)(p16 ? (plan.box_u + 3) / 4 * 4 : fu) * rows16 * (fp32 && st.filtered ? 8 : 4) + 127) / 128 * 128;
+    if ((113 * 1024 - 64) / (box + sizeof(ViewCoef) + 2 * sizeof(uint64_t)) < 2)
+      return set_error(ctx, FBP_ERR_UNSUPPORTED, "staged detector window does not fit in shared memory");
+  }
   if (use_quad) {
     // byte ring for the windows + entry records
     const size_t fixed = kQuadEntries * (sizeof(QuadCoef) + 2 * sizeof(uint64_t) + sizeof(long long)) +
@@ -1825,7 +1982,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     // (pairs of rows when filtered) would not fit an SM (half, tile height 8)
     const size_t entry = fp32 ? 4 * (((size_t)fu * fv * (st.filtered ? 8 : 4) + 127) / 128 * 128) : 0;
     const size_t limit = ((ctx->quad_tile_ny == 8 ? 113 * 1024 : (size_t)kMaxDynamicSmem) - 1024) / 128 * 128;
-    if (entry > limit) {
+    if (quad && entry > limit) {
       use_quad = false;  // the largest quad does not fit: generic path
       if (ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC)
         return set_error(ctx, FBP_ERR_UNSUPPORTED, "detector windows too large for the symmetric backprojector");
@@ -1854,8 +2011,14 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   }
 
   if (packed && !(st.pack_ready && st.filt_layout == layout))
-    if (int rc = prepare_packed(ctx, st, layout)) return rc;
-  a.inv_scale = (layout == kLayoutPair16 || layout == kLayoutQuadG16) ? st.inv_scale : nullptr;  // set by the pack
+    if (int rc = prepare_packed(ctx, st, layout, orb)) {
+      // no room for the interleaved copy: the plain kernel reads the rows
+      // themselves, or pairs of at most the orbits' bytes
+      if (rc == FBP_ERR_OUT_OF_MEMORY && (orbit || layout == kLayoutQuad32))
+        return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, true);
+      return rc;
+    }
+  a.inv_scale = is_p16_layout(layout) || layout == kLayoutQuadG16 ? st.inv_scale : nullptr;  // set by the pack
   a.resident = occ * ctx->num_sms;  // CTAs resident at once (view-group skew of the symmetric kernel)
   a.band = std::max(1, (int)std::lround(std::sqrt((double)a.resident)));
   if (is_quad_layout(layout)) {
@@ -1874,7 +2037,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   // box row) and at most the ring; larger windows are gathered directly
   // (the widest box of the interleaved layouts is widened, within 128, to a
   // bank-friendly row stride, as choose_boxes picks the narrower ones)
-  const int planes = is_quad_layout(layout) ? (int)(esize / 16) : 0;
+  const int planes = is_quad_layout(layout) ? esize / 16 : 0;  // 0: 8-byte elements
   int mbu = is_quad_layout(layout) ? std::min(bu, 128) : bu;
   if (planes > 0)
     for (int wider = mbu; wider <= 128 && wider < mbu + 8; ++wider)
@@ -1890,6 +2053,15 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     static const std::vector<unsigned> no_hist;
     choose_boxes(is_quad_layout(layout) ? plan.hist : no_hist, mbu, mbv, a.align, a.pair_rows, planes, plan.sel_w,
                  plan.sel_h);
+    // 4-byte rows: a warp's lanes fall on two or three neighbouring rows, ten
+    // to twenty columns wide; widths of 12 to 20 mod 32 keep those off one
+    // another's banks (FP32 rows, 300 x 251 x 300, 451 views: 8.58 -> 7.40 ms)
+    if (!is_quad_layout(layout))
+      for (int i = 0; i < kNW; ++i) {
+        int w = plan.sel_w[i];
+        while (w < mbu && !(w % 32 >= 12 && w % 32 <= 20)) w += 4;
+        plan.sel_w[i] = w;
+      }
     plan.sel_layout = layout;
     plan.sel_u = mbu;
     plan.sel_v = mbv;
@@ -1899,10 +2071,11 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   for (int i = 0; i < kNW; ++i)
     for (int j = 0; j < kNH; ++j) {
       if (is_quad_layout(layout)) {  // [group][element row][plane][element column][2 x 8 bytes]
-        const uint32_t planes = (uint32_t)esize / 16;
-        const uint64_t d4[4] = {2ull * pitch_el, planes, rows_v, (uint64_t)st.n / 4};
-        const uint64_t s4[3] = {16ull * pitch_el, (uint64_t)esize * pitch_el, (uint64_t)esize * pitch_el * rows_v};
-        const uint32_t b4[4] = {2u * maps.w[i], planes, (uint32_t)maps.h[j], 1};
+        const uint32_t words = esize == 8 ? 1 : 2;  // 8-byte words per column of a plane
+        const uint32_t np = (uint32_t)std::max(1, planes);
+        const uint64_t d4[4] = {(uint64_t)words * pitch_el, np, rows_v, (uint64_t)orb.groups};
+        const uint64_t s4[3] = {8ull * words * pitch_el, (uint64_t)esize * pitch_el, (uint64_t)esize * pitch_el * rows_v};
+        const uint32_t b4[4] = {words * maps.w[i], np, (uint32_t)maps.h[j], 1};
         if (int rc = make_tensor_map_4d(ctx, &maps.map[i * kNH + j], CU_TENSOR_MAP_DATA_TYPE_UINT64,
                                         const_cast<void*>(base), d4, s4, b4))
           return rc;
@@ -1948,15 +2121,18 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   p.occ = occ;
   p.use_quad = use_quad;
   p.is2d = is2d;
+  p.orbit = orbit;
   return FBP_OK;
 }
 
 int launch_bp_plan(fbp_context* ctx, const BPLaunchPlan& p) {
   const int NY = p.ny_tile;
-  ctx->last_bp[0] = p.use_quad  ? FBP_BACKPROJECTOR_SYMMETRIC
-                    : NY == 8   ? FBP_BACKPROJECTOR_GENERIC_Y8
-                                : FBP_BACKPROJECTOR_GENERIC;
-  ctx->last_bp[1] = p.layout;
+  ctx->last_bp[0] = p.orbit      ? FBP_BACKPROJECTOR_GENERIC
+                    : p.use_quad ? FBP_BACKPROJECTOR_SYMMETRIC
+                    : NY == 8    ? FBP_BACKPROJECTOR_GENERIC_Y8
+                                 : FBP_BACKPROJECTOR_GENERIC;
+  // orbits: what the views' samples are stored as
+  ctx->last_bp[1] = !p.orbit ? p.layout : is_p16_layout(p.layout) ? kLayoutPair16 : kLayoutRaw32;
   ctx->last_bp[2] = p.a.box_u;
   ctx->last_bp[3] = p.a.box_v;
   ctx->last_bp[4] = NY;
@@ -1976,7 +2152,7 @@ int launch_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol,
 }
 
 long long bp_plan_batch_key(const BPLaunchPlan& p) {
-  if (!p.use_quad) return 0;  // the persistent launch runs the four-fold symmetric kernel
+  if (!p.use_quad || p.orbit) return 0;  // the persistent launch runs the four-fold symmetric kernel
   return 1 + p.layout + 16LL * p.ny_tile + 4096LL * p.occ + 65536LL * p.a.box_bytes;
 }
 
@@ -1998,7 +2174,7 @@ cudaError_t launch_quad_multi_cfg(const QuadQueue& qq, size_t smem, int grid, cu
 cudaError_t launch_quad_multi(int layout, int ny_tile, const QuadQueue& qq, size_t smem, int grid,
                               cudaStream_t stream) {
 #define FBP_LAUNCH(L, NY, YW, OCC) launch_quad_multi_cfg<L, NY, YW, OCC>(qq, smem, grid, stream)
-  FBP_QUAD_SHAPES(FBP_LAUNCH)
+  switch (layout) { FBP_SYMMETRIC_SHAPES(FBP_LAUNCH) }
 #undef FBP_LAUNCH
 }
 
@@ -2009,7 +2185,7 @@ cudaError_t launch_quad_multi(int layout, int ny_tile, const QuadQueue& qq, size
 // of (job, tile orbit, y-slab) work items, largest jobs first in the order
 // given. The job table goes up through the launcher's pinned staging.
 long long bp_plan_tiles(const BPLaunchPlan& p) {
-  return (long long)(p.a.ntx >> 1) * (p.a.ntx >> 1) * ((p.a.ny + p.ny_tile - 1) / p.ny_tile);
+  return (long long)p.a.nbx * p.a.nbz * ((p.a.ny + p.ny_tile - 1) / p.ny_tile);
 }
 
 int launch_bp_batch(fbp_context* L, BPLaunchPlan* const* plans, int n, const long long* tile_begin,
@@ -2051,8 +2227,6 @@ int launch_bp_batch(fbp_context* L, BPLaunchPlan* const* plans, int n, const lon
     hj[i].a = p.a;
     hj[i].a.minmax = nullptr;  // no histogram range for batched jobs
     hj[i].item0 = items;
-    hj[i].nbh = p.a.ntx >> 1;
-    hj[i].nty = (p.a.ny + p.ny_tile - 1) / p.ny_tile;
     const long long all = bp_plan_tiles(p);
     const long long t0 = tile_begin ? std::max(0LL, tile_begin[i]) : 0;
     const long long t1 = tile_end ? std::min(all, tile_end[i]) : all;
@@ -2473,27 +2647,14 @@ int launch_bp2d(fbp_context* ctx, const BPGeom& g, const float* sino, long long 
   const int win = ((int)std::ceil(width) + 8 + 3) / 4 * 4;
   if (win > kWin2DMax) return FBP_ERR_UNSUPPORTED;
   // rotational orbits of the view set
-  const double turns = g.span / (2.0 * pi);
-  const long long whole = llround(turns), halves = llround(2.0 * turns);
-  const bool full_turn = fabs(turns - (double)whole) < 1e-9;
-  const bool half_turn = !full_turn && fabs(2.0 * turns - (double)halves) < 1e-9;  // an odd number of halves
-  const bool square = g.nx == g.nz;
-  const int K = g.nviews;
   // Four slots halve the work of two, but also the tiles: below one CTA a SM
   // (the cluster split included) two are faster (parallel 256^2, 360 views,
   // half a turn: 27.1 us with four slots, 21.0 with two)
+  const int K = g.nviews;
   const int half = ((g.nx + 1) / 2 + kTile2D - 1) / kTile2D;
-  const bool four = square && half * half * kMaxSplit2D >= ctx->num_sms;
-  int slots = 1, groups = K, phases = 1, mirror = 1;  // mirror: rows of an element before their mirror images
-  if (four && full_turn && whole % 4 == 1 && K % 4 == 0) {
-    slots = 4, groups = K / 4, phases = 4, mirror = 4;
-  } else if (four && !cone && half_turn && halves % 4 == 1 && K % 2 == 0) {
-    slots = 4, groups = K / 2, phases = 2, mirror = 2;
-  } else if (full_turn && (whole % 2 == 1 || whole % 2 == -1) && K % 2 == 0) {
-    slots = 2, groups = K / 2, phases = 2, mirror = 2;
-  } else if (!cone) {
-    slots = 2, groups = K, phases = 1, mirror = 1;
-  }
+  const Orbits orb = find_orbits(cone, g.span / (2.0 * pi), K,
+                                 g.nx == g.nz && half * half * kMaxSplit2D >= ctx->num_sms);
+  const int slots = orb.slots, groups = orb.groups, phases = orb.phases, mirror = orb.mirror;
   const int rx = slots == 4 ? (g.nx + 1) / 2 : g.nx, rz = slots == 1 ? g.nz : (g.nz + 1) / 2;
   const int tiles_x = (rx + kTile2D - 1) / kTile2D, tiles_z = (rz + kTile2D - 1) / kTile2D;
   const long long tiles = (long long)tiles_x * tiles_z;

@@ -639,23 +639,40 @@ __global__ void pack_quadg24_kernel(const float* src, long long spitch, int m, i
   }
 }
 
-// f32 rows -> kLayoutQuad32: the four views' samples of one detector pixel as
-// one 16-byte element. Grid: x over columns, y over detector rows, z over view
-// groups. 4 bytes read and 4 written per sample.
-__global__ void __launch_bounds__(256) pack_quad32_kernel(const float* __restrict__ src, long long spitch, int m,
-                                                          int n_views, int n_v, bool sinogram,
-                                                          float4* __restrict__ out) {
-  const int Q = n_views >> 2, g = blockIdx.z, c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m) return;
-  for (int iv = blockIdx.y; iv < n_v; iv += gridDim.y) {
-    float v[4];
+// f32 rows -> the orbits' layouts: the slots' samples of one detector pixel
+// (FP32), or its FP16 row pair (row e - 1, row e minus it as read back: the
+// values of pack_pair16_kernel), as one element. Grid: x over element columns,
+// y over element rows, z over groups. FP32: 4 bytes read and 4 written per
+// sample and slot.
+template <int SLOTS, bool P16>
+__global__ void __launch_bounds__(256) pack_orbit_kernel(const float* __restrict__ src, long long spitch, int m,
+                                                         int n_views, int n_v, bool sinogram, int groups, int mirror,
+                                                         const float* __restrict__ scale, long long pitch,
+                                                         float* __restrict__ out) {
+  const int g = blockIdx.z, c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= pitch) return;
+  for (int e = blockIdx.y; e < n_v + (P16 ? 1 : 0); e += gridDim.y) {
+    float v[SLOTS];
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int view = g + s * Q;
-      const long long r = sinogram ? (long long)iv * n_views + view : (long long)view * n_v + iv;
-      v[s] = __ldg(src + r * spitch + c);
+    for (int s = 0; s < SLOTS; ++s) {
+      // slots past `mirror` views are the first ones' mirror images
+      const int view = g + (s < mirror ? s : s - mirror) * groups, col = s < mirror ? c : m - 1 - c;
+      auto at = [&](int iv) {
+        const long long r = sinogram ? (long long)iv * n_views + view : (long long)view * n_v + iv;
+        return c < m && iv >= 0 && iv < n_v ? __ldg(src + r * spitch + col) : 0.f;
+      };
+      if constexpr (P16) {
+        const float sc = scale[view];
+        const __half hl = __float2half_rn(at(e - 1) * sc);
+        const __half2 x = __halves2half2(hl, __float2half_rn(fmaf(at(e), sc, -__half2float(hl))));
+        v[s] = *reinterpret_cast<const float*>(&x);
+      } else {
+        v[s] = at(e);
+      }
     }
-    out[((long long)g * n_v + iv) * m + c] = make_float4(v[0], v[1], v[2], v[3]);
+    float* o = out + (((long long)g * (n_v + (P16 ? 1 : 0)) + e) * pitch + c) * SLOTS;
+    if constexpr (SLOTS == 4) *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<float2*>(o) = make_float2(v[0], v[1]);
   }
 }
 
@@ -797,7 +814,8 @@ int launch_view_scales(fbp_context* ctx, const RowSet& rs, float limit, float* v
   return launched(ctx, "view scale kernels");
 }
 
-int launch_pack(fbp_context* ctx, const Stack& s, int layout, void* out, long long pitch, const float* view_scale) {
+int launch_pack(fbp_context* ctx, const Stack& s, int layout, const Orbits& o, void* out, long long pitch,
+                const float* view_scale) {
   if (layout == kLayoutPair16) {
     if (s.v + 1 > 65535 || s.n > 65535)
       return set_error(ctx, FBP_ERR_UNSUPPORTED, "the pair layout takes up to 65534 rows and 65535 views");
@@ -824,13 +842,17 @@ int launch_pack(fbp_context* ctx, const Stack& s, int layout, void* out, long lo
                                                        static_cast<uint4*>(out));
     return launched(ctx, "pack_quadg24_kernel");
   }
-  if (layout == kLayoutQuad32) {
-    if (s.n % 4) return set_error(ctx, FBP_ERR_UNSUPPORTED, "the interleaved layout needs a multiple of 4 views");
-    if (s.n / 4 > 65535) return set_error(ctx, FBP_ERR_UNSUPPORTED, "the interleaved layout takes up to 262140 views");
-    const dim3 grid((s.u + 255) / 256, std::min(s.v, 65535), s.n / 4);
-    pack_quad32_kernel<<<grid, 256, 0, ctx->stream>>>(s.f32, s.pitch, s.u, s.n, s.v, s.sinogram,
-                                                      static_cast<float4*>(out));
-    return launched(ctx, "pack_quad32_kernel");
+  if (is_quad_layout(layout) && !is_grad_layout(layout)) {
+    if (o.groups > 65535) return set_error(ctx, FBP_ERR_UNSUPPORTED, "interleaved views take up to 65535 view groups");
+    const int rows = s.v + (is_pair_layout(layout) ? 1 : 0);
+    const dim3 grid((unsigned)((pitch + 255) / 256), std::min(rows, 65535), o.groups);
+    auto kern = layout == kLayoutQuad32    ? pack_orbit_kernel<4, false>
+                : layout == kLayoutDuo32   ? pack_orbit_kernel<2, false>
+                : layout == kLayoutQuadP16 ? pack_orbit_kernel<4, true>
+                                           : pack_orbit_kernel<2, true>;
+    kern<<<grid, 256, 0, ctx->stream>>>(s.f32, s.pitch, s.u, s.n, s.v, s.sinogram, o.groups, o.mirror, view_scale, pitch,
+                                        static_cast<float*>(out));
+    return launched(ctx, "pack_orbit_kernel");
   }
   return set_error(ctx, FBP_ERR_INVALID_ARGUMENT, "unknown packed layout");
 }

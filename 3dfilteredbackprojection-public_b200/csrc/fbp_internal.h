@@ -50,11 +50,38 @@ enum FiltLayout : int {
   // holds the FP32 samples of views g + s K/4, s = 0..3. 16 bytes per element,
   // one plane; a tap reads two columns of two rows.
   kLayoutQuad32 = 5,
+  // The other rotational orbits of the generic kernel's geometries (struct
+  // Orbits): two views' FP32 samples (8 bytes), and four or two views' FP16
+  // row pairs (kLayoutPair16's values; 16 or 8 bytes).
+  kLayoutDuo32 = 6,
+  kLayoutQuadP16 = 7,
+  kLayoutDuoP16 = 8,
 };
 
+// Layouts of interleaved views, [group][element row][element column].
 constexpr bool is_quad_layout(int layout) { return layout >= kLayoutQuadG16; }
-// Layouts whose element carries its neighbours (one element row more than detector rows).
-constexpr bool is_pair_layout(int layout) { return layout == kLayoutPair16 || layout == kLayoutQuadG16 || layout == kLayoutQuadG24; }
+// Layouts whose element carries its neighbours (one element row more than
+// detector rows; the gradient quads one column more too).
+constexpr bool is_grad_layout(int layout) { return layout == kLayoutQuadG16 || layout == kLayoutQuadG24; }
+constexpr bool is_p16_layout(int layout) {
+  return layout == kLayoutPair16 || layout == kLayoutQuadP16 || layout == kLayoutDuoP16;
+}
+constexpr bool is_pair_layout(int layout) { return is_grad_layout(layout) || is_p16_layout(layout); }
+constexpr int slots_of(int layout) { return layout == kLayoutDuo32 || layout == kLayoutDuoP16 ? 2 : 4; }
+
+// How the views of a circular scan fall into rotational orbits: the pixel that
+// projects to detector position u at view k = g + m groups (m < phases) does
+// so, turned r times, at the view of slot (m + r) mod slots of group g: view
+// g + s groups for s < mirror, and the mirror image of view g + (s - mirror)
+// groups from there on (parallel beam: the view half a turn on).
+//   4 slots  one turn, K % 4 == 0 (4 phases, mirror 4); half a turn of
+//            parallel beam, K even (2 phases, mirror 2). Quarter turns.
+//   2 slots  one turn, K even (2 phases, mirror 2); any other parallel-beam
+//            view set (1 phase, mirror 1: the half-turned pixel in the same view)
+//   1 slot   any other fan / cone view set
+struct Orbits {
+  int slots = 1, groups = 0, phases = 1, mirror = 1;
+};
 
 // A stack of detector rows. Projections are [view][v][u] (rows ordered view
 // major), sinograms [v][view][u] (rows ordered v major). Rows of u samples
@@ -86,7 +113,11 @@ struct Stack {
   size_t rows() const { return (size_t)v * n; }
   size_t bytes32() const { return (size_t)pitch * rows() * sizeof(float); }
   static int elem_bytes(int layout) {
-    return layout == kLayoutQuadG24 ? 48 : layout == kLayoutQuadG16 ? 32 : layout == kLayoutQuad32 ? 16 : 4;
+    return layout == kLayoutQuadG24                                   ? 48
+           : layout == kLayoutQuadG16                                 ? 32
+           : layout == kLayoutQuad32 || layout == kLayoutQuadP16      ? 16
+           : layout == kLayoutDuo32 || layout == kLayoutDuoP16        ? 8
+                                                                      : 4;
   }
 };
 
@@ -235,8 +266,10 @@ int launch_elementwise_pre(fbp_context* ctx, const RowSet& rs);  // weight / log
 int launch_view_scales(fbp_context* ctx, const RowSet& rs, float limit, float* view_scale, float* inv_scale);
 // Pack the stack's f32 rows into a compact backprojector layout: kLayoutPair16
 // with row pitch `pitch` elements or kLayoutQuadG16 (FP16 with the per-view
-// scales view_scale), kLayoutQuadG24 (24-bit) or kLayoutQuad32 (no scale).
-int launch_pack(fbp_context* ctx, const Stack& s, int layout, void* out, long long pitch, const float* view_scale);
+// scales view_scale), kLayoutQuadG24 (24-bit, no scale), or the orbits' plain
+// samples and FP16 row pairs.
+int launch_pack(fbp_context* ctx, const Stack& s, int layout, const Orbits& o, void* out, long long pitch,
+                const float* view_scale);
 int launch_fft_rows(fbp_context* ctx, float2* data, int n, int rows, int inverse);
 int launch_fft_shift_rows(fbp_context* ctx, float2* data, int n, int rows, int shift);
 bool toeplitz_supported(int m);
@@ -260,13 +293,13 @@ struct BPGeom {
 // themselves; `mixed`: the reduced layouts. Sums are FP32 in every form.
 int launch_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, int clip_ylimit, bool mixed);
 // The same in two steps: plan (footprint pass, packing, tensor maps; work on
-// ctx's stream) and launch. Plans with the same non-zero batch key can also run
+// ctx's stream; `plain`: no interleaved views) and launch. Plans with the same non-zero batch key can also run
 // together in one persistent launch on another context's stream.
 struct BPLaunchPlan;
 BPLaunchPlan* new_bp_plan();
 void free_bp_plan(BPLaunchPlan* p);
 int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, int clip_ylimit, bool mixed,
-                     BPLaunchPlan* plan);
+                     BPLaunchPlan* plan, bool plain = false);
 int launch_bp_plan(fbp_context* ctx, const BPLaunchPlan& p);
 long long bp_plan_batch_key(const BPLaunchPlan& p);
 long long bp_plan_tiles(const BPLaunchPlan& p);  // work items (tile orbits x y-slabs) of a batchable plan
@@ -280,7 +313,7 @@ int launch_bp_batch(fbp_context* launcher, BPLaunchPlan* const* plans, int n, co
                     const long long* tile_end = nullptr);
 // (fbp_api.cu) size the stack's packed buffer for `layout`, compute the
 // per-view scales and pack the f32 rows into it.
-int prepare_packed(fbp_context* ctx, Stack& s, int layout);
+int prepare_packed(fbp_context* ctx, Stack& s, int layout, const Orbits& o);
 int launch_clip(fbp_context* ctx, float* vol, int nx, int ny, int nz, int y_limit);
 // 2D backprojection (g.ny == 1) of filtered rows [views][pitch] into image
 // [nz][nx]; FBP_ERR_UNSUPPORTED (nothing launched) when a tile's detector

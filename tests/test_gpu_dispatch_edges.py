@@ -5,6 +5,7 @@ import math
 
 import numpy as np
 import pytest
+import torch
 
 from conftest import relative_rmse
 
@@ -198,3 +199,75 @@ def test_generic_row_steps(fbp, oracle, precision, variant, n, ny, views, du):
     err, info = _noise_bp(fbp, oracle, c, precision, variant, sinograms=ny == 47)
     assert info["kernel"] == (variant.lower() if ny > 1 else "generic")  # one slice: the 2D tile
     assert err < TOL_BP["FP32" if precision == "MIXED24" else precision]
+
+
+@pytest.mark.parametrize("precision", ["FP32", "MIXED", "MIXED24"])
+@pytest.mark.parametrize("beam,n,ny,views,turns,du", [
+    ("cone", 50, 9, 8, 1.0, 1.5), ("cone", 49, 20, 12, 1.0, 2.25), ("cone", 33, 17, 4, 1.0, 0.75),     # quarter turns
+    ("cone", 64, 33, 10, 1.0, 1.5), ("cone", 49, 18, 14, 1.0, 0.5), ("cone", 17, 5, 2, 1.0, 2.25),      # half turns
+    ("cone", 40, 16, 9, 1.0, 1.5), ("cone", 40, 16, 12, 0.25, 1.5), ("cone", 40, 7, 12, 2.0, 1.5),      # none
+    ("parallel", 64, 24, 10, 0.5, 1.0), ("parallel", 49, 11, 66, 0.5, 0.8), ("parallel", 50, 8, 2, 0.5, 1.3),
+    ("parallel", 48, 16, 11, 0.5, 1.0), ("parallel", 49, 17, 13, 1.0, 0.7), ("parallel", 50, 40, 6, 0.3, 1.0),
+    ("parallel", 50, 21, 8, 1.0, 1.0), ("parallel", 17, 3, 6, 1.0, 1.0)])
+def test_orbits_of_the_generic_geometries(fbp, oracle, precision, beam, n, ny, views, turns, du):
+    """Two- and four-fold orbits off the symmetric kernel's sizes, mirrored
+    ones of parallel beam, odd sizes with their centre column or middle row,
+    and view sets without any, on white noise with a start angle, through
+    projections and sinograms."""
+    offset = float(np.float32(0.7))
+    c = dict(du=du, dv=du, span=2 * math.pi * float(np.float32(turns)), offset=offset, nu=int(2.0 * n / du),
+             nv=int(1.6 * n / du), nviews=views, nx=n, ny=ny, nz=n, vox=1.0)
+    if beam == "cone":
+        err, info = _noise_bp(fbp, oracle, dict(c, sod=4.0 * n, sdd=6.0 * n), precision, "AUTO", sinograms=n % 2 == 1)
+    else:
+        proj = np.random.default_rng(n + views).standard_normal((views, c["nv"], c["nu"])).astype(np.float32)
+        s = fbp.FBP3D(0)
+        s.set_clip_after_backprojection(False)
+        s.set_precision(getattr(fbp.Precision, precision))
+        if n % 2:
+            s.upload_sinograms(np.ascontiguousarray(proj.transpose(1, 0, 2)))
+            s.project_backward_parallel_from_sinograms(turns, n, ny, offset)
+        else:
+            s.upload_projections(proj)
+            s.project_backward_parallel_from_projections(turns, n, ny, offset)
+        got, info = s.read_volume(), s.last_backprojection()
+        s.ctx.close()
+        ref = oracle.bp_parallel3d(proj.astype(np.float64), dict(c, du=n / c["nu"], dv=ny / c["nv"]))
+        err = relative_rmse(got, ref)
+    assert info["kernel"] == "generic" and info["layout"] == ("pairs16" if precision == "MIXED" else "rows32")
+    assert err < TOL_BP["FP32" if precision == "MIXED24" else precision]
+
+
+@pytest.mark.parametrize("precision", ["FP32", "MIXED"])
+@pytest.mark.parametrize("views", [24, 26])
+def test_orbit_unstaged_windows(fbp, oracle, precision, views):
+    """Windows wider than the widest box of the four- and two-view elements."""
+    c = dict(sod=110.0, sdd=330.0, du=0.84, dv=0.84, span=2 * math.pi, offset=0.0, nu=260, nv=150, nviews=views, nx=50,
+             ny=16, nz=50, vox=1.0)
+    err, info = _noise_bp(fbp, oracle, c, precision, "AUTO")
+    assert info["kernel"] == "generic" and info["box"][0] > 128
+    assert err < TOL_BP[precision]
+
+
+@pytest.mark.parametrize("n,ny", [(64, 16), (120, 64)])
+def test_no_room_for_the_interleaved_copy(fbp, oracle, n, ny):
+    """FP32 views that fill the device: the interleaved copy (as many bytes
+    again) does not fit, and the plain kernel runs on the rows themselves."""
+    views, nu, nv = 128, 1024, 256
+    c = dict(sod=300.0, sdd=400.0, du=1.0, dv=1.0, span=2 * math.pi, offset=0.0, nu=nu, nv=nv, nviews=views, nx=n,
+             ny=ny, nz=n, vox=1.0)
+    proj = np.random.default_rng(n).standard_normal((views, nv, nu)).astype(np.float32)
+    s = fbp.FBP3D(0)
+    s.set_clip_after_backprojection(False)
+    s.set_precision(fbp.Precision.FP32)
+    s.upload_projections(proj)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    spare = torch.empty(max(0, torch.cuda.mem_get_info()[0] - proj.nbytes // 2), dtype=torch.uint8, device="cuda")
+    s.project_backward_cone_fdk_from_projections(300.0, 100.0, float(nu), float(n), 1.0, n, ny, 0.0)
+    got, info = s.read_volume(), s.last_backprojection()
+    s.ctx.close()
+    del spare
+    torch.cuda.empty_cache()
+    assert info["kernel"] == "generic" and info["layout"] == "rows32" and info["tile_ny"] == 16
+    assert relative_rmse(got, oracle.bp_cone(proj.astype(np.float64), c)) < TOL_BP["FP32"]
