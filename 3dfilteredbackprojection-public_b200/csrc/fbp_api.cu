@@ -571,13 +571,22 @@ int make_tensor_map_4d(fbp_context* ctx, CUtensorMap* map, CUtensorMapDataType d
                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
-int make_tensor_map_2d_bf16_sw128(fbp_context* ctx, CUtensorMap* map, void* base, uint64_t inner, uint64_t outer,
-                                  uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer) {
+int make_tensor_map_2d_bf16_sw64(fbp_context* ctx, CUtensorMap* map, void* base, uint64_t inner, uint64_t outer,
+                                 uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer) {
   const uint64_t dims[2] = {inner, outer};
   const uint64_t strides[1] = {pitch_bytes};
   const uint32_t box[2] = {box_inner, box_outer};
   return encode_tiled(ctx, map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box,
-                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+                      CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+}
+
+int make_tensor_map_2d_f32_sw128(fbp_context* ctx, CUtensorMap* map, void* base, uint64_t inner, uint64_t outer,
+                                 uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer) {
+  const uint64_t dims[2] = {inner, outer};
+  const uint64_t strides[1] = {pitch_bytes};
+  const uint32_t box[2] = {box_inner, box_outer};
+  return encode_tiled(ctx, map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box,
+                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
 int prepare_packed(fbp_context* ctx, Stack& s, int layout, const Orbits& o) {

@@ -48,7 +48,6 @@ namespace fbp {
 namespace {
 
 constexpr int kMaxStages = 8;                // shared-memory ring stages (one view each)
-constexpr int kMaxDynamicSmem = 227 * 1024;  // sm_100: largest dynamic shared memory of one CTA
 constexpr uint32_t kWaitLimit = 1u << 22;  // mbarrier polls before giving up
 
 struct ViewCoef {

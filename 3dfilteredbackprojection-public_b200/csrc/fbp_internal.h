@@ -364,13 +364,18 @@ int write_volume_files(fbp_context* ctx, const char* directory);
 int launch_project_ellipsoids(fbp_context* ctx, const double* d_ell, int count, const BPGeom& g,
                               float* out, int pitch);
 
+constexpr int kMaxDynamicSmem = 227 * 1024;  // sm_100: largest dynamic shared memory of one CTA
+
 // ---- TMA helpers ----
 int make_tensor_map_3d(fbp_context* ctx, CUtensorMap* map, CUtensorMapDataType dtype, void* base,
                        const uint64_t dims[3], const uint64_t strides_bytes[2], const uint32_t box[3]);
 int make_tensor_map_4d(fbp_context* ctx, CUtensorMap* map, CUtensorMapDataType dtype, void* base,
                        const uint64_t dims[4], const uint64_t strides_bytes[3], const uint32_t box[4]);
-// 2D BF16 rows (inner x outer, row pitch in bytes) with 128-byte swizzle.
-int make_tensor_map_2d_bf16_sw128(fbp_context* ctx, CUtensorMap* map, void* base, uint64_t inner, uint64_t outer,
-                                  uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer);
+// 2D rows (inner x outer, row pitch in bytes): BF16 with 64-byte swizzle, FP32
+// with 128-byte swizzle.
+int make_tensor_map_2d_bf16_sw64(fbp_context* ctx, CUtensorMap* map, void* base, uint64_t inner, uint64_t outer,
+                                 uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer);
+int make_tensor_map_2d_f32_sw128(fbp_context* ctx, CUtensorMap* map, void* base, uint64_t inner, uint64_t outer,
+                                 uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer);
 
 }  // namespace fbp

@@ -271,3 +271,36 @@ def test_no_room_for_the_interleaved_copy(fbp, oracle, n, ny):
     torch.cuda.empty_cache()
     assert info["kernel"] == "generic" and info["layout"] == "rows32" and info["tile_ny"] == 16
     assert relative_rmse(got, oracle.bp_cone(proj.astype(np.float64), c)) < TOL_BP["FP32"]
+
+
+# Split-BF16 rows: 2^-17 of white noise through the filter, as for the row
+# tests of the tensor-core filter (0.7e-5 to 1.3e-5 in an emulation).
+TOL_TOEPLITZ = 5e-5
+
+
+@pytest.mark.parametrize("views,nv,m", [
+    (1, 1, 64), (1, 3, 65), (1, 127, 95), (2, 64, 96), (3, 43, 97), (5, 26, 127), (1, 131, 128), (7, 11, 129),  # one tile
+    (1, 130, 191), (1, 130, 193), (2, 65, 255), (1, 129, 256), (1, 129, 257), (2, 61, 320), (1, 200, 383),
+    (2, 67, 385), (1, 77, 511), (1, 77, 513), (1, 130, 769), (3, 9, 1151), (1, 9, 2048), (1, 9, 2049), (1, 5, 8191),
+    (3, 1601, 70), (7, 1601, 640), (7, 1601, 641), (3, 1601, 650), (3, 1601, 2100),   # rows a warp, staged or not
+    (9, 8601, 130), (2, 20001, 700)])                                                     # more than one chunk
+@pytest.mark.parametrize("pre", [False, True])
+def test_toeplitz_rows_and_widths(fbp, oracle, views, nv, m, pre):
+    """The tensor-core row filter at the edges of its tiles, K blocks, rows a
+    warp and chunks, with and without the fused log and weight."""
+    rng = np.random.default_rng(m + nv)
+    proj = (np.exp(-0.5 * rng.random((views, nv, m))) * 1e4 if pre else rng.standard_normal((views, nv, m)) + 2.0)
+    proj = proj.astype(np.float32)
+    s = fbp.FBP3D(0)
+    s.set_filter_impl(fbp.FilterImpl.TOEPLITZ)
+    s.upload_projections(proj)
+    ref = proj.astype(np.float64)
+    if pre:
+        s.log_normalize_projections(1e4)
+        s.apply_fdk_weights_to_projections(3.0 * m, 1.0 * m, float(m))
+        ref = oracle.fdk_weight(-np.log(ref / 1e4), 4.0 * m, 1.0, 1.0)
+    s.apply_filter_to_projections(0)
+    got = s.download_projections()
+    s.ctx.close()
+    ref = oracle.filter_rows(ref.reshape(-1, m), 0).reshape(proj.shape)
+    assert relative_rmse(got, ref) < TOL_TOEPLITZ
