@@ -95,7 +95,7 @@ struct BPArgs {
   const uint4* qg;
   int qg_pitch, qg_rows;  // element columns per plane row, element rows per group
   // orbits of the interleaved layouts (struct Orbits) and their representative
-  // tiles; wrap: slots the sums move by from the last phase back to the first
+  // tiles; wrap: slots past one that the sums move by from the last phase to the first
   int groups, mirror, wrap;
   int nbx, nbz;
   int resident;           // CTAs resident on the GPU at once (view-group skew of the interleaved walk)
@@ -626,7 +626,6 @@ constexpr int kQFirst = 4;   // first quad of a work item (a tile orbit and y-sl
 constexpr int kQLast = 8;    // last quad of a work item: the consumers store its voxels next
 constexpr int kQExit = 16;   // multi-job launch: the queue is empty, the CTA leaves
 constexpr int kQTurn = 32;   // last view of a quarter turn: the sums move on by one slot
-constexpr int kQWrap = 128;  // .. from the last phase back to the first
 constexpr int kQShort = 64;  // rows advance by less than one per voxel everywhere in the tile
 
 // 16-byte aligned so that consumers read a record with vector loads: four for
@@ -769,7 +768,10 @@ constexpr int quad_threads(int layout, int NY, int YW) {
 // first quad and store its voxels after its last. An item's arithmetic and
 // view order do not depend on the launch, so a job's volume is the same bits
 // alone or batched with others.
-template <int LAYOUT, int NY, int YW, int OCC, bool MULTI>
+// EDGES: volumes that are not whole tiles to the half, and walks whose last
+// phase does not lead back by one slot (the epilogue's conditions cost the
+// 24-bit and the 12-high FP32 shapes 2 to 3% through their registers).
+template <int LAYOUT, int NY, int YW, int OCC, bool MULTI, bool EDGES>
 __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
     bp_quad_kernel(const __grid_constant__ BoxMaps maps, const __grid_constant__ BPArgs a,
                    const __grid_constant__ QuadQueue qq) {
@@ -779,6 +781,10 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
   constexpr bool P16 = is_p16_layout(LAYOUT);
   constexpr bool GRAD = is_grad_layout(LAYOUT);
   constexpr int S = slots_of(LAYOUT);
+  // whether a step tells the end of a phase, or the walk counts (512^3, 24-bit
+  // 46.5 / 46.4 ms, 960-wide FP32 273.8 / 266.4, 768^3 FP16 163.7 / 165.6: what
+  // ptxas keeps in registers)
+  constexpr bool FLAGGED = MULTI || LAYOUT == kLayoutQuadG16;
   constexpr int NPL = Q24 ? 3 : GRAD ? 2 : 1;  // planes per element row
   constexpr int CB = S == 4 ? 16 : 8;          // bytes per column of a plane
   constexpr int ESZ = CB * NPL;
@@ -880,8 +886,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
           for (int r = 0; r < S; ++r)
             qc.ws[r] = ja.inv_scale ? ja.inv_scale[k % Q + (r < ja.mirror ? r : r - ja.mirror) * Q] : 1.0f;
           qc.flags = (skip ? kQSkip : 0) | (direct ? kQDirect : 0) | (it == 0 ? kQFirst : 0) |
-                     (it == K - 1 ? kQLast : 0) | ((k + 1) % Q == 0 ? kQTurn : 0) | (k == K - 1 ? kQWrap : 0) |
-                     (vc.skip & 2 ? kQShort : 0);
+                     (it == K - 1 ? kQLast : 0) | ((k + 1) % Q == 0 ? kQTurn : 0) | (vc.skip & 2 ? kQShort : 0);
           // window: width (elements) and rows
           const int BU = direct ? need_u : jm.w[wi], BV = direct ? rows : jm.h[hi];
           qc.grp = k % Q;
@@ -1030,8 +1035,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
   reset();
   int e = 0;
   uint32_t ph = 0;
-  bool bad = false, stop = false, last = false, leave = false;
-  int turned = 0;  // slots the sums move by after this view
+  bool bad = false, stop = false, last = false, leave = false, turned = false;
   long long item = -1;  // work item being accumulated
   int jb = 0;         // its job
   // one quad: wait for its window, apply it to the 4 x NY voxels, release it
@@ -1318,7 +1322,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
       e = 0;
       ph ^= 1;
     }
-    turned = flags & kQTurn ? (flags & kQWrap ? (MULTI ? 1 : a.wrap) : 1) : 0;
+    if (FLAGGED) turned = (flags & kQTurn) != 0;
   };
   // the item's sums into its voxels: the rotated columns, (x, z) ->
   // (n-1-z, x) -> (n-1-x, n-1-z) -> (z, n-1-x), or (x, z) -> (n-1-x, n-1-z)
@@ -1333,8 +1337,8 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
     // row; columns that are their own image are rotation 0's alone
     const int n = ja.nx, h = n >> 1;
     const int ix = til.ix0 + tx, iz = til.iz0 + tz;
-    const bool mid = (n & 1) && iz == h && (S == 2 || ix == h);
-    const bool own = (S == 4 ? ix < n - h : ix < n) && (iz < h || mid);
+    const bool mid = EDGES && (n & 1) && iz == h && (S == 2 || ix == h);
+    const bool own = !EDGES || ((S == 4 ? ix < n - h : ix < n) && (iz < h || mid));
     const int cx[4] = {ix, S == 4 ? n - 1 - iz : n - 1 - ix, n - 1 - ix, iz};
     const int cz[4] = {iz, S == 4 ? ix : n - 1 - iz, n - 1 - iz, n - 1 - ix};
     float* const vol = ja.vol;
@@ -1365,13 +1369,15 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
     const int K = a.nviews;
     // the phases, the first one entered at its view k0 mod Q and finished at
     // the end (the turns stay out of the inner loop)
-    const int Q = a.groups, first = Q - item_tile<TY>(a, item).k0 % Q;
+    const int Q = a.groups, k0 = item_tile<TY>(a, item).k0, first = Q - k0 % Q;
     int left = K;
     for (int n = first; left > 0 && !stop; n = min(Q, left)) {
       left -= n;
 #pragma unroll 2
       for (int q = 0; q < n; ++q) { step(); if (stop) break; }
-      for (int i = 0; i < turned; ++i) turn();
+      if (FLAGGED ? turned : (k0 - left) % Q == 0) turn();
+      if (EDGES && k0 == left)  // from the last phase back to the first
+        for (int i = 0; i < a.wrap; ++i) turn();
     }
     if (bad) atomicCAS(a.err, 0, kDevFootprint);
     if (stop || *s_abort) return;
@@ -1382,7 +1388,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
     do step();
     while (!(stop || leave || turned || last));
     if (stop || leave) break;
-    for (int i = 0; i < turned; ++i) turn();
+    if (turned) turn();
     if (last) {
       if (bad) atomicCAS(job_args<MULTI>(a, qq, jb).err, 0, kDevFootprint);
       bad = false;
@@ -1503,9 +1509,9 @@ cudaError_t launch_cfg(const BoxMaps& maps, const BPArgs& a, size_t smem, cudaSt
   return cudaGetLastError();
 }
 
-template <int LAYOUT, int NY, int YW, int OCC>
+template <int LAYOUT, int NY, int YW, int OCC, bool EDGES>
 cudaError_t launch_quad_cfg(const BoxMaps& maps, const BPArgs& a, size_t smem, cudaStream_t stream) {
-  auto kern = bp_quad_kernel<LAYOUT, NY, YW, OCC, false>;
+  auto kern = bp_quad_kernel<LAYOUT, NY, YW, OCC, false, EDGES>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   if (e != cudaSuccess) return e;
   // all of L1 as shared memory, so that two CTAs of up to 113 KB share an SM
@@ -1533,16 +1539,15 @@ cudaError_t launch_quad_cfg(const BoxMaps& maps, const BPArgs& a, size_t smem, c
 
 cudaError_t launch_quad(int layout, int ny_tile, const BoxMaps& maps, const BPArgs& a, size_t smem,
                         cudaStream_t stream) {
-#define FBP_LAUNCH(L, NY, YW, OCC) launch_quad_cfg<L, NY, YW, OCC>(maps, a, smem, stream)
-  switch (layout) {
-    case kLayoutDuo32:
-      return FBP_LAUNCH(kLayoutDuo32, 16, 1, 2);
-    case kLayoutQuadP16:
-      return FBP_LAUNCH(kLayoutQuadP16, 8, 1, 2);
-    case kLayoutDuoP16:
-      return FBP_LAUNCH(kLayoutDuoP16, 16, 1, 2);
-      FBP_SYMMETRIC_SHAPES(FBP_LAUNCH)
-  }
+#define FBP_LAUNCH(L, NY, YW, OCC) launch_quad_cfg<L, NY, YW, OCC, false>(maps, a, smem, stream)
+#define FBP_EDGES(L, NY, YW, OCC) launch_quad_cfg<L, NY, YW, OCC, true>(maps, a, smem, stream)
+  if (layout == kLayoutDuo32) return FBP_EDGES(kLayoutDuo32, 16, 1, 2);
+  if (layout == kLayoutQuadP16) return FBP_EDGES(kLayoutQuadP16, 8, 1, 2);
+  if (layout == kLayoutDuoP16) return FBP_EDGES(kLayoutDuoP16, 16, 1, 2);
+  if (layout == kLayoutQuad32 && (a.nx % 32 || a.wrap))
+    return ny_tile == 12 ? FBP_EDGES(kLayoutQuad32, 12, 1, 2) : FBP_EDGES(kLayoutQuad32, 8, 1, 2);
+  switch (layout) { FBP_SYMMETRIC_SHAPES(FBP_LAUNCH) }
+#undef FBP_EDGES
 #undef FBP_LAUNCH
 }
 
@@ -1558,7 +1563,9 @@ int quad_occ(int layout, int ny_tile) {
 // high 0.56, 0.59, 1.11, 7.6. FP32 and 24-bit take 12 from 36 waves on
 // (about 440^3): 8 and 12 high 0.31 and 0.47, 0.50 and 0.77, 1.40 and 1.48, 9.8
 // and 10.1 at those sizes, then 18.9 and 17.6 at 480 x 490 x 480 (480 views),
-// 38.1 and 37.2 at 512^3 (720 views; 24-bit 49.3 and 46.4).
+// 38.1 and 37.2 at 512^3 (720 views; 24-bit 49.3 and 46.4); and where it makes
+// one wave of more than 1.2 (160 x 128 x 160: 0.87 and 0.72, 24-bit 0.90 and
+// 0.86; 128 x 153 x 128, 1.08 waves, 0.59 and 0.81).
 int quad_tile_height(int asked, int layout, int orbits, int ny, int num_sms) {
   if (asked) return asked;
   if (layout == kLayoutDuo32 || layout == kLayoutDuoP16) return 16;
@@ -1571,7 +1578,7 @@ int quad_tile_height(int asked, int layout, int orbits, int ny, int num_sms) {
     const double c16 = 0.36 * (fullest(16) + 0.15), c24 = 0.47 * (fullest(24) + 0.2);
     return c8 < c16 && c8 < c24 ? 8 : c16 < c24 ? 16 : 24;
   }
-  return waves(8) >= 36.0 ? 12 : 8;
+  return waves(8) >= 36.0 || (waves(8) > 1.2 && waves(12) <= 1.0) ? 12 : 8;
 }
 
 template <int TX, int TZ, int NY>
@@ -1847,7 +1854,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   }
   a.groups = orb.groups;
   a.mirror = orb.mirror;
-  a.wrap = (orb.slots - orb.phases + 1) % orb.slots;
+  a.wrap = (orb.slots - orb.phases) % orb.slots;
   const int half = ((g.nx + 1) / 2 + 15) / 16;
   a.nbx = orb.slots == 4 ? half : (g.nx + 15) / 16;
   a.nbz = orb.slots == 1 ? (g.nx + 15) / 16 : half;
@@ -2159,7 +2166,7 @@ namespace {
 
 template <int LAYOUT, int NY, int YW, int OCC>
 cudaError_t launch_quad_multi_cfg(const QuadQueue& qq, size_t smem, int grid, cudaStream_t stream) {
-  auto kern = bp_quad_kernel<LAYOUT, NY, YW, OCC, true>;
+  auto kern = bp_quad_kernel<LAYOUT, NY, YW, OCC, true, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
