@@ -44,7 +44,9 @@ __device__ __forceinline__ float load_pre(const RowSet& rs, long long r, int i) 
 }
 
 __device__ __forceinline__ int row_view(const RowSet& rs, long long r) {
-  return rs.sinogram ? (int)(r % rs.n_views) : (int)(r / rs.n_v);
+  if (r >> 32) return rs.sinogram ? (int)(r % rs.n_views) : (int)(r / rs.n_v);
+  const unsigned row = (unsigned)r;
+  return (int)(rs.sinogram ? row % (unsigned)rs.n_views : row / (unsigned)rs.n_v);
 }
 
 }  // namespace fbp
