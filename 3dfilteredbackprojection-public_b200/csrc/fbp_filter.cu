@@ -302,11 +302,11 @@ __device__ __forceinline__ void fft_inverse(float2 (&x)[E], const float2* tws, i
 // over the pairs; a block holds as many groups as its size allows. Groups of
 // up to a warp synchronise by warp, larger ones through a named barrier each.
 //
-// Bound: the load / store unit (78-83% busy: exchanges, twiddles and the two
-// half-written elements of a pair). Measured into FP32 pairs, before = radix-4
-// passes through shared memory with block barriers: 138240 rows of 384 (n =
-// 512) 819 -> 211 us (637 MB: 3.0 TB/s), 138240 rows of 768 (n = 1024) 1628 ->
-// 493 us, 92160 rows of 1536 (n = 2048) 2288 -> 646 us. Four blocks a SM at 64
+// Bound: the load / store unit (78-83% busy: exchanges and twiddles). Measured
+// with the rows in place, before = radix-4 passes through shared memory with
+// block barriers into pairs of rows: 138240 rows of 384 (n = 512) 819 -> 183 us
+// (425 MB: 2.3 TB/s), 138240 rows of 768 (n = 1024) 1628 -> 424 us, 92160 rows
+// of 1536 (n = 2048) 2288 -> 518 us. Four blocks a SM at 64
 // registers spill and are 1-14% slower, E = 16 for n = 1024, 2048 1.4 times
 // slower, the twiddles held in registers (one block a SM) 2 times.
 template <int L>
@@ -616,8 +616,8 @@ __device__ __forceinline__ uint32_t store24(float x) {
 // stored as 3-byte little-endian fields of 12 words, written as three
 // 16-byte plane entries. 4 bytes read and 12 written per sample;
 // with the nearest of three candidates searched for and the fields shifted into
-// place it was bound by its instructions (480 views of 768 x 768: 2.92 ms, now
-// 1.31; the bytes take 0.69).
+// place it was bound by its instructions (720 views of 768 x 768: 2.92 ms, now
+// 1.31; the bytes take 1.04).
 __global__ void pack_quadg24_kernel(const float* src, long long spitch, int m, int n_views, int n_v, bool sinogram,
                                     uint4* out) {
   // grid: x over element columns, y over runs of kPackRows element rows, z

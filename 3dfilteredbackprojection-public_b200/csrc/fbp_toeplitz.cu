@@ -638,7 +638,12 @@ int launch_filter_toeplitz(fbp_context* ctx, const RowSet& rs, int n, int filter
   // and 256 KB per padded sample) stay in the L2 cache between the two kernels
   const long long wave = (long long)ctx->num_sms * BM;
   const long long cap = std::min((96LL << 20), 65536LL * 4 * (kp + 64)) / (4LL * kx);
-  const long long chunk = std::min<long long>(rs.rows, cap >= wave ? cap / wave * wave : std::max(cap / BM, 1LL) * BM);
+  long long rows = cap / wave * wave;
+  if (rows == 0) {  // long rows: the row tiles of whole waves of 256-wide tiles
+    const long long nt = (m + BN - 1) / BN, w = cap / BM * nt / ctx->num_sms;
+    rows = std::max(w > 0 ? w * ctx->num_sms / nt : cap / BM, 1LL) * BM;
+  }
+  const long long chunk = std::min<long long>(rs.rows, rows);
   const size_t sbytes = sizeof(__nv_bfloat16) * (size_t)chunk * kx;
   unsigned char* sp = static_cast<unsigned char*>(scratch(ctx, 2 * sbytes + 1024));
   if (!sp) return FBP_ERR_OUT_OF_MEMORY;
