@@ -2018,9 +2018,10 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
 
   if (packed && !(st.pack_ready && st.filt_layout == layout))
     if (int rc = prepare_packed(ctx, st, layout, orb)) {
-      // no room for the interleaved copy: the plain kernel reads the rows
-      // themselves, or pairs of at most the orbits' bytes
-      if (rc == FBP_ERR_OUT_OF_MEMORY && (orbit || layout == kLayoutQuad32))
+      // no room for the interleaved copy, or more view groups than its packer
+      // takes: the plain kernel reads the rows themselves, or pairs of at most
+      // the orbits' bytes
+      if ((rc == FBP_ERR_OUT_OF_MEMORY || rc == FBP_ERR_UNSUPPORTED) && (orbit || layout == kLayoutQuad32))
         return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, true);
       return rc;
     }

@@ -304,3 +304,20 @@ def test_toeplitz_rows_and_widths(fbp, oracle, views, nv, m, pre):
     s.ctx.close()
     ref = oracle.filter_rows(ref.reshape(-1, m), 0).reshape(proj.shape)
     assert relative_rmse(got, ref) < TOL_TOEPLITZ
+
+
+def test_more_view_groups_than_the_packer_takes(fbp):
+    """65540 views without a turn (one group each) run on the plain kernel."""
+    views, n, ny = 65540, 208, 8
+    sino = np.random.default_rng(3).standard_normal((2, views, 32)).astype(np.float32)
+    out = []
+    for variant in (fbp.Backprojector.AUTO, fbp.Backprojector.GENERIC_Y8):
+        s = fbp.FBP3D(0)
+        s.set_clip_after_backprojection(False)
+        s.set_precision(fbp.Precision.FP32)
+        s.set_backprojector(variant)
+        s.upload_sinograms(sino)
+        s.project_backward_parallel_from_sinograms(0.3, n, ny, 0.1)
+        out.append(s.read_volume())
+        s.ctx.close()
+    assert relative_rmse(out[0], out[1]) < TOL_BP["FP32"]
