@@ -414,8 +414,7 @@ int autotune_backprojector(fbp_context* ctx, Stack& s, const fbp::BPGeom& g, boo
       rc = r;
       break;
     }
-    s.pack_ready = true;  // the timed launch reuses the packed views
-    cudaEventRecord(e0, ctx->stream);
+    cudaEventRecord(e0, ctx->stream);  // the timed launch reuses what that one packed
     r = fbp::launch_backproject(ctx, gt, s, ctx->vol + (size_t)y0 * g.nx, 0, mixed);
     cudaEventRecord(e1, ctx->stream);
     if (r || (r = sync_host(ctx, true))) {
@@ -469,6 +468,7 @@ int setup_backproject(fbp_context* ctx, Stack& s, fbp::BPGeom& g, int* ylim, boo
   if (!(g.du > 0.0) || !(g.vox > 0.0))
     return fbp::set_error(ctx, FBP_ERR_INVALID_ARGUMENT, "detector and volume widths must be positive");
   FBP_TRY(flush_pending(ctx, s));
+  s.pack_ready = false;  // a new call, other rows
   FBP_TRY(ensure_volume(ctx, g.nx, g.ny, g.nz, false));
   *ylim = ctx->clip_after_bp ? clip_limit : 0;
   *mixed = ctx->precision != FBP_PRECISION_FP32;
@@ -488,7 +488,6 @@ int backproject(fbp_context* ctx, Stack& s, fbp::BPGeom g) {
       rc = fbp::launch_backproject(ctx, g, s, ctx->vol, ylim, mixed);
       apply_shape(ctx, saved);
     }
-    s.pack_ready = false;
     // the outer slices can have wider windows than the tuning slab: the
     // untuned selection still applies there
     if (rc != FBP_ERR_UNSUPPORTED) return rc;
@@ -596,6 +595,9 @@ int prepare_packed(fbp_context* ctx, Stack& s, int layout, const Orbits& o) {
   const int esize = Stack::elem_bytes(layout);
   const int fpitch = fbp::is_grad_layout(layout) ? s.u + 1 : round_up(s.u, std::max(1, 16 / esize));
   const size_t need = (size_t)(quad ? o.groups : s.n) * (s.v + pair) * (size_t)fpitch * esize;
+  // until these rows are packed, filt holds nothing that a later slab may take
+  s.pack_ready = false;
+  s.filt_layout = kLayoutRaw32;
   if (!s.filt || s.filt_bytes < need) {
     cudaFree(s.filt);
     s.filt = nullptr;
@@ -620,6 +622,7 @@ int prepare_packed(fbp_context* ctx, Stack& s, int layout, const Orbits& o) {
   if (int rc = launch_pack(ctx, s, layout, o, s.filt, fpitch, scale)) return rc;
   s.filt_layout = layout;
   s.filt_pitch = fpitch;
+  s.pack_ready = true;
   return FBP_OK;
 }
 
@@ -1427,7 +1430,7 @@ int fbp_reconstruct_fdk_to_host(fbp_context* ctx, const float* projections, int 
   Stack& s = ctx->proj;
   // upload (the host buffer should be pinned), weights, filter
   if (!(s.f32 && s.u == cols && s.v == rows && s.n == count)) FBP_TRY(alloc_stack(ctx, s, cols, rows, count, false));
-  s.filtered = false;
+  s.filtered = s.pack_ready = false;
   s.log_pending = s.weights_pending = false;
   FBP_TRY(fbp::cuda_check(ctx,
                           copy_rows(s.f32, (size_t)s.pitch * 4, projections, (size_t)cols * 4, (size_t)cols * 4,
@@ -1466,7 +1469,8 @@ int fbp_reconstruct_fdk_to_host(fbp_context* ctx, const float* projections, int 
     if (rc == FBP_OK) apply_shape(ctx, shape);
   }
   // y-slab k is backprojected straight into the whole volume, then copied to
-  // the host on the copy stream while slab k + 1 computes
+  // the host on the copy stream while slab k + 1 computes. A slab reuses the
+  // views that an earlier one packed, where it wants them in that layout.
   for (int k = 0; k < slabs && rc == FBP_OK; ++k) {
     const int y0 = (int)((long long)v * k / slabs), y1 = (int)((long long)v * (k + 1) / slabs);
     fbp::BPGeom gs = gg;
@@ -1481,7 +1485,6 @@ int fbp_reconstruct_fdk_to_host(fbp_context* ctx, const float* projections, int 
       apply_shape(ctx, saved);
       rc = fbp::launch_backproject(ctx, gs, s, ctx->vol + (size_t)y0 * h, ylim, mixed);
     }
-    s.pack_ready = true;  // the first slab packed the views: the others reuse them
     if (rc) break;
     if ((rc = fbp::cuda_check(ctx, cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming), "event")) ||
         (rc = fbp::cuda_check(ctx, cudaEventRecord(done[k], ctx->stream), "event")) ||

@@ -101,7 +101,10 @@ struct Stack {
   float* inv_scale = nullptr;     // per view (x2: [inv | scale]) for the FP16 layouts
   int scale_cap = 0;              // views inv_scale has room for
   size_t f32_cap = 0;             // bytes allocated at f32 (buffers only grow: no cudaFree between jobs)
-  bool pack_ready = false;        // filt already holds f32 packed as filt_layout (slabs of one reconstruction)
+  // filt holds f32 as it is, packed as filt_layout. Set by prepare_packed alone
+  // (a slab or a tuning launch may run on the rows and pack nothing), cleared
+  // where a call that backprojects begins: nothing tells of writes to f32 between calls.
+  bool pack_ready = false;
   // Log normalisation and FDK weights recorded by their calls and applied
   // inside the filter kernel's load (log first, then weight), or by a
   // standalone pass when something else reads the rows first.
