@@ -1971,12 +1971,14 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   size_t smem = 0;
   bool use_quad = quad || orbit;
   if (orbit) {
-    // what the plain kernel refuses stays refused: two windows of its ring
-    // (16-voxel tiles; rows, or pairs of filtered FP32 rows) in half an SM
+    // Windows of a size at which two in half an SM (the plain kernel's least
+    // ring; rows, or pairs of filtered FP32 rows) are in doubt, by these tiles'
+    // windows taken to 16 voxels: the plain kernel, whose own windows decide.
+    // They are smaller than that where the rows spread with the distance too.
     const int rows16 = ((p16 ? bv : fv) - 2) * 16 / NY + 2;
     const size_t box = ((size_t)(p16 ? (plan.box_u + 3) / 4 * 4 : fu) * rows16 * (fp32 && st.filtered ? 8 : 4) + 127) / 128 * 128;
     if ((113 * 1024 - 64) / (box + sizeof(ViewCoef) + 2 * sizeof(uint64_t)) < 2)
-      return set_error(ctx, FBP_ERR_UNSUPPORTED, "staged detector window does not fit in shared memory");
+      return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, true);
   }
   if (use_quad) {
     // byte ring for the windows + entry records

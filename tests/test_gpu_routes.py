@@ -100,3 +100,27 @@ def test_slabs_after_a_packing_that_found_no_room(fbp):
     t.ctx.close()
     assert layout == "rows32"
     assert relative_rmse(got, ref) < TOL_BP
+
+
+# --------------------------------------------------------------- windows near the kernels' limits
+@pytest.mark.parametrize("precision,views,cols,rows", [
+    ("FP32", 180, 217, 217), ("FP32", 182, 217, 217),                           # 67 x 87 samples a 16-high tile
+    ("MIXED24", 180, 300, 300), ("MIXED", 180, 300, 300), ("MIXED", 182, 300, 300)])  # 91 x 119
+def test_windows_too_large_for_an_estimate(fbp, oracle, precision, views, cols, rows):
+    """Volumes off the symmetric sizes whose 8- or 12-high tiles' windows,
+    taken to 16 voxels, would not fit twice in half an SM, while the plain
+    kernel's do."""
+    n, ny, width, sod, odd = 100, 100, 193.33, 150.0, 50.0
+    c = dict(sod=sod, sdd=sod + odd, du=float(np.float32(width)) / cols, dv=float(np.float32(width)) / cols,
+             span=2 * math.pi, offset=0.0, nu=cols, nv=rows, nviews=views, nx=n, ny=ny, nz=n, vox=1.0)
+    proj = _noise(5, views, rows, cols)
+    s = _solver(fbp, precision)
+    s.upload_projections(proj)
+    s.apply_filter_to_projections(0)
+    filtered = s.download_projections()
+    s.project_backward_cone_fdk_from_projections(sod, odd, width, float(n), 1.0, n, ny, 0.0)
+    got = s.read_volume()
+    s.ctx.close()
+    ref = oracle.bp_cone(filtered.astype(np.float64), c)
+    # FP16 views: 2^-12 of a value (2.4e-4)
+    assert relative_rmse(got, ref) < (4e-4 if precision == "MIXED" else TOL_BP)
