@@ -1783,7 +1783,7 @@ struct BPLaunchPlan {
   BoxMaps maps;
   size_t smem = 0;
   int layout = 0, ny_tile = 0, occ = 2;
-  bool use_quad = false, is2d = false;
+  bool use_quad = false;
   bool orbit = false;  // the quad kernel on an orbit of the generic backprojector's geometries
 };
 
@@ -1791,7 +1791,7 @@ BPLaunchPlan* new_bp_plan() { return new BPLaunchPlan(); }
 void free_bp_plan(BPLaunchPlan* p) { delete p; }
 
 int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, int clip_ylimit, bool mixed,
-                     BPLaunchPlan* plan_out, bool plain) {
+                     BPLaunchPlan* plan_out, const PlanLimits& lim) {
   const double pi = 3.14159265358979323846;
   // MIXED24: 24-bit views for the symmetric kernel (FP32 rows otherwise)
   const bool c24 = mixed && ctx->precision == FBP_PRECISION_MIXED24;
@@ -1802,7 +1802,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   const long long iturns = llround(turns);
   const bool symmetric = !is2d && g.nx == g.nz && g.nx % 32 == 0 && g.nviews % 4 == 0 &&
                          fabs(turns - (double)iturns) < 1e-9 && iturns % 4 == 1;
-  const bool quad = symmetric && !plain &&
+  const bool quad = symmetric && !lim.plain &&
                     (ctx->bp_variant == FBP_BACKPROJECTOR_AUTO || ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC);
   if (ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC && !symmetric)
     return set_error(ctx, FBP_ERR_UNSUPPORTED,
@@ -1814,7 +1814,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   // the plain kernel's.
   const bool p16 = mixed && !c24;
   Orbits orb = find_orbits(g.kind == FBP_GEOMETRY_CONE, turns, g.nviews, g.nx == g.nz);
-  const bool orbit = !quad && !is2d && !plain && g.nx == g.nz && ctx->bp_stages == 0 &&
+  const bool orbit = !quad && !is2d && !lim.plain && g.nx == g.nz && ctx->bp_stages == 0 &&
                      (ctx->bp_variant == FBP_BACKPROJECTOR_AUTO || ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC) &&
                      choose_orbits(g, turns, p16, ctx->num_sms, &orb);
   // what the selected kernel reads: interleaved views (symmetric, orbits), FP16
@@ -1875,7 +1875,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   const int NY = is2d    ? 1
                  : quad  ? quad_tile_height(ctx->quad_tile_ny, layout, a.nbx * a.nbz, g.ny, ctx->num_sms)
                  : orbit ? quad_tile_height(0, layout, a.nbx * a.nbz, g.ny, ctx->num_sms)
-                         : (ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC_Y8 ? 8 : 16);
+                         : std::min(lim.max_height, ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC_Y8 ? 8 : 16);
   a.ntx = (g.nx + TX - 1) / TX;
   a.ntz = (g.nz + TZ - 1) / TZ;
   const int nty = (g.ny + NY - 1) / NY;
@@ -1920,7 +1920,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     // few blocks: each adds its whole shared histogram to the global one
     const int blocks = (int)std::max(1LL, std::min<long long>((ntiles + 7) / 8, (long long)ctx->num_sms * 2));
     const size_t hist_smem = sizeof(unsigned) * kBoxHist * kBoxHist;
-    auto fk = is2d       ? footprint_kernel<16, 16, 1>
+    auto fk = NY == 1    ? footprint_kernel<16, 16, 1>
               : NY == 8  ? footprint_kernel<16, 16, 8>
               : NY == 12 ? footprint_kernel<16, 16, 12>
               : NY == 16 ? footprint_kernel<16, 16, 16>
@@ -1962,6 +1962,11 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     return set_error(ctx, FBP_ERR_UNSUPPORTED,
                      "detector footprint of a voxel tile exceeds the 256-element TMA box; geometry magnification "
                      "too large for the staged backprojector");
+  // A box holds 256 rows. FP32 rows take one more than the pairs of rows that
+  // the limit above is about (parallel beam, 17 detector rows a voxel: 257 for
+  // 16 voxels): lower tiles, down to one slice.
+  if (layout == kLayoutRaw32 && bv > 256 && NY > 1)
+    return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{true, NY > 8 ? 8 : 1});
   a.box_u = bu;
   a.box_v = bv;
   // two CTAs per SM: each gets half of the 228 KB shared memory
@@ -1978,7 +1983,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     const int rows16 = ((p16 ? bv : fv) - 2) * 16 / NY + 2;
     const size_t box = ((size_t)(p16 ? (plan.box_u + 3) / 4 * 4 : fu) * rows16 * (fp32 && st.filtered ? 8 : 4) + 127) / 128 * 128;
     if ((113 * 1024 - 64) / (box + sizeof(ViewCoef) + 2 * sizeof(uint64_t)) < 2)
-      return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, true);
+      return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{true});
   }
   if (use_quad) {
     // byte ring for the windows + entry records
@@ -2004,7 +2009,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
       // re-plan with the generic tile height
       const int saved = ctx->bp_variant;
       ctx->bp_variant = FBP_BACKPROJECTOR_GENERIC;
-      const int rc = plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out);
+      const int rc = plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, lim);
       ctx->bp_variant = saved;
       return rc;
     }
@@ -2024,7 +2029,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
       // takes: the plain kernel reads the rows themselves, or pairs of at most
       // the orbits' bytes
       if ((rc == FBP_ERR_OUT_OF_MEMORY || rc == FBP_ERR_UNSUPPORTED) && (orbit || layout == kLayoutQuad32))
-        return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, true);
+        return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{true});
       return rc;
     }
   a.inv_scale = is_p16_layout(layout) || layout == kLayoutQuadG16 ? st.inv_scale : nullptr;  // set by the pack
@@ -2054,7 +2059,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
         mbu = wider;
         break;
       }
-  const int mbv = is_quad_layout(layout) ? std::min(bv, std::max(1, (int)(a.box_bytes / (esize * mbu)))) : bv;
+  const int mbv = is_quad_layout(layout) ? std::min({bv, 256, std::max(1, (int)(a.box_bytes / (esize * mbu)))}) : bv;
   if (!(plan.sel_layout == layout && plan.sel_u == mbu && plan.sel_v == mbv)) {
     // the interleaved layouts take the boxes fitted to the histogram (C4: the
     // MIXED backprojection 1405 -> 1289 ms); the others keep the quarter steps
@@ -2129,7 +2134,6 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   p.ny_tile = NY;
   p.occ = occ;
   p.use_quad = use_quad;
-  p.is2d = is2d;
   p.orbit = orbit;
   return FBP_OK;
 }
@@ -2146,7 +2150,7 @@ int launch_bp_plan(fbp_context* ctx, const BPLaunchPlan& p) {
   ctx->last_bp[3] = p.a.box_v;
   ctx->last_bp[4] = NY;
   cudaError_t e = p.use_quad ? launch_quad(p.layout, NY, p.maps, p.a, p.smem, ctx->stream)
-                  : p.is2d   ? launch_layout<16, 16, 1>(p.layout, p.maps, p.a, p.smem, ctx->stream)
+                  : NY == 1  ? launch_layout<16, 16, 1>(p.layout, p.maps, p.a, p.smem, ctx->stream)
                   : NY == 8  ? launch_layout<16, 16, 8>(p.layout, p.maps, p.a, p.smem, ctx->stream)
                              : launch_layout<16, 16, 16>(p.layout, p.maps, p.a, p.smem, ctx->stream);
   if (e == cudaSuccess) ctx->launches++;

@@ -296,13 +296,17 @@ struct BPGeom {
 // themselves; `mixed`: the reduced layouts. Sums are FP32 in every form.
 int launch_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, int clip_ylimit, bool mixed);
 // The same in two steps: plan (footprint pass, packing, tensor maps; work on
-// ctx's stream; `plain`: no interleaved views) and launch. Plans with the same non-zero batch key can also run
+// ctx's stream) and launch. Plans with the same non-zero batch key can also run
 // together in one persistent launch on another context's stream.
 struct BPLaunchPlan;
+struct PlanLimits {
+  bool plain = false;   // no interleaved views
+  int max_height = 16;  // of the plain kernel's tiles
+};
 BPLaunchPlan* new_bp_plan();
 void free_bp_plan(BPLaunchPlan* p);
 int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, int clip_ylimit, bool mixed,
-                     BPLaunchPlan* plan, bool plain = false);
+                     BPLaunchPlan* plan, const PlanLimits& lim = {});
 int launch_bp_plan(fbp_context* ctx, const BPLaunchPlan& p);
 long long bp_plan_batch_key(const BPLaunchPlan& p);
 long long bp_plan_tiles(const BPLaunchPlan& p);  // work items (tile orbits x y-slabs) of a batchable plan

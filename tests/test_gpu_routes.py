@@ -124,3 +124,25 @@ def test_windows_too_large_for_an_estimate(fbp, oracle, precision, views, cols, 
     ref = oracle.bp_cone(filtered.astype(np.float64), c)
     # FP16 views: 2^-12 of a value (2.4e-4)
     assert relative_rmse(got, ref) < (4e-4 if precision == "MIXED" else TOL_BP)
+
+
+@pytest.mark.parametrize("variant,height,rows,ny", [("AUTO", 8, 271, 16), ("GENERIC", 8, 271, 16), ("AUTO", 8, 542, 32),
+                                                    ("GENERIC", 16, 270, 16), ("GENERIC_Y8", 1, 582, 16),
+                                                    ("SYMMETRIC", 8, 582, 16)])
+def test_windows_of_257_rows(fbp, oracle, variant, height, rows, ny):
+    """Parallel beam with 17 detector rows a voxel (36 for tiles of eight):
+    the filtered rows of a tile are one more than a staged box holds."""
+    n, views, turns = (64, 92, 1.0) if variant == "SYMMETRIC" else (48, 91, 0.5)
+    cols = n // 2 if variant == "SYMMETRIC" else n  # narrow enough for the ring to hold the whole height
+    c = dict(du=n / cols, dv=ny / rows, span=2 * math.pi * turns, offset=0.0, nu=cols, nv=rows, nviews=views, nx=n, ny=ny,
+             nz=n, vox=1.0)
+    s = _solver(fbp, variant=variant)
+    s.upload_projections(_noise(6, views, rows, cols))
+    s.apply_filter_to_projections(0)
+    filtered = s.download_projections()
+    s.project_backward_parallel_from_projections(turns, n, ny, 0.0)
+    got, info = s.read_volume(), s.last_backprojection()
+    s.ctx.close()
+    # a voxel moves the position by 17 to 36 rows, whose rounding (2 ulp below 512) is 6e-5 of a row
+    assert relative_rmse(got, oracle.bp_parallel3d(filtered.astype(np.float64), c)) < 6e-5
+    assert info["tile_ny"] == height
