@@ -2140,12 +2140,11 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
 
 int launch_bp_plan(fbp_context* ctx, const BPLaunchPlan& p) {
   const int NY = p.ny_tile;
-  ctx->last_bp[0] = p.orbit      ? FBP_BACKPROJECTOR_GENERIC
+  ctx->last_bp[0] = p.orbit      ? FBP_BACKPROJECTOR_ORBITS
                     : p.use_quad ? FBP_BACKPROJECTOR_SYMMETRIC
                     : NY == 8    ? FBP_BACKPROJECTOR_GENERIC_Y8
                                  : FBP_BACKPROJECTOR_GENERIC;
-  // orbits: what the views' samples are stored as
-  ctx->last_bp[1] = !p.orbit ? p.layout : is_p16_layout(p.layout) ? kLayoutPair16 : kLayoutRaw32;
+  ctx->last_bp[1] = p.layout;
   ctx->last_bp[2] = p.a.box_u;
   ctx->last_bp[3] = p.a.box_v;
   ctx->last_bp[4] = NY;

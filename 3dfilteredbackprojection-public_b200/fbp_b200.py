@@ -422,8 +422,9 @@ class FBP3D:
         """Kernel, staged layout and window box of the last backprojection."""
         v, l, bu, bv, ny = C.c_int(), C.c_int(), C.c_int(), C.c_int(), C.c_int()
         self.ctx.call("fbp_last_backprojection", C.byref(v), C.byref(l), C.byref(bu), C.byref(bv), C.byref(ny))
-        names = {0: "rows32", 2: "pairs16", 3: "quads16", 4: "quads24", 5: "quads32"}
-        kernels = {Backprojector.SYMMETRIC: "symmetric", Backprojector.GENERIC_Y8: "generic_y8"}
+        names = {0: "rows32", 2: "pairs16", 3: "quads16", 4: "quads24", 5: "quads32", 6: "duos32", 7: "quads_pairs16",
+                 8: "duos_pairs16"}
+        kernels = {Backprojector.SYMMETRIC: "symmetric", Backprojector.GENERIC_Y8: "generic_y8", 4: "orbits"}
         return {"kernel": kernels.get(v.value, "generic"),
                 "layout": names.get(l.value, str(l.value)), "box": (bu.value, bv.value), "tile_ny": ny.value}
 

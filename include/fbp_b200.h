@@ -71,6 +71,9 @@ extern "C" {
                                       /* volume, views % 4 == 0 over one full turn */
 #define FBP_BACKPROJECTOR_GENERIC_Y8 3 /* generic with 16x16x8 tiles (8 voxels per  */
                                        /* thread along y), any geometry            */
+/* Reported, not set: AUTO's kernel for square volumes off the symmetric sizes
+ * (rotational orbits of four or two tiles), where it is the faster one. */
+#define FBP_BACKPROJECTOR_ORBITS 4
 
 /* ---- geometry kinds ------------------------------------------------------- */
 #define FBP_GEOMETRY_CONE 0     /* flat-panel cone beam, circular orbit         */
@@ -148,9 +151,10 @@ int fbp_set_symmetric_tile(fbp_context* ctx, int voxels_per_thread_y);
 int fbp_memory_in_use(const fbp_context* ctx, size_t* bytes);
 /* What the last backprojection ran (no counterpart in the reference, whose
  * backprojection is one fixed shader): *variant = FBP_BACKPROJECTOR_GENERIC,
- * _GENERIC_Y8 or _SYMMETRIC; *layout = staged view layout (0 FP32 rows,
+ * _GENERIC_Y8, _SYMMETRIC or _ORBITS; *layout = staged view layout (0 FP32 rows,
  * 2 FP16 row pairs, 3 FP16 four-view gradient quads, 4 24-bit four-view
- * gradient quads, 5 FP32 four-view quads);
+ * gradient quads, 5 FP32 four-view quads, 6 two views of FP32 samples, 7 and 8
+ * four and two views of FP16 row pairs);
  * *box_u x *box_v = largest staged detector window in elements; *tile_ny =
  * tile height along y. Any output pointer may be NULL. FBP_ERR_STATE
  * before the first backprojection. */

@@ -146,3 +146,67 @@ def test_windows_of_257_rows(fbp, oracle, variant, height, rows, ny):
     # a voxel moves the position by 17 to 36 rows, whose rounding (2 ulp below 512) is 6e-5 of a row
     assert relative_rmse(got, oracle.bp_parallel3d(filtered.astype(np.float64), c)) < 6e-5
     assert info["tile_ny"] == height
+
+
+# --------------------------------------------------------------- rotational orbits off the symmetric sizes
+FOUR, TWO = {"FP32": "quads32", "MIXED24": "quads32", "MIXED": "quads_pairs16"}, \
+            {"FP32": "duos32", "MIXED24": "duos32", "MIXED": "duos_pairs16"}
+FOUR_HIGH = dict(FOUR, MIXED="pairs16")  # 588 plain tiles: four waves, as many as FP16 orbits eight high would take
+# 24-bit views exist for the symmetric kernel only: FP32 here. FP16 views: 2^-12 a value (2.4e-4).
+TOL_ORBIT = {"FP32": TOL_BP, "MIXED24": TOL_BP, "MIXED": 4e-4}
+
+
+def _orbit_case(fbp, oracle, precision, beam, n, ny, views, turns, cols, rows, sinograms=False, scale=2.0):
+    offset = float(np.float32(0.7))
+    proj = _noise(n + views, views, rows, cols)
+    s = _solver(fbp, precision)
+    width = scale * n if beam == "cone" else float(n)
+    c = dict(span=2 * math.pi * float(np.float32(turns)), offset=offset, nu=cols, nv=rows, nviews=views, nx=n, ny=ny,
+             nz=n, vox=1.0, du=float(np.float32(width)) / cols)
+    what = "sinograms" if sinograms else "projections"
+    getattr(s, "upload_" + what)(np.ascontiguousarray(proj.transpose(1, 0, 2)) if sinograms else proj)
+    if beam == "cone":
+        c.update(dv=c["du"], sod=4.0 * n, sdd=6.0 * n)
+        getattr(s, "project_backward_cone_fdk_from_" + what)(4.0 * n, 2.0 * n, width, float(n), turns, n, ny, offset)
+        ref = oracle.bp_cone(proj.astype(np.float64), c)
+    else:
+        c.update(dv=ny / rows)
+        getattr(s, "project_backward_parallel_from_" + what)(turns, n, ny, offset)
+        ref = oracle.bp_parallel3d(proj.astype(np.float64), c)
+    got, info = s.read_volume(), s.last_backprojection()
+    s.ctx.close()
+    return relative_rmse(got, ref), info
+
+
+@pytest.mark.parametrize("precision", ["FP32", "MIXED", "MIXED24"])
+@pytest.mark.parametrize("beam,n,ny,views,turns,cols,rows,layout,height", [
+    # quarter turns: whole and odd sizes, one group, more turns, 12-high tiles
+    ("cone", 100, 49, 12, 1.0, 130, 80, FOUR, 8), ("cone", 97, 50, 4, 1.0, 90, 70, FOUR, 8),
+    ("cone", 111, 60, 36, 5.0, 300, 200, FOUR, 8), ("cone", 97, 177, 8, 1.0, 130, 240, FOUR_HIGH, 12),
+    # half turns, the other way round, an odd number of them
+    ("cone", 100, 49, 14, 1.0, 130, 80, TWO, 16), ("cone", 97, 53, 2, 1.0, 90, 70, TWO, 16),
+    ("cone", 99, 64, 12, -1.0, 260, 180, TWO, 16), ("cone", 112, 50, 10, 3.0, 130, 80, TWO, 16),
+    # parallel beam: half a turn (mirrored quarter turns), half turns, the half-turned voxel in the same view
+    ("parallel", 100, 49, 10, 0.5, 130, 49, FOUR, 8), ("parallel", 97, 51, 66, 0.5, 110, 77, FOUR, 8),
+    ("parallel", 113, 50, 2, 0.5, 100, 40, FOUR, 8), ("parallel", 100, 49, 12, 1.0, 130, 60, FOUR, 8),
+    ("parallel", 97, 52, 14, 1.0, 130, 60, TWO, 16), ("parallel", 100, 50, 11, 0.5, 111, 49, TWO, 16),
+    ("parallel", 97, 49, 13, 1.0, 140, 90, TWO, 16), ("parallel", 98, 49, 9, 0.3, 120, 49, TWO, 16)])
+def test_orbits(fbp, oracle, precision, beam, n, ny, views, turns, cols, rows, layout, height):
+    """Volumes large enough for rotational orbits: four and two slots, mirrored
+    ones, odd sizes with their centre column or middle row, volumes that end
+    inside a tile, with a start angle, through projections and sinograms."""
+    err, info = _orbit_case(fbp, oracle, precision, beam, n, ny, views, turns, cols, rows, sinograms=n % 2 == 1)
+    plain = layout[precision] == "pairs16"
+    assert info["kernel"] == ("generic" if plain else "orbits") and info["layout"] == layout[precision]
+    assert info["tile_ny"] == (16 if plain else height)
+    assert err < TOL_ORBIT[precision]
+
+
+@pytest.mark.parametrize("precision", ["FP32", "MIXED"])
+@pytest.mark.parametrize("views,layout", [(10, FOUR), (11, TWO)])
+def test_orbits_unstaged_windows(fbp, oracle, precision, views, layout):
+    """Windows wider than the widest box (128 elements) are gathered from the
+    views in global memory (zero outside the detector)."""
+    err, info = _orbit_case(fbp, oracle, precision, "parallel", 100, 49, views, 0.5, 660, 49)
+    assert info["kernel"] == "orbits" and info["layout"] == layout[precision] and info["box"][0] > 128
+    assert err < TOL_ORBIT[precision]
