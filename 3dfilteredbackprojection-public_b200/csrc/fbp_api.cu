@@ -317,10 +317,11 @@ fbp::BPGeom cone_geom(const Stack& s, float sod, float odd, float det_w, float v
 
 // Autotuner: the first backprojection of a geometry (with autotuning on) times
 // each applicable shape - the four-fold symmetric kernel with its own choice
-// of tile height, with 16 or with 8, the generic kernel
-// with 16 or 8 voxels per thread, each with its full view ring or a 4-stage
-// one - on a central slab of up to 48 y-slices (written into the volume,
-// which the real launch then overwrites) and keeps the fastest for that
+// of tile height, with 16 or with 8, the rotational orbits where the rule
+// takes them, the generic kernel with 16 or 8 voxels per thread, each with its
+// full view ring or a 4-stage one - on a central slab of up to 48 y-slices
+// (written into the volume, which the real launch then overwrites; orbits and
+// tile heights are the whole height's) and keeps the fastest for that
 // geometry, form, stack layout and GPU. With a cache file set, choices are
 // read from it and new ones appended, so other processes skip the timing.
 using TuneShape = fbp_context::TuneShape;
@@ -394,11 +395,12 @@ int autotune_backprojector(fbp_context* ctx, Stack& s, const fbp::BPGeom& g, boo
   gt.ny_total = g.ny_total > 0 ? g.ny_total : g.ny;
   gt.y_off = g.y_off + y0;
   gt.ny = nt;
+  gt.rule_ny = g.ny;
   gt.vol_ystride = g.vol_ystride > 0 ? g.vol_ystride : g.ny;
-  const TuneShape cand[7] = {{FBP_BACKPROJECTOR_SYMMETRIC, 0, 0},  {FBP_BACKPROJECTOR_SYMMETRIC, 16, 0},
-                             {FBP_BACKPROJECTOR_SYMMETRIC, 8, 0},  {FBP_BACKPROJECTOR_GENERIC, 0, 0},
-                             {FBP_BACKPROJECTOR_GENERIC, 0, 4},    {FBP_BACKPROJECTOR_GENERIC_Y8, 0, 0},
-                             {FBP_BACKPROJECTOR_GENERIC_Y8, 0, 4}};
+  const TuneShape cand[8] = {{FBP_BACKPROJECTOR_SYMMETRIC, 0, 0},  {FBP_BACKPROJECTOR_SYMMETRIC, 16, 0},
+                             {FBP_BACKPROJECTOR_SYMMETRIC, 8, 0},  {FBP_BACKPROJECTOR_ORBITS, 0, 0},
+                             {FBP_BACKPROJECTOR_GENERIC, 0, 0},    {FBP_BACKPROJECTOR_GENERIC, 0, 4},
+                             {FBP_BACKPROJECTOR_GENERIC_Y8, 0, 0}, {FBP_BACKPROJECTOR_GENERIC_Y8, 0, 4}};
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   FBP_TRY(fbp::cuda_check(ctx, cudaEventCreate(&e0), "event"));
   FBP_TRY(fbp::cuda_check(ctx, cudaEventCreate(&e1), "event"));

@@ -1756,11 +1756,11 @@ static Orbits find_orbits(bool cone, double turns, int K, bool square) {
 // (300 x 251 x 300, 450 to 452 views; 256^3 parallel; the 0.4 is what a SM's
 // last tiles lose by running alone, 100 x 80 x 100). FP32: four slots 1.13 (8
 // high) or 1.76 (12 high), two slots 1.42; FP16 pairs: 1.36 and 1.44.
-static bool choose_orbits(const BPGeom& g, double turns, bool p16, int num_sms, Orbits* orb) {
+static bool choose_orbits(const BPGeom& g, int ny, double turns, bool p16, int num_sms, Orbits* orb) {
   const bool cone = g.kind == FBP_GEOMETRY_CONE;
   const int t16 = (g.nx + 15) / 16, half = ((g.nx + 1) / 2 + 15) / 16;
   auto cost = [&](long long columns, int height, double rel) {
-    const long long tiles = columns * ((g.ny + height - 1) / height);
+    const long long tiles = columns * ((ny + height - 1) / height);
     return rel * ((double)((tiles + num_sms - 1) / num_sms) + 0.4);
   };
   double best = cost((long long)t16 * t16, 16, 1.0);
@@ -1802,21 +1802,24 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   const long long iturns = llround(turns);
   const bool symmetric = !is2d && g.nx == g.nz && g.nx % 32 == 0 && g.nviews % 4 == 0 &&
                          fabs(turns - (double)iturns) < 1e-9 && iturns % 4 == 1;
-  const bool quad = symmetric && !lim.plain &&
+  const bool quad = symmetric && lim.symmetric &&
                     (ctx->bp_variant == FBP_BACKPROJECTOR_AUTO || ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC);
   if (ctx->bp_variant == FBP_BACKPROJECTOR_SYMMETRIC && !symmetric)
     return set_error(ctx, FBP_ERR_UNSUPPORTED,
                      "the four-fold symmetric backprojector needs nx == nz (a multiple of 32), views % 4 == 0 and "
                      "views over one full turn");
-  // The generic backprojector's geometries that still have rotational orbits
-  // (any size; half turns, parallel beam) run on the same kernel, four or two
-  // voxels to a tap position, where that is faster; an explicit view ring is
-  // the plain kernel's.
+  // Square volumes off those sizes that still have rotational orbits (half
+  // turns, parallel beam) run on the same kernel, four or two voxels to a tap
+  // position, where that is faster; an explicit view ring is the plain kernel's.
   const bool p16 = mixed && !c24;
   Orbits orb = find_orbits(g.kind == FBP_GEOMETRY_CONE, turns, g.nviews, g.nx == g.nz);
-  const bool orbit = !quad && !is2d && !lim.plain && g.nx == g.nz && ctx->bp_stages == 0 &&
-                     (ctx->bp_variant == FBP_BACKPROJECTOR_AUTO || ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC) &&
-                     choose_orbits(g, turns, p16, ctx->num_sms, &orb);
+  const int rule_ny = g.rule_ny > 0 ? g.rule_ny : g.ny;
+  const bool tuned_orbits = ctx->bp_variant == FBP_BACKPROJECTOR_ORBITS;  // the tuner's shape, never a caller's
+  const bool orbit = !quad && !is2d && lim.orbits && g.nx == g.nz && ctx->bp_stages == 0 &&
+                     (ctx->bp_variant == FBP_BACKPROJECTOR_AUTO || (tuned_orbits && !symmetric)) &&
+                     choose_orbits(g, rule_ny, turns, p16, ctx->num_sms, &orb);
+  if (tuned_orbits && lim.orbits && !orbit)
+    return set_error(ctx, FBP_ERR_UNSUPPORTED, "rotational orbits are not this volume's faster form");
   // what the selected kernel reads: interleaved views (symmetric, orbits), FP16
   // pairs (MIXED) or the FP32 rows themselves
   const bool packed = quad || orbit || p16;
@@ -1873,8 +1876,8 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   // tile configuration: 16 x 16 columns, NY voxels along y (1 for 2D)
   const int TX = 16, TZ = 16;
   const int NY = is2d    ? 1
-                 : quad  ? quad_tile_height(ctx->quad_tile_ny, layout, a.nbx * a.nbz, g.ny, ctx->num_sms)
-                 : orbit ? quad_tile_height(0, layout, a.nbx * a.nbz, g.ny, ctx->num_sms)
+                 : quad  ? quad_tile_height(ctx->quad_tile_ny, layout, a.nbx * a.nbz, rule_ny, ctx->num_sms)
+                 : orbit ? quad_tile_height(0, layout, a.nbx * a.nbz, rule_ny, ctx->num_sms)
                          : std::min(lim.max_height, ctx->bp_variant == FBP_BACKPROJECTOR_GENERIC_Y8 ? 8 : 16);
   a.ntx = (g.nx + TX - 1) / TX;
   a.ntz = (g.nz + TZ - 1) / TZ;
@@ -1966,7 +1969,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
   // the limit above is about (parallel beam, 17 detector rows a voxel: 257 for
   // 16 voxels): lower tiles, down to one slice.
   if (layout == kLayoutRaw32 && bv > 256 && NY > 1)
-    return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{true, NY > 8 ? 8 : 1});
+    return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{false, false, NY > 8 ? 8 : 1});
   a.box_u = bu;
   a.box_v = bv;
   // two CTAs per SM: each gets half of the 228 KB shared memory
@@ -1983,7 +1986,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     const int rows16 = ((p16 ? bv : fv) - 2) * 16 / NY + 2;
     const size_t box = ((size_t)(p16 ? (plan.box_u + 3) / 4 * 4 : fu) * rows16 * (fp32 && st.filtered ? 8 : 4) + 127) / 128 * 128;
     if ((113 * 1024 - 64) / (box + sizeof(ViewCoef) + 2 * sizeof(uint64_t)) < 2)
-      return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{true});
+      return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{false, false});
   }
   if (use_quad) {
     // byte ring for the windows + entry records
@@ -2005,14 +2008,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
     }
   }
   if (!use_quad) {
-    if (quad) {
-      // re-plan with the generic tile height
-      const int saved = ctx->bp_variant;
-      ctx->bp_variant = FBP_BACKPROJECTOR_GENERIC;
-      const int rc = plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, lim);
-      ctx->bp_variant = saved;
-      return rc;
-    }
+    if (quad) return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{false, lim.orbits});
     a.box_bytes = (int)max_box;
     const size_t per_stage = a.box_bytes + sizeof(ViewCoef) + 2 * sizeof(uint64_t);
     int stages = (int)std::min<size_t>(kMaxStages, (smem_cap - 64) / per_stage);
@@ -2029,7 +2025,7 @@ int plan_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol, i
       // takes: the plain kernel reads the rows themselves, or pairs of at most
       // the orbits' bytes
       if ((rc == FBP_ERR_OUT_OF_MEMORY || rc == FBP_ERR_UNSUPPORTED) && (orbit || layout == kLayoutQuad32))
-        return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{true});
+        return plan_backproject(ctx, g, st, vol, clip_ylimit, mixed, plan_out, PlanLimits{false, false});
       return rc;
     }
   a.inv_scale = is_p16_layout(layout) || layout == kLayoutQuadG16 ? st.inv_scale : nullptr;  // set by the pack

@@ -290,6 +290,7 @@ struct BPGeom {
   int row_off = 0, nv_total = 0;
   int y_off = 0, ny_total = 0;
   int vol_ystride = 0;  // y-slices between z planes of the output (0: ny); a slab of a whole volume
+  int rule_ny = 0;      // height that kernels and tile heights are chosen for (0: ny); the tuner's slab
 };
 // Backproject the stack's rows, packed first into the layout that the
 // selected kernel reads (prepare_packed) where that is not the rows
@@ -300,8 +301,8 @@ int launch_backproject(fbp_context* ctx, const BPGeom& g, Stack& st, float* vol,
 // together in one persistent launch on another context's stream.
 struct BPLaunchPlan;
 struct PlanLimits {
-  bool plain = false;   // no interleaved views
-  int max_height = 16;  // of the plain kernel's tiles
+  bool symmetric = true, orbits = true;  // neither: the plain kernel
+  int max_height = 16;                   // of the plain kernel's tiles
 };
 BPLaunchPlan* new_bp_plan();
 void free_bp_plan(BPLaunchPlan* p);

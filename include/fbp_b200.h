@@ -65,7 +65,8 @@ extern "C" {
 #define FBP_FILTER_IMPL_TOEPLITZ 2 /* tcgen05 split-BF16 Toeplitz GEMM       */
 
 /* ---- backprojector variants ----------------------------------------------- */
-#define FBP_BACKPROJECTOR_AUTO 0      /* symmetric when the geometry allows it      */
+#define FBP_BACKPROJECTOR_AUTO 0      /* symmetric when the geometry allows it, then */
+                                      /* orbits where they are faster, then generic */
 #define FBP_BACKPROJECTOR_GENERIC 1   /* one 16x16x16 tile per CTA, any geometry    */
 #define FBP_BACKPROJECTOR_SYMMETRIC 2 /* four-fold orbit of tiles per CTA: square  */
                                       /* volume, views % 4 == 0 over one full turn */
@@ -123,15 +124,15 @@ int fbp_set_clip_after_backprojection(fbp_context* ctx, int enable);
 int fbp_set_backprojector(fbp_context* ctx, int variant);
 /* 1: with the variant AUTO, the first backprojection of each geometry (form,
  * staged layout, detector band and volume slab included) times the
- * applicable kernels - symmetric, generic with 16 and with 8 voxels per
- * thread along y - on a central slab of up to 48 y-slices and keeps the
+ * applicable kernels - symmetric, orbits, generic with 16 and with 8 voxels
+ * per thread along y - on a central slab of up to 48 y-slices and keeps the
  * fastest for later calls of that geometry; 0 (default): AUTO picks the
- * symmetric kernel when the geometry allows it. No counterpart in the
+ * kernel by the geometry. No counterpart in the
  * reference, whose backprojection is one fixed shader. */
 int fbp_set_autotune(fbp_context* ctx, int enable);
 /* With autotuning on: the shapes the tuner times are the symmetric kernel
- * with its own choice of tile height, with 16 and with 8, and the generic
- * kernel with 16 or 8 voxels per thread, each with its full view ring or a
+ * with its own choice of tile height, with 16 and with 8, the orbits, and the
+ * generic kernel with 16 or 8 voxels per thread, each with its full view ring or a
  * 4-stage one. A cache
  * file (path; NULL or "" = none) keeps the choices across processes: they are
  * read from it on the first tuning and each new choice is appended as one

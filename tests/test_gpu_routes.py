@@ -210,3 +210,41 @@ def test_orbits_unstaged_windows(fbp, oracle, precision, views, layout):
     err, info = _orbit_case(fbp, oracle, precision, "parallel", 100, 49, views, 0.5, 660, 49)
     assert info["kernel"] == "orbits" and info["layout"] == layout[precision] and info["box"][0] > 128
     assert err < TOL_ORBIT[precision]
+
+
+# --------------------------------------------------------------- kernels asked for and tuned
+@pytest.mark.parametrize("precision,layout", [("FP32", "rows32"), ("MIXED24", "rows32"), ("MIXED", "pairs16")])
+@pytest.mark.parametrize("variant,height", [("GENERIC", 16), ("GENERIC_Y8", 8)])
+def test_the_generic_kernel_when_asked_for(fbp, oracle, precision, layout, variant, height):
+    """GENERIC is the plain kernel, also where AUTO takes orbits."""
+    n, ny, views, cols, rows = 100, 49, 12, 130, 80
+    proj = _noise(8, views, rows, cols)
+    c = dict(span=2 * math.pi, offset=0.0, nu=cols, nv=rows, nviews=views, nx=n, ny=ny, nz=n, vox=1.0, du=200.0 / cols,
+             dv=200.0 / cols, sod=400.0, sdd=600.0)
+    info = {}
+    for v in (variant, "AUTO"):
+        s = _solver(fbp, precision, variant=v)
+        s.upload_projections(proj)
+        s.project_backward_cone_fdk_from_projections(400.0, 200.0, 200.0, float(n), 1.0, n, ny, 0.0)
+        got, info[v] = s.read_volume(), s.last_backprojection()
+        s.ctx.close()
+        assert relative_rmse(got, oracle.bp_cone(proj.astype(np.float64), c)) < TOL_ORBIT[precision]
+    assert info[variant]["kernel"] == variant.lower() and info[variant]["layout"] == layout
+    assert info[variant]["tile_ny"] == height and info["AUTO"]["kernel"] == "orbits"
+
+
+@pytest.mark.parametrize("precision", ["FP32", "MIXED"])
+@pytest.mark.parametrize("n,ny", [(100, 64), (100, 100), (96, 200), (50, 40)])
+def test_the_tuned_kernel_is_the_one_that_runs(fbp, tmp_path, precision, n, ny):
+    """The shape recorded in the tuner's cache file is what the whole volume
+    runs on, although the tuner's slab is 48 slices high."""
+    s = _solver(fbp, precision, tune=True)
+    s.set_autotune_cache(tmp_path / "tune.txt")
+    s.upload_projections(_noise(9, 60, 90, 130))
+    s.project_backward_cone_fdk_from_projections(4.0 * n, 2.0 * n, 2.0 * n, float(n), 1.0, n, ny, 0.0)
+    s.synchronize()
+    info = s.last_backprojection()
+    s.ctx.close()
+    variant, quad_ny = (int(x) for x in (tmp_path / "tune.txt").read_text().split("|")[1].split()[:2])
+    assert info["kernel"] == {1: "generic", 2: "symmetric", 3: "generic_y8", 4: "orbits"}[variant]
+    assert not quad_ny or info["tile_ny"] == quad_ny
