@@ -2425,9 +2425,10 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
           const double Ux = -a.vox * s * a.du_per_mm, Uz = a.vox * c * a.du_per_mm;
           const double U0 = (-Xc * s + Zc * c) * a.du_per_mm;
           // Detector window over the tile's four corners (u is monotonic along
-          // each edge, so the corners bound it). FP32 is enough here, to well
-          // under the window's margin; the FP64 chain of a lane is what delays
-          // a CTA's first steps, so it holds no division.
+          // each edge, so the corners bound it). FP32 is enough for columns
+          // counted from the detector's centre, to well under the window's
+          // margin; the FP64 chain of a lane is what delays a CTA's first
+          // steps, so it holds no division.
           float umin = 3e38f, umax = -3e38f, dmin = 3e38f;
           const float fUx = (float)Ux, fUz = (float)Uz, fU0 = (float)U0;
           const float fDx = (float)Dx, fDz = (float)Dz, fD0 = (float)D0;
@@ -2436,7 +2437,7 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
             const float x = (cc & 1) ? (float)(kTile2D - 1) : 0.f, z = (cc & 2) ? (float)(kTile2D - 1) : 0.f;
             const float D = fmaf(fDx, x, fmaf(fDz, z, fD0));
             const float n = fmaf(fUx, x, fmaf(fUz, z, fU0));
-            const float u = (CONE ? n * rcp_approx(D) : n) + (float)a.cu;
+            const float u = CONE ? n * rcp_approx(D) : n;
             dmin = fminf(dmin, D);
             umin = fminf(umin, u);
             umax = fmaxf(umax, u);
@@ -2444,9 +2445,9 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
           // one column of margin on each side for the FP32 rounding of u; a
           // window that starts left of the padding or past the detector holds
           // zeros only, whatever its origin
-          const int cap = 1 << 20;
-          const int u0 = (int)floorf(fminf(fmaxf(umin - 1.f, (float)-cap), (float)cap)) & ~(ALIGN - 1);
-          const bool fits = floorf(umax) + 3.f - (float)u0 <= (float)a.win;
+          const double cap = 1 << 30;
+          const int u0 = (int)floor(fmin(fmax(umin + a.cu - 1.0, -cap), cap)) & ~(ALIGN - 1);
+          const bool fits = floor(umax + a.cu) + 3.0 - u0 <= (double)a.win;
           if (!(dmin > 1e-6f) || !fits) atomicCAS(a.err, 0, kDevFootprint);
           start = min(max(u0 + a.pad, 0), a.pad + (a.nu + ALIGN - 1) / ALIGN * ALIGN);
           const double du0 = a.cu - u0;  // u - u0 = (N . (x, z, 1)) / D with N re-based

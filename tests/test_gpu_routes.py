@@ -248,3 +248,29 @@ def test_the_tuned_kernel_is_the_one_that_runs(fbp, tmp_path, precision, n, ny):
     variant, quad_ny = (int(x) for x in (tmp_path / "tune.txt").read_text().split("|")[1].split()[:2])
     assert info["kernel"] == {1: "generic", 2: "symmetric", 3: "generic_y8", 4: "orbits"}[variant]
     assert not quad_ny or info["tile_ny"] == quad_ny
+
+
+# --------------------------------------------------------------- 2D slices
+@pytest.mark.parametrize("kind", ["fan", "parallel"])
+@pytest.mark.parametrize("bins", [2_100_001, 40_000_003])
+def test_bp2d_wide_detectors(fbp, oracle, kind, bins):
+    """Rows far wider than the image: the columns that it sees lie around a
+    detector centre that FP32 no longer counts exactly (2^24 and more)."""
+    n, views = 40, 3 if bins > 1 << 24 else 8
+    det = 1.5 * bins
+    sino = np.zeros((views, bins), np.float32)
+    mid = slice(bins // 2 - 400, bins // 2 + 400)
+    sino[:, mid] = np.random.default_rng(11).standard_normal((views, 800)).astype(np.float32)
+    f2 = fbp.FBP2D(0)
+    if kind == "fan":
+        sod, sdd = 200.0, 300.0
+        img = f2.project_backward(sino, fbp.Geometry.cone(sod, sdd - sod, det, 1.0 * n, 1.0, 0.1), (n, n))
+    else:
+        sod = sdd = 0.0
+        img = f2.project_backward(sino, fbp.Geometry.parallel(det, 1.0 * n, 0.5, 0.1), (n, n))
+    # the oracle sees the middle of the detector alone
+    c = dict(nx=n, ny=1, nz=n, vox=1.0, nu=800 + bins % 2, nv=1, nviews=views, du=float(np.float32(det)) / bins, dv=1.0,
+             span=2 * math.pi * (1.0 if kind == "fan" else 0.5), offset=float(np.float32(0.1)), sod=sod, sdd=sdd)
+    part = np.ascontiguousarray(sino[:, bins // 2 - 400:bins // 2 + 400 + bins % 2]).astype(np.float64)
+    ref = (oracle.bp_fan2d if kind == "fan" else oracle.bp_parallel2d)(part, c)
+    assert relative_rmse(img, ref) < TOL_BP
