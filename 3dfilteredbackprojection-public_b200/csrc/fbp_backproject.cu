@@ -2483,8 +2483,10 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
     // --------------------------------------------------------------- consumers
     const float fx = (float)lane, fz = (float)(warp * kPix2D);
     const uint32_t wbase = smem_u32(wins);
-    // bit patterns of kMagic + column, column in [0, win - 2]: bounds the reads
-    const int lo = (int)kMagicBits, hi = (int)kMagicBits + a.win - 2;
+    // a tap's column is in [0, win - 2]: bounds the reads. worst: the largest
+    // one that a tap asked for (negative ones are larger than any)
+    const uint32_t last = (uint32_t)(a.win - 2);
+    uint32_t worst = 0;
     const float2 magic2 = make_float2(kMagic, kMagic);
     int e = 0;
     uint32_t ph = 0;
@@ -2500,7 +2502,7 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
         for (int i = 0; i < n; ++i) {
           const float4 N = *reinterpret_cast<const float4*>(&coef[e * kSteps2D + i]);
           const float2 D = *reinterpret_cast<const float2*>(&coef[e * kSteps2D + i].Dz);
-          const uint32_t c0 = wbase + (uint32_t)(e * kSteps2D + i) * win_bytes - kMagicBits * (4u * SLOTS);
+          const uint32_t c0 = wbase + (uint32_t)(e * kSteps2D + i) * win_bytes;
           // pixels j, j + 1 as packed pairs, stepped along z
           const float n0 = fmaf(N.x, fx, fmaf(N.y, fz, N.z)), d0 = fmaf(N.w, fx, fmaf(D.x, fz, D.y));
           float2 num = make_float2(n0, n0 + N.y), den = make_float2(d0, d0 + D.x);
@@ -2521,10 +2523,11 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
             const float2 fu = fsub2(u, fsub2(t, magic2));
             const float wb[2] = {CONE ? W.x * fu.x : fu.x, CONE ? W.y * fu.y : fu.y};
             const float wa[2] = {W.x - wb[0], W.y - wb[1]};
-            const int bits[2] = {max(min(__float_as_int(t.x), hi), lo), max(min(__float_as_int(t.y), hi), lo)};
+            const uint32_t col[2] = {__float_as_uint(t.x) - kMagicBits, __float_as_uint(t.y) - kMagicBits};
+            worst = max(worst, max(col[0], col[1]));
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
-              const uint32_t at = (uint32_t)bits[p] * (4u * SLOTS) + c0;
+              const uint32_t at = min(col[p], last) * (4u * SLOTS) + c0;
               if constexpr (SLOTS == 4) {
                 const uint4 A = lds_u4(at), B = lds_u4(at + 16);
                 const float2 wa2 = make_float2(wa[p], wa[p]), wb2 = make_float2(wb[p], wb[p]);
@@ -2563,6 +2566,8 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
         acc[0][j] = t;
       }
     }
+    // cannot happen when the window above is right (a NaN angle's taps are NaN)
+    if (worst > last && worst != 0x7fffffffu - kMagicBits) atomicCAS(a.err, 0, kDevFootprint);
   }
   if (warp < NCW) {
     // after `phases` turns rotation r sits in slot (r + phases) mod SLOTS
