@@ -181,10 +181,15 @@ __device__ __forceinline__ float2 unpack2(unsigned long long r) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
   return d;
 }
-// packed FP32 pairs (sm_100): a b + c, a + b toward zero, a - b
+// packed FP32 pairs (sm_100): a b + c, a b, a + b toward zero, a - b
 __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
   unsigned long long d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 __device__ __forceinline__ unsigned long long add2_rz(unsigned long long a, unsigned long long b) {
@@ -238,13 +243,15 @@ __global__ void __launch_bounds__(32 * kColWarps) forward_columns_kernel(const F
     const float* p10 = p00 + px;
     const float* p01 = p00 + pz;
     const float* p11 = p01 + px;
-    // pairs over z; lerp along y, x, z
+    // pairs over z; weighted sums along y, x, z (a + w (b - a) would turn an
+    // infinite voxel into NaN, and rounds the difference as well)
     const unsigned long long a0 = pack2(__ldg(p00), __ldg(p01)), a1 = pack2(__ldg(p00 + 1), __ldg(p01 + 1));
     const unsigned long long b0 = pack2(__ldg(p10), __ldg(p11)), b1 = pack2(__ldg(p10 + 1), __ldg(p11 + 1));
-    const unsigned long long wy2 = pack2(wy, wy);
-    const unsigned long long ax = fma2(wy2, sub2(a1, a0), a0), bx = fma2(wy2, sub2(b1, b0), b0);
-    const float2 z = unpack2(fma2(pack2(w.x, w.x), sub2(bx, ax), ax));
-    acc += fmaf(w.y, z.y - z.x, z.x);
+    const float vx = 1.f - w.x, vy = 1.f - wy;
+    const unsigned long long wy2 = pack2(wy, wy), vy2 = pack2(vy, vy);
+    const unsigned long long ax = fma2(wy2, a1, mul2(vy2, a0)), bx = fma2(wy2, b1, mul2(vy2, b0));
+    const float2 z = unpack2(fma2(pack2(w.x, w.x), bx, mul2(pack2(vx, vx), ax)));
+    acc += fmaf(w.y, z.y, (1.f - w.y) * z.x);
   }
   const long long row = a.sinogram ? (long long)iv * a.nviews + k : (long long)k * a.nv + iv;
   a.out[row * a.pitch + iu] = acc * r.step;

@@ -274,3 +274,21 @@ def test_bp2d_wide_detectors(fbp, oracle, kind, bins):
     part = np.ascontiguousarray(sino[:, bins // 2 - 400:bins // 2 + 400 + bins % 2]).astype(np.float64)
     ref = (oracle.bp_fan2d if kind == "fan" else oracle.bp_parallel2d)(part, c)
     assert relative_rmse(img, ref) < TOL_BP
+
+
+# --------------------------------------------------------------- forward projection
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.float32(3e38)])
+def test_forward_of_an_infinite_voxel(fbp, value):
+    """Rays through an infinite (or the largest) voxel sum to infinity, as the
+    weighted sum of the neighbours does: no NaN from a difference."""
+    n, views = 24, 5
+    vol = np.full((n, n, n), -1.0 if value > 0 else 1.0, np.float32)
+    vol[11, 12, 13] = value
+    s = fbp.FBP3D(0)
+    s.generate_blank_volume(n, n, n)
+    s.write_volume_data(vol)
+    s.project_forward_cone_to_projections(4.0 * n, 2.0 * n, 1.5 * n, float(n), 1.0, views, 0.3)
+    got = s.download_projections()
+    s.ctx.close()
+    assert not np.isnan(got).any()
+    assert (np.abs(got) > 1e37).any(axis=(1, 2)).all() and (np.abs(got) < 1e3).any(axis=(1, 2)).all()
