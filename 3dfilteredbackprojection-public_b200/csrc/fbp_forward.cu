@@ -46,15 +46,15 @@ struct FPArgs {
 };
 
 // Ray of detector pixel (iu, iv) at the view (c, s), clipped to the volume box:
-// n samples of length step, the first at voxel-index position f0 (the centre
-// of voxel 0 at `origin`), each next one by d (FP32). n = 0: the ray misses
+// n samples of length step, the first at voxel-index position f0 (voxel centres
+// at integers), each next one by d (FP32). n = 0: the ray misses
 // the box.
 struct RayMarch {
   long long n;
   float step, fx0, fy0, fz0, dx, dy, dz;
 };
 
-__device__ __forceinline__ RayMarch ray_march(const FPArgs& a, double c, double s, int iu, int iv, double origin) {
+__device__ __forceinline__ RayMarch ray_march(const FPArgs& a, double c, double s, int iu, int iv) {
   const double u = (iu + 0.5 - 0.5 * a.nu) * a.du, v = (iv + 0.5 - 0.5 * a.nv) * a.dv;
   const double hx = 0.5 * a.nx * a.vox, hy = 0.5 * a.ny * a.vox, hz = 0.5 * a.nz * a.vox;
   double S[3], D[3];
@@ -100,9 +100,9 @@ __device__ __forceinline__ RayMarch ray_march(const FPArgs& a, double c, double 
     const double step = (t1 - t0) / r.n;
     const double tm = t0 + 0.5 * step;
     r.step = (float)step;
-    r.fx0 = (float)((S[0] + tm * D[0]) / a.vox + 0.5 * a.nx - 0.5 + origin);
-    r.fy0 = (float)((S[1] + tm * D[1]) / a.vox + 0.5 * a.ny - 0.5 + origin);
-    r.fz0 = (float)((S[2] + tm * D[2]) / a.vox + 0.5 * a.nz - 0.5 + origin);
+    r.fx0 = (float)((S[0] + tm * D[0]) / a.vox + 0.5 * a.nx - 0.5);
+    r.fy0 = (float)((S[1] + tm * D[1]) / a.vox + 0.5 * a.ny - 0.5);
+    r.fz0 = (float)((S[2] + tm * D[2]) / a.vox + 0.5 * a.nz - 0.5);
     r.dx = (float)(step * D[0] / a.vox);
     r.dy = (float)(step * D[1] / a.vox);
     r.dz = (float)(step * D[2] / a.vox);
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(128) forward_rows_kernel(const FPArgs a) {
   sincos(a.offset + a.span * k / a.nviews, &s, &c);
   const long long sx = 1, sy = a.nx, sz = (long long)a.nx * a.ny;
   for (int iv = blockIdx.y; iv < a.nv; iv += gridDim.y) {
-    const RayMarch r = ray_march(a, c, s, iu, iv, 0.0);
+    const RayMarch r = ray_march(a, c, s, iu, iv);
     float acc = 0.f;
     for (long long q = 0; q < r.n; ++q) {
       const float fq = (float)q;
@@ -203,7 +203,7 @@ __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigne
   return d;
 }
 
-constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: x + kMagic toward zero is kMagic + floor(x) for 0 <= x < 2^22
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: x + kMagic toward zero is kMagic + floor(x) for |x| < 2^22
 constexpr uint32_t kMagicBits = 0x4B400000u;
 // Detector rows from which the column march is the faster one although it
 // leaves lanes idle below 32 (256 x ny x 256, 180 views, ms: rows 1.21, 1.91,
@@ -218,11 +218,11 @@ __global__ void __launch_bounds__(32 * kColWarps) forward_columns_kernel(const F
   if (iu >= a.nu || iv >= a.nv) return;
   double s, c;
   sincos(a.offset + a.span * k / a.nviews, &s, &c);
-  const RayMarch r = ray_march(a, c, s, iu, iv, 1.0);
+  const RayMarch r = ray_march(a, c, s, iu, iv);
   const uint32_t px = (uint32_t)py, pz = (uint32_t)py * (uint32_t)(a.nx + 2);
-  // element of the cell (i, j, l) of the bordered copy; the position's bit
-  // patterns minus kMagicBits are i, j, l
-  const uint32_t base = 0u - kMagicBits * (px + pz + 1u);
+  // element of the cell (i, j, l), which the bordered copy has at i + 1, j + 1,
+  // l + 1; the position's bit patterns minus kMagicBits are i, j, l
+  const uint32_t base = (1u - kMagicBits) * (px + pz + 1u);
   const unsigned long long dxz = pack2(r.dx, r.dz), fxz0 = pack2(r.fx0, r.fz0);
   const unsigned long long magic2 = pack2(kMagic, kMagic);
   float acc = 0.f, fq = 0.f;
