@@ -349,6 +349,13 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return r;
 }
 
+// The same after one Newton-Raphson step, r + r (1 - x r): as good as a rounded
+// division here (error against FP64 to three digits), at a third of its cost.
+__device__ __forceinline__ float rcp_newton(float x) {
+  const float r = rcp_approx(x);
+  return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
 // FP16 x FP16 + FP32 with one rounding to FP32.
 __device__ __forceinline__ float fma_f16_f32(__half a, __half b, float c) {
   float d;
@@ -473,7 +480,7 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
     const ViewCoef g = coef[s];
     if (!(g.skip & 1)) {
       const float D = fmaf(g.Dx, fx, fmaf(g.Dz, fz, g.D0));
-      const float rD = rcp_approx(D);
+      const float rD = rcp_newton(D);
       const float ul = fmaf(g.Nx, fx, fmaf(g.Nz, fz, g.N0)) * rD;
       const float vl = fmaf(g.Vx, fx, fmaf(g.Vz, fz, g.V0)) * rD;
       const float dvv = a.dvn * rD;
@@ -492,9 +499,10 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
         const uint32_t c0 = smem_u32(smem + (size_t)s * a.box_bytes) + (uint32_t)(iu * ESZ) - kMagicBits * RB;
         // floor and fraction of v with the rounding constant: v + kMagic toward
         // zero is kMagic + floor(v), whose bit pattern times RB plus c0 is the
-        // element's address; two voxels at a time in packed FP32, stepped by 2 dvv
-        float2 v2 = make_float2(vl, vl + dvv);
-        const float2 step2 = make_float2(2.f * dvv, 2.f * dvv), magic2 = make_float2(kMagic, kMagic);
+        // element's address; two voxels at a time in packed FP32. v is formed anew
+        // for each voxel: stepped from the one before, its rounding adds up
+        const float2 magic2 = make_float2(kMagic, kMagic);
+        auto v_at = [&](int j) { return make_float2(fmaf((float)j, dvv, vl), fmaf((float)(j + 1), dvv, vl)); };
         if constexpr (LAYOUT == kLayoutRaw32) {
           // where the rows advance by less than one per voxel, march along the
           // column: a voxel's upper row, interpolated in u (the distance weight
@@ -508,8 +516,7 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
             uint32_t before = 0;
 #pragma unroll
             for (int j = 0; j < NY; j += 2) {
-              if (j) v2 = fadd2(v2, step2);
-              const float2 t2 = fadd2_rz(v2, magic2);
+              const float2 v2 = v_at(j), t2 = fadd2_rz(v2, magic2);
               const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
 #pragma unroll
               for (int p = 0; p < 2 && j + p < NY; ++p) {
@@ -529,8 +536,7 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
           // element = (row v, row v + 1 minus row v); the u-lerp of both in FP32
 #pragma unroll
           for (int j = 0; j < NY; j += 2) {
-            if (j) v2 = fadd2(v2, step2);
-            const float2 t2 = fadd2_rz(v2, magic2);
+            const float2 v2 = v_at(j), t2 = fadd2_rz(v2, magic2);
             const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
 #pragma unroll
             for (int p = 0; p < 2 && j + p < NY; ++p) {
@@ -1061,7 +1067,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
     if (!(flags & kQSkip)) {
       // explicit roundings (no contraction): the same bits in every instantiation
       const float D = fmaf(g.Dx, fx, fmaf(g.Dz, fz, g.D0));
-      const float rD = rcp_approx(D);
+      const float rD = EDGES ? rcp_newton(D) : rcp_approx(D);
       const float ul = __fmul_rn(fmaf(g.Nx, fx, fmaf(g.Nz, fz, g.N0)), rD);
       const float dvv = __fmul_rn(g.dvn, rD);
       const float vl0 = __fmul_rn(fmaf(g.Vx, fx, fmaf(g.Vz, fz, g.V0)), rD);
@@ -1075,25 +1081,37 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
       if (iu >= 0 && iu <= g.bu2 && vl >= 0.f && vlast < g.vmax) {
         const uint32_t c0 = g.cbase + (uint32_t)(iu * CB);
         // v of voxels j and j + 1, stepped by 2 dvv from (vl, vl + dvv): no
-        // per-pair constants (a few ulps of v from the repeated additions);
+        // per-pair constants (a few ulps of v from the repeated additions, which
+        // the orbits of the plain kernel's geometries do without as that does);
         // floor and fraction of the pair with packed FP32 ops
         static_assert(NY % 2 == 0, "voxels stepped in pairs");
         const float2 magic2 = make_float2(kMagic, kMagic);
         const float dv2 = 2.f * dvv;
         const float2 step2 = make_float2(dv2, dv2);
         float2 v2 = make_float2(vl, vl + dvv);
+        auto advance = [&](int j) {
+          if constexpr (EDGES)
+            v2 = ffma2(make_float2((float)j, (float)(j + 1)), make_float2(dvv, dvv), make_float2(vl, vl));
+          else if (j)
+            v2 = fadd2(v2, step2);
+        };
         if constexpr (Q32) {
           // weights of the two columns, the distance weight folded in
           const float wbs = __fmul_rn(W, fu), was = __fsub_rn(W, wbs);
           const float2 wa = make_float2(was, was), wb = make_float2(wbs, wbs);
           // an element row at this thread's detector position: the slots' pairs, interpolated in u
           auto blend = [&](const float2& A, const float2& B) { return ffma2(wb, B, fmul2(wa, A)); };
+          // One rounding into a sum: the two products added to it one after the
+          // other cost an operation less and a fifth more error (256^3 x 360 4.0
+          // -> 4.8e-7 against FP64; 2.76 and 2.82 ms). Two forms of the
+          // interpolation, by what ptxas makes of them (12 high 42.3 and 43.4 ms
+          // at a drawn 420^3; 8 high 2.84 and 2.82 ms).
           auto add = [&](const float2 (&lo)[S / 2], const float2 (&hi)[S / 2], float fv, int j) {
-            const float fl = 1.f - fv;
+            const float2 fv2 = make_float2(fv, fv), fl2 = make_float2(1.f - fv, 1.f - fv);
 #pragma unroll
             for (int p = 0; p < S / 2; ++p) {
-              const float2 d = ffma2(make_float2(fv, fv), hi[p],
-                                     ffma2(make_float2(fl, fl), lo[p], make_float2(acc[2 * p][j], acc[2 * p + 1][j])));
+              const float2 t = NY == 12 ? ffma2(fv2, hi[p], fmul2(fl2, lo[p])) : ffma2(fv2, fsub2(hi[p], lo[p]), lo[p]);
+              const float2 d = fadd2(make_float2(acc[2 * p][j], acc[2 * p + 1][j]), t);
               acc[2 * p][j] = d.x;
               acc[2 * p + 1][j] = d.y;
             }
@@ -1116,7 +1134,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
               uint32_t before = 0;  // bit pattern of the previous voxel's row
 #pragma unroll
               for (int j = 0; j < NY; j += 2) {
-                if (j) v2 = fadd2(v2, step2);
+                advance(j);
                 const float2 t2 = fadd2_rz(v2, magic2);
                 const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
 #pragma unroll
@@ -1193,7 +1211,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
             };
 #pragma unroll
             for (int j = 0; j < NY; j += 2) {
-              if (j) v2 = fadd2(v2, step2);
+              advance(j);
               const float2 t2 = fadd2_rz(v2, magic2);
               const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
 #pragma unroll
@@ -1274,7 +1292,7 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
             const uint32_t plane = g.plane;
 #pragma unroll
             for (int j = 0; j < NY; j += 2) {
-              if (j) v2 = fadd2(v2, step2);
+              advance(j);
               const float2 t2 = fadd2_rz(v2, magic2);
               const float2 fv2 = fsub2(v2, fsub2(t2, magic2));
               const uint32_t a0 = __float_as_uint(t2.x) * RB + c0, a1 = __float_as_uint(t2.y) * RB + c0;

@@ -292,3 +292,37 @@ def test_forward_of_an_infinite_voxel(fbp, value):
     s.ctx.close()
     assert not np.isnan(got).any()
     assert (np.abs(got) > 1e37).any(axis=(1, 2)).all() and (np.abs(got) < 1e3).any(axis=(1, 2)).all()
+
+
+# --------------------------------------------------------------- FP32 sums
+# K values near c added up, each addition rounded once: an error of ulp(S) /
+# sqrt(12) for the running sum S, independent from one to the next. Summed over
+# S = c, 2c .. 1024 c that is 4.2e-7 (1024 c a power of two) to 4.8e-7 (half way to
+# the next) of the sum. Two roundings an addition: 5.9e-7 to 6.8e-7. The values
+# scatter by 3%, which an error of 2e-5 of a sample in the tap's position turns
+# into less than 1e-8 of the sum.
+TOL_SUM = 5.3e-7
+
+
+def _near_one(seed, *shape):
+    return (1.0 + 0.05 * (2.0 * np.random.default_rng(seed).random(shape) - 1.0)).astype(np.float32)
+
+
+@pytest.mark.parametrize("kernel,n,ny,views,rows", [
+    ("symmetric", 64, 20, 1024, 60), ("symmetric", 160, 128, 1024, 260), ("orbits", 100, 49, 1024, 120),
+    ("orbits", 100, 49, 1022, 120), ("generic", 50, 24, 1023, 70)])
+def test_fp32_sums_round_once(fbp, oracle, kernel, n, ny, views, rows):
+    cols = int(2.4 * n)
+    c = dict(sod=4.0 * n, sdd=6.0 * n, du=1.2, dv=1.2, span=2 * math.pi, offset=0.0, nu=cols, nv=rows, nviews=views,
+             nx=n, ny=ny, nz=n, vox=1.0)
+    c["du"] = c["dv"] = float(np.float32(1.2 * cols)) / cols
+    proj = _near_one(12, views, rows, cols)
+    s = _solver(fbp)
+    s.upload_projections(proj)
+    s.project_backward_cone_fdk_from_projections(4.0 * n, 2.0 * n, 1.2 * cols, float(n), 1.0, n, ny, 0.0)
+    got, info = s.read_volume(), s.last_backprojection()
+    s.ctx.close()
+    m = slice(n // 4, n - n // 4)  # inside the field of view
+    ref = oracle.bp_cone(proj.astype(np.float64), c)[m, :, m]
+    assert info["kernel"] == kernel
+    assert relative_rmse(got[m, :, m], ref) < TOL_SUM
