@@ -326,3 +326,23 @@ def test_fp32_sums_round_once(fbp, oracle, kernel, n, ny, views, rows):
     ref = oracle.bp_cone(proj.astype(np.float64), c)[m, :, m]
     assert info["kernel"] == kernel
     assert relative_rmse(got[m, :, m], ref) < TOL_SUM
+
+
+@pytest.mark.parametrize("kind,n,views,turns", [("fan", 600, 1023, 1.0), ("fan", 960, 1024, 1.0),
+                                                ("parallel", 600, 1023, 0.5)])
+def test_2d_sums_round_once(fbp, oracle, kind, n, views, turns):
+    bins = int(2.4 * n)
+    sino = _near_one(13, views, bins)
+    det = 1.0 * bins if kind == "fan" else 1.5 * n
+    f2 = fbp.FBP2D(0)
+    if kind == "fan":
+        sod, sdd = 4.0 * n, 5.0 * n
+        img = f2.project_backward(sino, fbp.Geometry.cone(sod, n, det, float(n), turns, 0.0), (n, n))
+    else:
+        sod = sdd = 0.0
+        img = f2.project_backward(sino, fbp.Geometry.parallel(det, float(n), turns, 0.0), (n, n))
+    c = dict(nx=n, ny=1, nz=n, vox=1.0, nu=bins, nv=1, nviews=views, du=float(np.float32(det)) / bins, dv=1.0,
+             span=2 * math.pi * turns, offset=0.0, sod=sod, sdd=sdd)
+    ref = (oracle.bp_fan2d if kind == "fan" else oracle.bp_parallel2d)(sino.astype(np.float64), c)
+    m = slice(n // 4, n - n // 4)
+    assert relative_rmse(img.reshape(n, n)[m, m], np.asarray(ref).reshape(n, n)[m, m]) < TOL_SUM
