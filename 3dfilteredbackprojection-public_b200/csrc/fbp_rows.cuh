@@ -28,9 +28,7 @@ __device__ __forceinline__ float pre_log(const RowSet& rs, float x) {
 
 // sdd / distance for a detector column u off the centre
 __device__ __forceinline__ float pre_weight(const RowSet& rs, float dist2, float u) {
-  float inv;  // rsqrtf without its scaling of subnormal arguments
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(fmaf(u, u, dist2)));
-  return rs.w_sdd * inv;
+  return rs.w_sdd * rsqrtf(fmaf(u, u, dist2));
 }
 
 __device__ __forceinline__ float pre_op(const RowSet& rs, long long r, int i, float x) {

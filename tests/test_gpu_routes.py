@@ -346,3 +346,26 @@ def test_2d_sums_round_once(fbp, oracle, kind, n, views, turns):
     ref = (oracle.bp_fan2d if kind == "fan" else oracle.bp_parallel2d)(sino.astype(np.float64), c)
     m = slice(n // 4, n - n // 4)
     assert relative_rmse(img.reshape(n, n)[m, m], np.asarray(ref).reshape(n, n)[m, m]) < TOL_SUM
+
+
+# --------------------------------------------------------------- weights
+@pytest.mark.parametrize("what", ["weights", "FFT", "TOEPLITZ"])
+def test_fdk_weights_of_tiny_lengths(fbp, oracle, what):
+    """Lengths in a unit that makes their squares subnormal (9e-40, with steps
+    of 1.6e-6 of that: 8e-7 of the weight)."""
+    views, rows, cols = 3, 5, 96
+    sod, odd, width = 2e-20, 1e-20, 4e-20
+    proj = _near_one(14, views, rows, cols)
+    s = _solver(fbp)
+    s.upload_projections(proj)
+    s.apply_fdk_weights_to_projections(sod, odd, width)
+    f = lambda x: float(np.float32(x))  # noqa: E731
+    ref = oracle.fdk_weight(proj.astype(np.float64), f(sod) + f(odd), f(width) / cols, f(width) / cols)
+    if what != "weights":
+        s.set_filter_impl(getattr(fbp.FilterImpl, what))
+        s.apply_filter_to_projections(0)
+        ref = oracle.filter_rows(ref.reshape(-1, cols), 0).reshape(proj.shape)
+    got = s.download_projections()
+    s.ctx.close()
+    # the filter's output is a tenth of its input here; split rows: 2^-17 of a value
+    assert relative_rmse(got, ref) < {"weights": 2e-6, "FFT": 2e-5, "TOEPLITZ": 1e-4}[what]
