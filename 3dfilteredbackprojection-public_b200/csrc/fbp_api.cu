@@ -125,7 +125,7 @@ int alloc_stack(fbp_context* ctx, Stack& s, int u, int v, int n, bool clear = tr
     cudaFree(s.f32);
     s.f32 = nullptr;
     s.f32_cap = 0;
-    if (cudaMalloc(&s.f32, need) != cudaSuccess) {
+    if (fbp::device_alloc(ctx, &s.f32, need) != cudaSuccess) {
       s.f32 = nullptr;
       cudaGetLastError();
       return fbp::set_error(ctx, FBP_ERR_OUT_OF_MEMORY, "cudaMalloc of the detector stack failed");
@@ -190,7 +190,7 @@ int ensure_volume(fbp_context* ctx, int x, int y, int z, bool clear) {
       cudaFree(ctx->vol);
       ctx->vol = nullptr;
       ctx->vol_cap = 0;
-      if (cudaMalloc(&ctx->vol, need) != cudaSuccess) {
+      if (fbp::device_alloc(ctx, &ctx->vol, need) != cudaSuccess) {
         ctx->vol = nullptr;
         ctx->vx = ctx->vy = ctx->vz = 0;
         cudaGetLastError();
@@ -519,13 +519,23 @@ int cuda_check(fbp_context* ctx, cudaError_t e, const char* what) {
   return set_error(ctx, code, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+cudaError_t device_alloc_bytes(fbp_context* ctx, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 void* scratch(fbp_context* ctx, size_t bytes) {
   if (bytes <= ctx->scratch_bytes) return ctx->d_scratch;
   cudaFree(ctx->d_scratch);
   ctx->d_scratch = nullptr;
   ctx->scratch_bytes = 0;
   size_t b = std::max<size_t>(bytes, 1 << 20);
-  if (cudaMalloc(&ctx->d_scratch, b) != cudaSuccess) {
+  if (device_alloc(ctx, &ctx->d_scratch, b) != cudaSuccess) {
     cudaGetLastError();
     set_error(ctx, FBP_ERR_OUT_OF_MEMORY, "cudaMalloc of scratch memory failed");
     ctx->d_scratch = nullptr;
@@ -604,7 +614,7 @@ int prepare_packed(fbp_context* ctx, Stack& s, int layout, const Orbits& o) {
     cudaFree(s.filt);
     s.filt = nullptr;
     s.filt_bytes = 0;
-    if (cuda_check(ctx, cudaMalloc(&s.filt, need), "cudaMalloc(packed views)")) return FBP_ERR_OUT_OF_MEMORY;
+    if (cuda_check(ctx, device_alloc(ctx, &s.filt, need), "cudaMalloc(packed views)")) return FBP_ERR_OUT_OF_MEMORY;
     s.filt_bytes = need;
   }
   if (!s.inv_scale || s.scale_cap < s.n) {

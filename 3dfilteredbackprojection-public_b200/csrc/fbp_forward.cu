@@ -284,19 +284,39 @@ int launch_forward(fbp_context* ctx, const float* vol, int nx, int ny, int nz, d
   a.pitch = pitch;
   a.sinogram = sinogram;
   // The column march needs detector rows to fill its warps, a bordered copy
-  // that 32-bit element indices reach, and room for it.
+  // that 32-bit element indices reach, and room for it. A copy of up to
+  // kKeptCopy stays with the context (its scratch); a larger one, up to 16 GB,
+  // belongs to the call: allocated and freed in stream order, it is the
+  // device's again at the next wait.
+  constexpr size_t kKeptCopy = 256u << 20;
   const int py = (ny + 2 + 3) / 4 * 4;
-  const size_t elems = (size_t)(nz + 2) * (nx + 2) * py;
+  const size_t elems = (size_t)(nz + 2) * (nx + 2) * py, bytes = elems * sizeof(float);
   if (nv >= kMinColumnRows && ny > 1 && elems < (1ull << 32) - 1 && nz + 2 <= 65535 && (ny + 33) / 32 <= 65535) {
-    if (float* cols = static_cast<float*>(scratch(ctx, elems * sizeof(float)))) {
+    const bool keep = bytes <= kKeptCopy;
+    void* cols = nullptr;
+    if (keep) {
+      cols = scratch(ctx, bytes);
+    } else if (cudaMallocAsync(&cols, bytes, ctx->stream) != cudaSuccess) {
+      cudaGetLastError();
+      cols = nullptr;
+    }
+    if (cols) {
+      float* const copy = static_cast<float*>(cols);
       volume_columns_kernel<<<dim3((nx + 2 + 31) / 32, (py + 31) / 32, nz + 2), 256, 0, ctx->stream>>>(vol, nx, ny, nz,
-                                                                                                      py, cols);
-      if (int rc = launched(ctx, "volume_columns_kernel")) return rc;
-      // the last element that a cell may start at (its far corner is the copy's last element)
-      const uint32_t last = (uint32_t)(elems - 2 - (size_t)py * (nx + 2) - py);
-      const dim3 grid((nu + kColWarps - 1) / kColWarps, (nv + 31) / 32, nviews);
-      forward_columns_kernel<<<grid, 32 * kColWarps, 0, ctx->stream>>>(a, cols, py, last);
-      return launched(ctx, "forward_columns_kernel");
+                                                                                                      py, copy);
+      int rc = launched(ctx, "volume_columns_kernel");
+      if (!rc) {
+        // the last element that a cell may start at (its far corner is the copy's last element)
+        const uint32_t last = (uint32_t)(elems - 2 - (size_t)py * (nx + 2) - py);
+        const dim3 grid((nu + kColWarps - 1) / kColWarps, (nv + 31) / 32, nviews);
+        forward_columns_kernel<<<grid, 32 * kColWarps, 0, ctx->stream>>>(a, copy, py, last);
+        rc = launched(ctx, "forward_columns_kernel");
+      }
+      if (!keep) {
+        const cudaError_t e = cudaFreeAsync(cols, ctx->stream);
+        if (!rc) rc = cuda_check(ctx, e, "cudaFreeAsync(volume copy)");
+      }
+      return rc;
     }
     ctx->last_error.clear();  // no room for the copy: march through the volume itself
   }

@@ -243,6 +243,13 @@ inline int launched(fbp_context* ctx, const char* what) {
   return cuda_check(ctx, cudaGetLastError(), what);
 }
 void* scratch(fbp_context* ctx, size_t bytes);
+// cudaMalloc, tried again after a wait for ctx's stream: what its work still
+// holds in stream order (launch_forward's copy of a large volume) comes back there.
+cudaError_t device_alloc_bytes(fbp_context* ctx, void** p, size_t bytes);
+template <class T>
+cudaError_t device_alloc(fbp_context* ctx, T** p, size_t bytes) {
+  return device_alloc_bytes(ctx, reinterpret_cast<void**>(p), bytes);
+}
 
 // ---- filter (fbp_filter.cu) ----
 struct RowSet {

@@ -619,7 +619,7 @@ int launch_filter_toeplitz(fbp_context* ctx, const RowSet& rs, int n, int filter
       cudaFree(t.th);
       t.th = nullptr;
       t.cap = 0;
-      if (cuda_check(ctx, cudaMalloc(&t.th, need), "cudaMalloc(Toeplitz operands)")) return FBP_ERR_OUT_OF_MEMORY;
+      if (cuda_check(ctx, device_alloc(ctx, &t.th, need), "cudaMalloc(Toeplitz operands)")) return FBP_ERR_OUT_OF_MEMORY;
       t.cap = need;
     }
     if (int rc = ensure_filter_tables(ctx, n, filter)) return rc;
