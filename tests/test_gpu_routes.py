@@ -396,3 +396,38 @@ def test_fdk_weights_of_tiny_lengths(fbp, oracle, what):
     s.ctx.close()
     # the filter's output is a tenth of its input here; split rows: 2^-17 of a value
     assert relative_rmse(got, ref) < {"weights": 2e-6, "FFT": 2e-5, "TOEPLITZ": 1e-4}[what]
+
+
+@pytest.mark.parametrize("kind", ["fan", "parallel"])
+def test_bp2d_without_room_for_the_packed_rows(fbp, oracle, kind):
+    """Rows that nearly fill the device: the packed copy does not fit, and the
+    rows are read where they are (detector narrower than the image, odd sizes)."""
+    n, nz, views, bins = 41, 37, 4100, 6001
+    sino = np.zeros((views, bins), np.float32)
+    sino[:, 2900:3101] = np.random.default_rng(16).standard_normal((views, 201))
+    sino[:, 0] = sino[:, -1] = 1.0
+    det = 0.2 * bins
+    d = torch.as_tensor(sino, device="cuda")
+    out = torch.empty((nz, n), device="cuda")
+    f2 = fbp.FBP2D(0)
+    if kind == "fan":
+        sod, sdd = 400.0, 500.0
+        g = fbp.Geometry.cone(sod, sdd - sod, det, float(n), 1.0, 0.1)
+    else:
+        sod = sdd = 0.0
+        g = fbp.Geometry.parallel(det, float(n), 0.5, 0.1)
+    f2.project_backward(d[:40, :400].contiguous(), g, (n, nz))  # modules, angles' buffer
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    spare = torch.empty(max(0, torch.cuda.mem_get_info()[0] - sino.nbytes // 2), dtype=torch.uint8, device="cuda")
+    try:
+        f2.project_backward(d, g, (n, nz), out=out)
+        got = out.cpu().numpy()
+    finally:
+        f2.ctx.close()
+        del spare, d, out
+        torch.cuda.empty_cache()
+    c = dict(nx=n, ny=1, nz=nz, vox=1.0, nu=bins, nv=1, nviews=views, du=float(np.float32(det)) / bins, dv=1.0,
+             span=2 * math.pi * (1.0 if kind == "fan" else 0.5), offset=float(np.float32(0.1)), sod=sod, sdd=sdd)
+    ref = (oracle.bp_fan2d if kind == "fan" else oracle.bp_parallel2d)(sino.astype(np.float64), c)
+    assert relative_rmse(got, ref) < TOL_BP
