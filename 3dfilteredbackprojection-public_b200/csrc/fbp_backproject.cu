@@ -2638,6 +2638,27 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
   if (nsplit > 1) cluster.sync();  // no CTA leaves while another reads its sums
 }
 
+// The rows where they are, a pixel a thread, positions in FP64: for a device
+// without room for the packed rows.
+__global__ void __launch_bounds__(256) bp2d_rows_kernel(const BP2DArgs a, int nviews) {
+  const int ix = blockIdx.x * 32 + threadIdx.x % 32;
+  for (int iz = blockIdx.y * 8 + threadIdx.x / 32; iz < a.nz && ix < a.nx; iz += gridDim.y * 8) {
+    const double X = (ix + 0.5 - 0.5 * a.nx) * a.vox, Z = (iz + 0.5 - 0.5 * a.nz) * a.vox;
+    float acc = 0.f;
+    for (int k = 0; k < nviews; ++k) {
+      const double c = a.trig[k].x, s = a.trig[k].y;
+      const double rD = 1.0 / (1.0 + (X * c + Z * s) * a.inv_sod);
+      const double u = (Z * c - X * s) * a.du_per_mm * rD + a.cu, fl = floor(u);
+      if (!(fl >= -1.0 && fl < (double)a.nu)) continue;
+      const int iu = (int)fl;
+      const float* p = a.rows + (long long)k * a.pitch + iu;
+      const float lo = iu >= 0 ? __ldg(p) : 0.f, hi = iu + 1 < a.nu ? __ldg(p + 1) : 0.f;
+      acc = fmaf((float)(rD * rD), fmaf((float)(u - fl), hi - lo, lo), acc);
+    }
+    a.image[(size_t)iz * a.nx + ix] = acc * a.scale;
+  }
+}
+
 template <bool CONE, int SLOTS>
 cudaError_t launch_bp2d_cfg(const BP2DArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
   auto kern = bp2d_kernel<CONE, SLOTS>;
@@ -2690,22 +2711,7 @@ int launch_bp2d(fbp_context* ctx, const BPGeom& g, const float* sino, long long 
   const int tiles_x = (rx + kTile2D - 1) / kTile2D, tiles_z = (rz + kTile2D - 1) / kTile2D;
   const long long tiles = (long long)tiles_x * tiles_z;
   if (int rc = ensure_trig(ctx, g)) return rc;
-  BP2DArgs a;
-  a.pad = win;
-  a.win = win;
-  a.pitch = (g.nu + 3) / 4 * 4 + 2LL * win;
-  const size_t bytes = sizeof(float) * (size_t)a.pitch * groups * slots;
-  float* rows = static_cast<float*>(scratch(ctx, bytes));
-  if (!rows) return FBP_ERR_OUT_OF_MEMORY;
-  const dim3 pgrid((unsigned)((a.pitch + 255) / 256), std::min(groups, 65535));
-  if (slots == 4)
-    pack2d_kernel<4><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
-  else if (slots == 2)
-    pack2d_kernel<2><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
-  else
-    pack2d_kernel<1><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
-  if (int rc = launched(ctx, "pack2d_kernel")) return rc;
-  a.rows = rows;
+  BP2DArgs a{};
   a.image = image;
   a.trig = ctx->d_trig;
   a.vox = g.vox;
@@ -2719,6 +2725,27 @@ int launch_bp2d(fbp_context* ctx, const BPGeom& g, const float* sino, long long 
   a.phases = phases;
   a.scale = cone ? (float)(pi / K * g.sdd / (g.sod * g.du)) : (float)(pi / K / g.du);
   a.err = ctx->d_err;
+  a.pad = win;
+  a.win = win;
+  a.pitch = (g.nu + 3) / 4 * 4 + 2LL * win;
+  const size_t bytes = sizeof(float) * (size_t)a.pitch * groups * slots;
+  float* rows = static_cast<float*>(scratch(ctx, bytes));
+  if (!rows) {
+    ctx->last_error.clear();
+    a.rows = sino;
+    a.pitch = pitch;
+    bp2d_rows_kernel<<<dim3((g.nx + 31) / 32, std::min((g.nz + 7) / 8, 65535)), 256, 0, ctx->stream>>>(a, K);
+    return launched(ctx, "bp2d_rows_kernel");
+  }
+  const dim3 pgrid((unsigned)((a.pitch + 255) / 256), std::min(groups, 65535));
+  if (slots == 4)
+    pack2d_kernel<4><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
+  else if (slots == 2)
+    pack2d_kernel<2><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
+  else
+    pack2d_kernel<1><<<pgrid, 256, 0, ctx->stream>>>(sino, pitch, g.nu, groups, a.pad, mirror, a.pitch, rows);
+  if (int rc = launched(ctx, "pack2d_kernel")) return rc;
+  a.rows = rows;
   const size_t entry = (size_t)kSteps2D * (win * slots * 4 + sizeof(Coef2D)) + 2 * sizeof(uint64_t);
   const size_t fixed = sizeof(float) * slots * kTile2D * kPart2D + 16;
   a.ring = (int)std::max<size_t>(2, std::min<size_t>(kMaxRing2D, (48 * 1024) / entry));
