@@ -1412,7 +1412,6 @@ __global__ void __launch_bounds__(quad_threads(LAYOUT, NY, YW), OCC)
       bad = false;
       if (*s_abort) break;
       store();
-      if (!MULTI) break;
       reset();
       last = false;
     }
