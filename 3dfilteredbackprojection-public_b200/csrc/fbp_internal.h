@@ -193,6 +193,8 @@ struct fbp_context {
   fbp::Stack sino;
 
   int* d_err = nullptr;          // device error word
+  int* h_err = nullptr;          // pinned word it is read back into
+  int h_err_page = -1;           // shared page of it (-1: its own allocation)
   int* d_minmax = nullptr;       // volume min / max as order-preserving int keys
   bool minmax_valid = false;     // d_minmax describes the current volume
   double2* d_trig = nullptr;     // per-view (cos, sin) in FP64

@@ -431,3 +431,33 @@ def test_bp2d_without_room_for_the_packed_rows(fbp, oracle, kind):
              span=2 * math.pi * (1.0 if kind == "fan" else 0.5), offset=float(np.float32(0.1)), sod=sod, sdd=sdd)
     ref = (oracle.bp_fan2d if kind == "fan" else oracle.bp_parallel2d)(sino.astype(np.float64), c)
     assert relative_rmse(got, ref) < TOL_BP
+
+
+# --------------------------------------------------------------- contexts
+def test_contexts_report_their_own_errors(fbp):
+    """More contexts than a shared page has error words: each reports its own
+    device error (a voxel behind the source), once, and no other's; words that
+    closed contexts gave back serve new ones."""
+    def project(s, sod):
+        s.upload_projections(np.ones((8, 24, 24), np.float32))
+        s.project_backward_cone_fdk_from_projections(sod, 60.0, 24.0, 16.0, 1.0, 16, 8, 0.0)
+
+    def expect(s, bad):
+        if bad:
+            with pytest.raises(fbp.FBPError) as e:
+                s.synchronize()
+            assert e.value.status == -7
+        s.synchronize()
+
+    solvers = [_solver(fbp) for _ in range(70)]
+    for turn in range(2):
+        bad = {3, 40, 66, 69} if turn == 0 else {0, 65}
+        for i, s in enumerate(solvers):
+            project(s, 2.0 if i in bad else 60.0)
+        for i, s in reversed(list(enumerate(solvers))):
+            expect(s, i in bad)
+        for i in range(0, 70, 3):
+            solvers[i].ctx.close()
+            solvers[i] = _solver(fbp)
+    for s in solvers:
+        s.ctx.close()
