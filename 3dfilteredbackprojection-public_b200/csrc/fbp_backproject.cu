@@ -25,7 +25,7 @@
 //     another.
 //   * Per view a consumer thread forms 1/D, its detector column u (constant
 //     along the column), the distance weight and the v step once; per voxel it
-//     steps v and takes floor / fraction with the 1.5 * 2^23 rounding constant
+//     forms v and takes floor / fraction with the 1.5 * 2^23 rounding constant
 //     (no conversion instructions). FP16 views are staged as row pairs
 //     (element (v, u) holds rows v and v + 1), FP32 views as plain rows along
 //     which the taps march.
@@ -610,15 +610,18 @@ __global__ void __launch_bounds__(TX* TZ + 32, 2) bp_kernel(const __grid_constan
 // as long as the rows advance by at most one per voxel, and a second one where
 // they advance by more.
 //
-// Bound: FP32, the load / store unit (80% busy: 2 to 3 wavefronts per 32
-// updates); MIXED, the FMA pipes' dependent chains (29 FMA-pipe operations per
-// four updates; 64% of issue slots at 16 consumer warps); 24-bit, both.
+// Bound (counters at 256^3): FP32, the shared-memory wavefronts of the load /
+// store unit (81% of its rate; issue slots 61%, heavy FMA pipe 60%); MIXED, the
+// FMA pipes' dependent chains (heavy pipe 70%, issue 65%, wavefronts 68%);
+// 24-bit, wavefronts 78% and issue 70% (12 bytes and four half-rate byte
+// permutes an update, which the FP32 form does without: it is the faster one);
+// FP16 row pairs on orbits, the heavy FMA pipe (76%).
 // Measured, backprojection with its packing, before = four row-pair windows
 // (FP32) or the quarters unrolled (MIXED), 8 consumer warps, one producer warp:
 //            256^3 x 360     512^3 x 720     480^3 x 480*    768^3 x 1024
-//   FP32     3.59 -> 2.47    55.6 -> 37.0    23.8 -> 17.6    264.6 -> 174.0 ms
-//   MIXED    2.66 -> 2.52    39.4 -> 36.6    15.9 -> 14.8    185.5 -> 165.4 ms
-//   24-bit   3.63 -> 3.32    52.8 -> 46.4    20.9 -> 19.7    247.5 -> 214.3 ms
+//   FP32     3.59 -> 2.51    55.6 -> 37.4    23.8 -> 17.3    264.6 -> 175.9 ms
+//   MIXED    2.66 -> 2.45    39.4 -> 36.2    15.9 -> 14.7    185.5 -> 163.6 ms
+//   24-bit   3.63 -> 3.11    52.8 -> 44.7    20.9 -> 19.1    247.5 -> 208.7 ms
 // (* the 1440^3 geometry at a third). Tried and slower: fetching a view's record
 // and projection before the previous view's taps (and two windows held at once
 // can need more than the ring), 16 voxels a thread for FP32.
@@ -1579,8 +1582,8 @@ int quad_occ(int layout, int ny_tile) {
 // 384^3: MIXED 8 high 0.29, 0.45, 1.18, 8.1; 16 high 0.42, 0.44, 1.16, 8.1; 24
 // high 0.56, 0.59, 1.11, 7.6. FP32 and 24-bit take 12 from 36 waves on
 // (about 440^3): 8 and 12 high 0.31 and 0.47, 0.50 and 0.77, 1.40 and 1.48, 9.8
-// and 10.1 at those sizes, then 18.9 and 17.6 at 480 x 490 x 480 (480 views),
-// 38.1 and 37.2 at 512^3 (720 views; 24-bit 49.3 and 46.4); and where it makes
+// and 10.1 at those sizes, then 18.8 and 17.3 at 480 x 490 x 480 (480 views),
+// 38.1 and 37.4 at 512^3 (720 views; 24-bit 46.8 and 44.7); and where it makes
 // one wave of more than 1.2 (160 x 128 x 160: 0.87 and 0.72, 24-bit 0.90 and
 // 0.86; 128 x 153 x 128, 1.08 waves, 0.59 and 0.81).
 int quad_tile_height(int asked, int layout, int orbits, int ny, int num_sms) {
@@ -2317,8 +2320,8 @@ int launch_bp_batch(fbp_context* L, BPLaunchPlan* const* plans, int n, const lon
 //
 // Measured (the packing included), before = one 32 x 32 tile of plain pixels
 // a CTA with its setup and staging between block barriers: fan 1024^2, 1440
-// views 2297 -> 523 us (84% of the shared-memory rate while a SM has work),
-// 1441 views 2301 -> 1172 us; fan 512^2, 720 views 467 -> 81 us; parallel
+// views 2297 -> 537 us (82% of the shared-memory rate while a SM has work),
+// 1441 views 2301 -> 1098 us; fan 512^2, 720 views 467 -> 83 us; parallel
 // 256^2, 360 views 132 -> 21 us (about 12 us of it two launches and a CTA's
 // start).
 constexpr int kTile2D = 32;     // representative pixels per tile side
@@ -2750,9 +2753,9 @@ int launch_bp2d(fbp_context* ctx, const BPGeom& g, const float* sino, long long 
   a.ring = (int)std::max<size_t>(2, std::min<size_t>(kMaxRing2D, (48 * 1024) / entry));
   size_t smem = fixed + a.ring * entry;
   // Split the views over a cluster until one and a half tiles a SM are in
-  // flight (fan 512^2, 720 views, 64 tiles: 158.8, 89.2, 81.1, 91.9 us split
-  // 1, 2, 4, 8 ways; 1024^2, 1440 views, 256 tiles: 522.9, 526.1, 520.7,
-  // 558.7 us). Clusters of 8 leave SMs of a GPC over.
+  // flight (fan 512^2, 720 views, 64 tiles: 164.0, 91.9, 83.0, 93.6 us split
+  // 1, 2, 4, 8 ways; 1024^2, 1440 views, 256 tiles: 537.3, 536.3, 532.3,
+  // 569.2 us). Clusters of 8 leave SMs of a GPC over.
   int split = 1;
   while (split < kMaxSplit2D && 2 * tiles * split < 3LL * ctx->num_sms && groups >= 16 * split) split *= 2;
   // CTAs that all find an SM of their own must not share one (the tap's

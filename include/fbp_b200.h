@@ -70,6 +70,8 @@ extern "C" {
 #define FBP_BACKPROJECTOR_GENERIC 1   /* one 16x16x16 tile per CTA, any geometry    */
 #define FBP_BACKPROJECTOR_SYMMETRIC 2 /* four-fold orbit of tiles per CTA: square  */
                                       /* volume, views % 4 == 0 over one full turn */
+                                      /* (FP32 views without room for their        */
+                                      /* interleaved copy: the generic kernel)     */
 #define FBP_BACKPROJECTOR_GENERIC_Y8 3 /* generic with 16x16x8 tiles (8 voxels per  */
                                        /* thread along y), any geometry            */
 /* Reported, not set: AUTO's kernel for square volumes off the symmetric sizes
