@@ -2321,7 +2321,7 @@ int launch_bp_batch(fbp_context* L, BPLaunchPlan* const* plans, int n, const lon
 // Measured (the packing included), before = one 32 x 32 tile of plain pixels
 // a CTA with its setup and staging between block barriers: fan 1024^2, 1440
 // views 2297 -> 537 us (82% of the shared-memory rate while a SM has work),
-// 1441 views 2301 -> 1098 us; fan 512^2, 720 views 467 -> 83 us; parallel
+// 1441 views 2301 -> 1132 us; fan 512^2, 720 views 467 -> 83 us; parallel
 // 256^2, 360 views 132 -> 21 us (about 12 us of it two launches and a CTA's
 // start).
 constexpr int kTile2D = 32;     // representative pixels per tile side
@@ -2445,30 +2445,29 @@ __global__ void __launch_bounds__(256 + 32, 2) bp2d_kernel(const BP2DArgs a) {
           const double Ux = -a.vox * s * a.du_per_mm, Uz = a.vox * c * a.du_per_mm;
           const double U0 = (-Xc * s + Zc * c) * a.du_per_mm;
           // Detector window over the tile's four corners (u is monotonic along
-          // each edge, so the corners bound it). FP32 is enough for columns
-          // counted from the detector's centre, to well under the window's
-          // margin; the FP64 chain of a lane is what delays a CTA's first
-          // steps, so it holds no division.
-          float umin = 3e38f, umax = -3e38f, dmin = 3e38f;
-          const float fUx = (float)Ux, fUz = (float)Uz, fU0 = (float)U0;
-          const float fDx = (float)Dx, fDz = (float)Dz, fD0 = (float)D0;
+          // each edge, so the corners bound it). The FP64 chain of a lane is what
+          // delays a CTA's first steps, so it holds no division: a Newton step on
+          // the FP32 reciprocal leaves 1e-13 of a column's distance.
+          double umin = 1e300, umax = -1e300, dmin = 1e300;
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) {
-            const float x = (cc & 1) ? (float)(kTile2D - 1) : 0.f, z = (cc & 2) ? (float)(kTile2D - 1) : 0.f;
-            const float D = fmaf(fDx, x, fmaf(fDz, z, fD0));
-            const float n = fmaf(fUx, x, fmaf(fUz, z, fU0));
-            const float u = CONE ? n * rcp_approx(D) : n;
-            dmin = fminf(dmin, D);
-            umin = fminf(umin, u);
-            umax = fmaxf(umax, u);
+            const double x = (cc & 1) ? kTile2D - 1 : 0, z = (cc & 2) ? kTile2D - 1 : 0;
+            double u = Ux * x + (Uz * z + U0);
+            if (CONE) {
+              const double D = Dx * x + (Dz * z + D0), r = (double)rcp_approx((float)D);
+              dmin = fmin(dmin, D);
+              u *= r * (2.0 - D * r);
+            }
+            umin = fmin(umin, u);
+            umax = fmax(umax, u);
           }
-          // one column of margin on each side for the FP32 rounding of u; a
-          // window that starts left of the padding or past the detector holds
-          // zeros only, whatever its origin
+          // one column of margin on each side for the FP32 rounding of the taps'
+          // positions; a window that starts left of the padding or past the
+          // detector holds zeros only, whatever its origin
           const double cap = 1 << 30;
           const int u0 = (int)floor(fmin(fmax(umin + a.cu - 1.0, -cap), cap)) & ~(ALIGN - 1);
           const bool fits = floor(umax + a.cu) + 3.0 - u0 <= (double)a.win;
-          if (!(dmin > 1e-6f) || !fits) atomicCAS(a.err, 0, kDevFootprint);
+          if (!(dmin > 1e-6) || !fits) atomicCAS(a.err, 0, kDevFootprint);
           start = min(max(u0 + a.pad, 0), a.pad + (a.nu + ALIGN - 1) / ALIGN * ALIGN);
           const double du0 = a.cu - u0;  // u - u0 = (N . (x, z, 1)) / D with N re-based
           cf.Nx = (float)(Ux + du0 * Dx);

@@ -399,6 +399,27 @@ def test_fdk_weights_of_tiny_lengths(fbp, oracle, what):
 
 
 @pytest.mark.parametrize("kind", ["fan", "parallel"])
+def test_bp2d_wide_images(fbp, oracle, kind):
+    """An image of one long row that spans 17 million detector columns: the
+    windows at its ends lie further from the detector's centre than FP32 counts."""
+    n, views, bins = 1_600_001, 2, 17_000_001
+    sino = np.random.default_rng(18).standard_normal((views, bins)).astype(np.float32)
+    det = 0.1 * bins if kind == "parallel" else 0.15 * bins
+    f2 = fbp.FBP2D(0)
+    if kind == "fan":
+        sod, sdd = 4.0 * n, 6.0 * n
+        img = f2.project_backward(sino, fbp.Geometry.cone(sod, sdd - sod, det, float(n), 1.0, 1.5), (n, 1))
+    else:
+        sod = sdd = 0.0
+        img = f2.project_backward(sino, fbp.Geometry.parallel(det, float(n), 0.5, 1.5), (n, 1))
+    c = dict(nx=n, ny=1, nz=1, vox=1.0, nu=bins, nv=1, nviews=views, du=float(np.float32(det)) / bins, dv=1.0,
+             span=2 * math.pi * (1.0 if kind == "fan" else 0.5), offset=float(np.float32(1.5)),
+             sod=float(np.float32(sod)), sdd=float(np.float32(sod)) + float(np.float32(sdd - sod)))
+    ref = (oracle.bp_fan2d if kind == "fan" else oracle.bp_parallel2d)(sino.astype(np.float64), c)
+    assert relative_rmse(img, ref) < TOL_BP
+
+
+@pytest.mark.parametrize("kind", ["fan", "parallel"])
 def test_bp2d_without_room_for_the_packed_rows(fbp, oracle, kind):
     """Rows that nearly fill the device: the packed copy does not fit, and the
     rows are read where they are (detector narrower than the image, odd sizes)."""
